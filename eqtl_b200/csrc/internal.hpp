@@ -226,7 +226,7 @@ struct Workspace {
   DevBuf<int2> ref_pairs;
   // batched REML (p > 3): covariate pair products, per-round weights and sums
   DevBuf<double> rb_P, rb_dlt, rb_W, rb_WY, rb_A, rb_B, rb_ld, rb_ydy;
-  DevBuf<double> rb_Wg, rb_Xw, rb_Ag, rb_Lg, rb_ldx, rb_ldD, rb_Bg, rb_Yg;  // grid phase
+  DevBuf<double> rb_Wg, rb_Xw, rb_Ag, rb_Lg, rb_ldx, rb_ldD, rb_Bg, rb_Yg, rb_V;  // grid phase
   DevBuf<uint8_t> rb_state;
   DevBuf<unsigned int> rb_active;
   // NB-GLM null fits: per gene and sample mu, w = mu / (1 + phi mu) and

@@ -350,7 +350,7 @@ __global__ void __launch_bounds__(256) reml_warp_kernel(const double* __restrict
 // with W[i, s] = 1 / max(delta_s lambda_i + 1, 1e-12), and one thread per
 // column advances its search (golden section, Newton) between rounds; the
 // grid phase, whose deltas every column shares, runs once before them.
-enum : int { kRbGolden = 1, kRbCentre, kRbNewtonPair, kRbNewtonStep, kRbFinal, kRbDone };
+enum : int { kRbGolden = 1, kRbCentre, kRbNewtonPair, kRbNewtonStep, kRbFinal };
 constexpr int kRbGridN = 35;  // f(1.0), then 1e-5 * 2^k for k = 0..33 (the loop dd <= 1e5, dd *= 2)
 constexpr int kRbMaxRounds = 40 + 1 + 2 * 8 + 1;  // golden, centre, Newton, final
 
@@ -442,40 +442,130 @@ __global__ void rb_grid_weights_kernel(const double* __restrict__ Xtil, const do
   }
 }
 
-// Lg[k] = Cholesky factor of X~'D_k X~ (row-major, lower), ldx[k] its log
-// determinant, or ldx[k] = NaN when it is not positive definite.
-__global__ void rb_grid_chol_kernel(const double* __restrict__ Ag, int p, double* Lg, double* ldx) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= kRbGridN) return;
-  const int nq = p * (p + 1) / 2;
-  double* L = Lg + static_cast<int64_t>(k) * p * p;
-  const double* Ac = Ag + static_cast<int64_t>(k) * nq;
-  double ld = 0.0;
-  for (int j = 0; j < p; ++j) {
-    double d = Ac[tri(j, j, p)];
-    for (int q = 0; q < j; ++q) d -= L[j * p + q] * L[j * p + q];
-    if (!(d > 0)) {
-      ldx[k] = CUDART_NAN;
-      return;
-    }
-    L[j * p + j] = sqrt(d);
-    ld += 2.0 * log(L[j * p + j]);
-    for (int i = j + 1; i < p; ++i) {
-      double v = Ac[tri(j, i, p)];
-      for (int q = 0; q < j; ++q) v -= L[i * p + q] * L[j * p + q];
-      L[i * p + j] = v / L[j * p + j];
-    }
-  }
-  ldx[k] = ld;
+// ---- one p x p factorisation per group of GW lanes (GW = 8, 16 or 32, p <= GW)
+// One thread per column used to factorise and solve alone: at p = 16 that is
+// a chain of ~1,500 dependent FP64 operations on local memory, 325 us a round
+// whatever the number of columns (72 % of a 500-column cis scan's device
+// time). Here lane i of the group holds row i in registers and the updates of
+// a step run across the lanes; every element still sees the same operations
+// in the same order (column k of the factor is subtracted before column
+// k + 1), so each factor, solution and -loglik keeps its bits.
+// Measured at n = 1000, p = 16: the null fits of 500 columns 18.3 -> 3.7 ms, of
+// 8,000 columns 39.7 -> 22.3 ms (this kernel 55 us a round there).
+template <int GW>
+__device__ __forceinline__ double rb_shfl(double v, int src) {
+  return __shfl_sync(0xffffffffu, v, src, GW);
 }
 
-// Per column: the 35 grid -logliks in the reference's order (f(1.0) first,
-// strict <), then the golden-section bracket; proposes the first round.
+// Lower Cholesky factor of the SPD matrix whose packed upper triangle is A
+// (tri order) and, in the same sweep, the forward solve L y = b (b == null:
+// not wanted): on return row[c] = L[gl][c] (c <= gl) in lane gl, diag = L[gl][gl],
+// y = y[gl], *logdet = log det A. Lanes gl >= p carry an identity. Returns
+// false (to the whole group) where a pivot is not positive; the values are
+// then meaningless. Every lane of the warp takes part.
+template <int GW>
+__device__ __forceinline__ bool rb_factor(const double* __restrict__ A, const double* __restrict__ b, int p, int gl,
+                                          double (&row)[GW], double& diag, double& y, double* logdet) {
+#pragma unroll
+  for (int c = 0; c < GW; ++c) row[c] = gl < p && c <= gl ? A[tri(c, gl, p)] : (c == gl ? 1.0 : 0.0);
+  y = b && gl < p ? b[gl] : 0.0;
+  diag = 1.0;
+  bool ok = true;
+#pragma unroll
+  for (int j = 0; j < GW; ++j) {
+    if (j < p) {  // uniform across the launch
+      const double d = rb_shfl<GW>(row[j], j);
+      ok = ok && d > 0;
+      const double ljj = sqrt(d);
+      const double lij = gl == j ? ljj : row[j] / ljj;
+      const double yj = rb_shfl<GW>(y, j) / ljj;
+      row[j] = lij;
+      if (gl == j) {
+        diag = ljj;
+        y = yj;
+      }
+      if (gl > j) y = fma(-lij, yj, y);
+#pragma unroll
+      for (int c = j + 1; c < GW; ++c)
+        if (c < p) {
+          const double lcj = rb_shfl<GW>(lij, c);
+          if (gl >= c) row[c] = fma(-lij, lcj, row[c]);
+        }
+    }
+  }
+  const double lg = log(diag);
+  double ld = 0.0;
+#pragma unroll
+  for (int j = 0; j < GW; ++j)
+    if (j < p) ld += 2.0 * rb_shfl<GW>(lg, j);
+  *logdet = ld;
+  return ok;
+}
+
+// Lg[k] = Cholesky factor of X~'D_k X~ (row-major, lower), ldx[k] its log
+// determinant, or ldx[k] = NaN when it is not positive definite. One group of
+// GW lanes per grid point.
+template <int GW>
+__global__ void __launch_bounds__(128) rb_grid_chol_kernel(const double* __restrict__ Ag, int p, double* Lg,
+                                                           double* ldx) {
+  const int k0 = (blockIdx.x * blockDim.x + threadIdx.x) / GW;
+  const int gl = threadIdx.x % GW;
+  const int k = min(k0, kRbGridN - 1);  // spare groups repeat the last point and write nothing
+  const int nq = p * (p + 1) / 2;
+  double row[GW], diag, y, ld;
+  const bool ok = rb_factor<GW>(Ag + static_cast<int64_t>(k) * nq, nullptr, p, gl, row, diag, y, &ld);
+  if (k0 >= kRbGridN) return;
+  double* L = Lg + static_cast<int64_t>(k) * p * p;
+  if (gl < p) {
+#pragma unroll
+    for (int c = 0; c < GW; ++c)
+      if (c <= gl) L[gl * p + c] = row[c];
+  }
+  if (gl == 0) ldx[k] = ok ? ld : CUDART_NAN;
+}
+
+// -loglik of every column at grid point k = blockIdx.y into V[k C + c] (one
+// thread per column and grid point: the 35 forward solves of a column used to
+// run one after the other in one thread, 514 us at 500 columns; the factor is
+// read from shared memory).
 // Bg[(k p + a) + 35 p c] = x~_a' D_k y_c, Yg[k + 35 c] = y_c' D_k y_c.
-__global__ void rb_grid_advance_kernel(int C, int p, int df, const double* __restrict__ Lg,
-                                       const double* __restrict__ ldx, const double* __restrict__ ldD,
-                                       const double* __restrict__ Bg, const double* __restrict__ Yg,
-                                       RemlBatchState* st, double* dlt) {
+template <int GW>
+__global__ void __launch_bounds__(128)
+    rb_grid_eval_kernel(int C, int p, int df, const double* __restrict__ Lg, const double* __restrict__ ldx,
+                        const double* __restrict__ ldD, const double* __restrict__ Bg,
+                        const double* __restrict__ Yg, double* V) {
+  __shared__ double L[GW * GW];
+  const int k = blockIdx.y;
+  for (int e = threadIdx.x; e < p * p; e += blockDim.x) L[e] = Lg[static_cast<int64_t>(k) * p * p + e];
+  __syncthreads();
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= C) return;
+  double v = 1e300;
+  const double lx = ldx[k];
+  if (lx == lx) {
+    const double dfd = static_cast<double>(df);
+    const double* b = Bg + static_cast<int64_t>(kRbGridN) * p * c + static_cast<int64_t>(k) * p;
+    double z[GW];
+    double q = Yg[k + static_cast<int64_t>(kRbGridN) * c];
+#pragma unroll
+    for (int i = 0; i < GW; ++i)
+      if (i < p) {
+        double t = b[i];
+#pragma unroll
+        for (int j = 0; j < i; ++j) t -= L[i * p + j] * z[j];
+        z[i] = t / L[i * p + i];
+        q -= z[i] * z[i];
+      }
+    if (q <= 0) q = 1e-12;
+    v = 0.5 * (dfd * log(q / dfd) + ldD[k] + lx);
+  }
+  V[static_cast<int64_t>(k) * C + c] = v;
+}
+
+// Per column: the best of the 35 grid -logliks in the reference's order
+// (f(1.0) first, strict <), then the golden-section bracket; proposes the
+// first round.
+__global__ void rb_grid_advance_kernel(int C, int df, const double* __restrict__ V, RemlBatchState* st, double* dlt) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= C) return;
   RemlBatchState s{};
@@ -483,24 +573,8 @@ __global__ void rb_grid_advance_kernel(int C, int p, int df, const double* __res
   if (df <= 0) {
     s.phase = kRbFinal;
   } else {
-    const double dfd = static_cast<double>(df);
     for (int k = 0; k < kRbGridN; ++k) {
-      double v = 1e300;
-      const double lx = ldx[k];
-      if (lx == lx) {
-        const double* L = Lg + static_cast<int64_t>(k) * p * p;
-        const double* b = Bg + static_cast<int64_t>(kRbGridN) * p * c + static_cast<int64_t>(k) * p;
-        double z[kMaxPLmm];
-        double q = Yg[k + static_cast<int64_t>(kRbGridN) * c];
-        for (int i = 0; i < p; ++i) {
-          double t = b[i];
-          for (int j = 0; j < i; ++j) t -= L[i * p + j] * z[j];
-          z[i] = t / L[i * p + i];
-          q -= z[i] * z[i];
-        }
-        if (q <= 0) q = 1e-12;
-        v = 0.5 * (dfd * log(q / dfd) + ldD[k] + lx);
-      }
+      const double v = V[static_cast<int64_t>(k) * C + c];
       if (k == 0) {
         s.best_ll = v;
         s.best_d = 1.0;
@@ -520,7 +594,10 @@ __global__ void rb_grid_advance_kernel(int C, int p, int df, const double* __res
 }
 
 // One warp per slot: W, W o y, sum log v (log of eight-factor products, as in
-// reml_eval_warp) and y'Dy. Slots with no delta (NaN) are skipped.
+// reml_eval_warp) and y'Dy. Slots with no delta (NaN) are skipped. Bound by the
+// latency of the FP64 reciprocals and loads when the columns are few, so a
+// lane takes eight of its samples per step, whose reciprocals overlap; the
+// sums keep each lane's sample order.
 __global__ void __launch_bounds__(256) rb_weights_kernel(const double* __restrict__ Ytil,
                                                          const double* __restrict__ lam, int n, int C,
                                                          const double* __restrict__ dlt, double* W, double* WY,
@@ -535,7 +612,47 @@ __global__ void __launch_bounds__(256) rb_weights_kernel(const double* __restric
   double* wy_out = WY + static_cast<int64_t>(s) * n;
   double acc_ld = 0.0, acc_y = 0.0, prod = 1.0;
   int nprod = 0;
-  for (int i = lane; i < n; i += 32) {
+  int i = lane;
+  for (; i + 7 * 32 < n; i += 8 * 32) {
+    double v[8], yi[8];
+    bool in = nprod == 0;
+#pragma unroll
+    for (int t = 0; t < 8; ++t) {
+      v[t] = delta * lam[i + 32 * t] + 1.0;
+      yi[t] = y[i + 32 * t];
+    }
+#pragma unroll
+    for (int t = 0; t < 8; ++t) {
+      if (v[t] < 1e-12) v[t] = 1e-12;
+      in = in && v[t] <= 1e36;
+      const double w = 1.0 / v[t];
+      w_out[i + 32 * t] = w;
+      wy_out[i + 32 * t] = w * yi[t];
+      acc_y += w * yi[t] * yi[t];
+    }
+    if (in) {  // eight factors of one product, whose log is due
+#pragma unroll
+      for (int t = 0; t < 8; ++t) prod *= v[t];
+      acc_ld += log(prod);
+      prod = 1.0;
+      continue;
+    }
+    for (int t = 0; t < 8; ++t) {  // a factor above 1e36 takes its own log
+      double u = delta * lam[i + 32 * t] + 1.0;
+      if (u < 1e-12) u = 1e-12;
+      if (u <= 1e36) {
+        prod *= u;
+        if (++nprod == 8) {
+          acc_ld += log(prod);
+          prod = 1.0;
+          nprod = 0;
+        }
+      } else {
+        acc_ld += log(u);
+      }
+    }
+  }
+  for (; i < n; i += 32) {
     double v = delta * lam[i] + 1.0;
     if (v < 1e-12) v = 1e-12;
     const double w = 1.0 / v;
@@ -565,51 +682,77 @@ __global__ void __launch_bounds__(256) rb_weights_kernel(const double* __restric
   }
 }
 
-// -loglik of slot s from its sums; A is unpacked into Af (p x p, row-major).
-__device__ double rb_negll(const double* __restrict__ Acol, const double* __restrict__ bcol, double y_dy,
-                           double logdet_d, int p, int df, double* Af, double* L) {
-  for (int a = 0; a < p; ++a)
-    for (int b = a; b < p; ++b) Af[a * p + b] = Af[b * p + a] = Acol[tri(a, b, p)];
-  double beta[kMaxPLmm];
-  double logdet_x = 0.0;
-  if (!chol_solve(Af, bcol, beta, &logdet_x, p, L)) return 1e300;
-  double q = y_dy;
-  for (int k = 0; k < p; ++k) q -= bcol[k] * beta[k];
-  if (q <= 0) q = 1e-12;
-  const double dfd = static_cast<double>(df);
-  return 0.5 * (dfd * log(q / dfd) + logdet_d + logdet_x);
+// L (row stride GW + 1) of this group in shared memory, and beta = (L L')^-1 b
+// from y = L^-1 b: every lane of the group runs the same back substitution,
+// each element's terms in increasing order, as chol_solve does.
+template <int GW>
+__device__ __forceinline__ void rb_back_solve(const double (&row)[GW], double y, int p, int gl, double* L,
+                                              double (&beta)[GW]) {
+#pragma unroll
+  for (int c = 0; c < GW; ++c) L[gl * (GW + 1) + c] = row[c];
+  __syncwarp();
+#pragma unroll
+  for (int i = GW - 1; i >= 0; --i) {
+    const double yi = rb_shfl<GW>(y, i);
+    beta[i] = 0.0;
+    if (i < p) {
+      double s = yi;
+#pragma unroll
+      for (int k = i + 1; k < GW; ++k)
+        if (k < p) s -= L[k * (GW + 1) + i] * beta[k];
+      beta[i] = s / L[i * (GW + 1) + i];
+    }
+  }
 }
 
-// One thread per column: reads the round's -loglik values, advances the
-// search exactly as optimize_delta_dev does, and proposes the next round's
-// deltas; in the final round writes delta and the prep_lmm caches.
-// PMAX bounds p for the per-thread p x p scratch (p <= 16 keeps the stack
-// frame small; 17..32 use the larger instance).
-template <int PMAX>
-__global__ void rb_advance_kernel(int C, int g0, int p, int df, const double* __restrict__ A,
-                                  const double* __restrict__ B, const double* __restrict__ ld,
-                                  const double* __restrict__ ydy, RemlBatchState* st, double* dlt,
-                                  unsigned int* active, double* delta_out, double* chi0_out, double* ainv_out,
-                                  double* rss_out, double* a00L_out) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= C) return;
-  RemlBatchState s = st[c];
-  if (s.phase == kRbDone) return;
+constexpr int kRbThreads = 128;
+
+// Two groups of GW lanes per column, one per slot, evaluate the round's
+// -logliks; one lane then advances the search exactly as optimize_delta_dev
+// does and proposes the next round's deltas. A column whose search has ended
+// keeps proposing its delta (kRbFinal) until every column's has: the caches are
+// formed for all of them at once (rb_final_kernel). *active counts the
+// columns still searching.
+template <int GW>
+__global__ void __launch_bounds__(kRbThreads)
+    rb_advance_kernel(int C, int p, int df, const double* __restrict__ A, const double* __restrict__ B,
+                      const double* __restrict__ ld, const double* __restrict__ ydy, RemlBatchState* st, double* dlt,
+                      unsigned int* active) {
+  constexpr int kGroups = kRbThreads / GW;
+  __shared__ double Ls[kGroups * GW * (GW + 1)];
+  __shared__ double val[kGroups];
+  const int grp = threadIdx.x / GW, gl = threadIdx.x % GW;
+  const int slot = grp & 1;
+  const int c0 = blockIdx.x * (kGroups / 2) + (grp >> 1);
+  const int c = min(c0, C - 1);  // spare groups repeat the last column and write nothing
   const int nq = p * (p + 1) / 2;
-  double Af[PMAX * PMAX], L[PMAX * PMAX];
-  auto f = [&](int slot) {
-    const int si = slot * C + c;
-    return rb_negll(A + static_cast<int64_t>(si) * nq, B + static_cast<int64_t>(si) * p, ydy[si], ld[si], p, df,
-                    Af, L);
-  };
+  const int si = slot * C + c;
+  // a slot without a delta this round holds an earlier round's sums; its value
+  // is not read
+  const double* b = B + static_cast<int64_t>(si) * p;
+  double row[GW], beta[GW], diag, y, logdet_x;
+  const bool ok = rb_factor<GW>(A + static_cast<int64_t>(si) * nq, b, p, gl, row, diag, y, &logdet_x);
+  rb_back_solve<GW>(row, y, p, gl, Ls + grp * GW * (GW + 1), beta);
+  if (gl == 0) {
+    double q = ydy[si];
+#pragma unroll
+    for (int k = 0; k < GW; ++k)
+      if (k < p) q -= b[k] * beta[k];
+    if (q <= 0) q = 1e-12;
+    const double dfd = static_cast<double>(df);
+    val[grp] = ok ? 0.5 * (dfd * log(q / dfd) + ld[si] + logdet_x) : 1e300;
+  }
+  __syncthreads();
+  if (gl != 0 || slot != 0 || c0 >= C) return;
+  RemlBatchState s = st[c];
+  if (s.phase == kRbFinal) return;
+  const double f0 = val[grp], f1 = val[grp + 1];
   switch (s.phase) {
     case kRbGolden: {
       const double phi = (1.0 + sqrt(5.0)) / 2.0;
       const double m1 = s.hi - (s.hi - s.lo) / phi;
       const double m2 = s.lo + (s.hi - s.lo) / phi;
-      const double f1 = f(0);
-      const double f2 = f(1);
-      if (f1 < f2) s.hi = m2;
+      if (f0 < f1) s.hi = m2;
       else s.lo = m1;
       if (++s.k == 40) {
         s.d = 0.5 * (s.lo + s.hi);
@@ -618,14 +761,14 @@ __global__ void rb_advance_kernel(int C, int g0, int p, int df, const double* __
       break;
     }
     case kRbCentre:
-      s.cur = f(0);
+      s.cur = f0;
       s.k = 0;
       s.h = fmax(s.d * 1e-4, 1e-9);
       s.phase = kRbNewtonPair;
       break;
     case kRbNewtonPair: {
-      const double fm = f(0);
-      const double fp = f(1);
+      const double fm = f0;
+      const double fp = f1;
       const double g1 = (fp - fm) / (2.0 * s.h);
       const double g2 = (fp - 2.0 * s.cur + fm) / (s.h * s.h);
       s.phase = kRbFinal;
@@ -637,7 +780,7 @@ __global__ void rb_advance_kernel(int C, int g0, int p, int df, const double* __
       break;
     }
     case kRbNewtonStep: {
-      const double vn = f(0);
+      const double vn = f0;
       s.phase = kRbFinal;
       if (vn < s.cur) {
         s.d = s.dn;
@@ -649,24 +792,76 @@ __global__ void rb_advance_kernel(int C, int g0, int p, int df, const double* __
       }
       break;
     }
-    case kRbFinal: {
-      const int si = c;  // slot 0
-      const double* Acol = A + static_cast<int64_t>(si) * nq;
-      for (int a = 0; a < p; ++a)
-        for (int b = a; b < p; ++b) Af[a * p + b] = Af[b * p + a] = Acol[tri(a, b, p)];
-      double e[kMaxPLmm], x[kMaxPLmm];
-      delta_out[g0 + c] = s.d;
-      reml_caches(Af, B + static_cast<int64_t>(si) * p, ydy[si], p, g0 + c, L, e, x, chi0_out, ainv_out, rss_out,
-                  a00L_out);
-      s.phase = kRbDone;
-      break;
-    }
     default:
       break;
   }
   st[c] = s;
   rb_propose(s, dlt[c], dlt[C + c]);
-  if (s.phase != kRbDone) atomicAdd(active, 1u);
+  if (s.phase != kRbFinal) atomicAdd(active, 1u);
+}
+
+// After the last round, whose slot 0 holds every column's sums at its final
+// delta: delta and the prep_lmm caches (reml_caches) with one group of GW lanes
+// per column; lane k solves column k of A00^-1.
+template <int GW>
+__global__ void __launch_bounds__(kRbThreads)
+    rb_final_kernel(int C, int g0, int p, const double* __restrict__ A, const double* __restrict__ B,
+                    const double* __restrict__ ydy, const RemlBatchState* __restrict__ st, double* delta_out,
+                    double* chi0_out, double* ainv_out, double* rss_out, double* a00L_out) {
+  constexpr int kGroups = kRbThreads / GW;
+  __shared__ double Ls[kGroups * GW * (GW + 1)];
+  const int grp = threadIdx.x / GW, gl = threadIdx.x % GW;
+  const int c0 = blockIdx.x * kGroups + grp;
+  const int c = min(c0, C - 1);
+  const int nq = p * (p + 1) / 2;
+  const double* b = B + static_cast<int64_t>(c) * p;
+  double row[GW], beta[GW], diag, y, logdet_x;
+  const bool ok = rb_factor<GW>(A + static_cast<int64_t>(c) * nq, b, p, gl, row, diag, y, &logdet_x);
+  double* L = Ls + grp * GW * (GW + 1);
+  rb_back_solve<GW>(row, y, p, gl, L, beta);
+  if (c0 >= C || gl >= p) return;
+  const int64_t g = g0 + c;
+  // column gl of A00^-1: L y = e_gl, then L' x = y
+  double x[GW];
+#pragma unroll
+  for (int i = 0; i < GW; ++i) {
+    x[i] = 0.0;
+    if (i < p) {
+      double s = i == gl ? 1.0 : 0.0;
+#pragma unroll
+      for (int k = 0; k < i; ++k) s -= L[i * (GW + 1) + k] * x[k];
+      x[i] = s / L[i * (GW + 1) + i];
+    }
+  }
+#pragma unroll
+  for (int i = GW - 1; i >= 0; --i)
+    if (i < p) {
+      double s = x[i];
+#pragma unroll
+      for (int k = i + 1; k < GW; ++k)
+        if (k < p) s -= L[k * (GW + 1) + i] * x[k];
+      x[i] = s / L[i * (GW + 1) + i];
+    }
+#pragma unroll
+  for (int i = 0; i < GW; ++i)
+    if (i < p) {
+      ainv_out[(g * p + i) * p + gl] = ok ? x[i] : 0.0;
+      a00L_out[(g * p + gl) * p + i] = ok && i <= gl ? row[i] : 0.0;
+    }
+  if (gl == 0) {
+    double rss = ydy[c];
+    if (ok) {
+#pragma unroll
+      for (int k = 0; k < GW; ++k)
+        if (k < p) rss -= b[k] * beta[k];
+      if (rss < 0) rss = 0;
+    }
+    rss_out[g] = rss;
+    delta_out[g] = st[c].d;
+#pragma unroll
+    for (int k = 0; k < GW; ++k)
+      if (k < p) chi0_out[g * p + k] = ok ? beta[k] : 0.0;
+  }
 }
 
 // Gene-side operands, one block per gene: rows (w o r~), (w o X~_k), w, each
@@ -1808,6 +2003,7 @@ __global__ void square_kernel(const double* __restrict__ x, int64_t count, doubl
 
 // Batched REML for p > kRemlWarpP over ws.Ytil / ws.Xtil into ws.delta,
 // chi0, ainv, rss: columns in chunks whose per-round buffers stay near 2 GB.
+template <int GW>
 static void reml_batched(eqtl_ctx* ctx, int n, int p, int G) {
   Workspace& ws = ctx->ws;
   cudaStream_t st = ctx->stream;
@@ -1835,7 +2031,7 @@ static void reml_batched(eqtl_ctx* ctx, int n, int p, int G) {
     EQTL_CHECK(cublasDgemm(h, CUBLAS_OP_N, CUBLAS_OP_N, nq, K, n, &one, ws.rb_P.p, nq, ws.rb_Wg.p, n, &zero,
                            ws.rb_Ag.p, nq) == CUBLAS_STATUS_SUCCESS,
                EQTL_E_CUDA, "REML grid X'DX failed");
-    rb_grid_chol_kernel<<<1, 64, 0, st>>>(ws.rb_Ag.p, p, ws.rb_Lg.p, ws.rb_ldx.p);
+    rb_grid_chol_kernel<GW><<<(K * GW + 127) / 128, 128, 0, st>>>(ws.rb_Ag.p, p, ws.rb_Lg.p, ws.rb_ldx.p);
     EQTL_CUDA(cudaGetLastError());
   }
   const int cmax = std::max(1024, static_cast<int>((int64_t(1) << 26) / std::max(n, 1)));
@@ -1870,13 +2066,16 @@ static void reml_batched(eqtl_ctx* ctx, int n, int p, int G) {
       EQTL_CHECK(cublasDgemm(h, CUBLAS_OP_T, CUBLAS_OP_N, K, C, n, &one, ws.rb_Wg.p, n, ws.rb_WY.p, n, &zero,
                              ws.rb_Yg.p, K) == CUBLAS_STATUS_SUCCESS,
                  EQTL_E_CUDA, "REML grid y'Dy failed");
-      ++ctx->launches;
-      rb_grid_advance_kernel<<<cblocks, 128, 0, st>>>(C, p, df, ws.rb_Lg.p, ws.rb_ldx.p, ws.rb_ldD.p, ws.rb_Bg.p,
-                                                       ws.rb_Yg.p, state, ws.rb_dlt.p);
+      ctx->launches += 2;
+      ws.rb_V.alloc(static_cast<size_t>(K) * C);
+      rb_grid_eval_kernel<GW><<<dim3(cblocks, K), 128, 0, st>>>(C, p, df, ws.rb_Lg.p, ws.rb_ldx.p, ws.rb_ldD.p,
+                                                                 ws.rb_Bg.p, ws.rb_Yg.p, ws.rb_V.p);
+      rb_grid_advance_kernel<<<cblocks, 128, 0, st>>>(C, df, ws.rb_V.p, state, ws.rb_dlt.p);
       EQTL_CUDA(cudaGetLastError());
     }
-    for (int round = 0; round < kRbMaxRounds; ++round) {
-      ctx->launches += 2;
+    // the sums of every slot's delta
+    auto sums = [&] {
+      ++ctx->launches;
       rb_weights_kernel<<<static_cast<unsigned>((slots + 7) / 8), 256, 0, st>>>(
           Y, ctx->basis.lambda.p, n, C, ws.rb_dlt.p, ws.rb_W.p, ws.rb_WY.p, ws.rb_ld.p, ws.rb_ydy.p);
       EQTL_CUDA(cudaGetLastError());
@@ -1886,14 +2085,17 @@ static void reml_batched(eqtl_ctx* ctx, int n, int p, int G) {
       EQTL_CHECK(cublasDgemm(h, CUBLAS_OP_T, CUBLAS_OP_N, p, static_cast<int>(slots), n, &one, ws.Xtil.p, n,
                              ws.rb_WY.p, n, &zero, ws.rb_B.p, p) == CUBLAS_STATUS_SUCCESS,
                  EQTL_E_CUDA, "REML X'Dy failed");
+    };
+    // the golden phase runs the same number of rounds for every column; from
+    // the Newton phase on, stop once no column is left searching
+    for (int round = 0; df > 0 && round < kRbMaxRounds - 1; ++round) {
+      sums();
+      ++ctx->launches;
       EQTL_CUDA(cudaMemsetAsync(ws.rb_active.p, 0, sizeof(unsigned int), st));
-      auto advance = p <= 16 ? rb_advance_kernel<16> : rb_advance_kernel<kMaxPLmm>;
-      advance<<<cblocks, 128, 0, st>>>(C, g0, p, df, ws.rb_A.p, ws.rb_B.p, ws.rb_ld.p, ws.rb_ydy.p, state,
-                                       ws.rb_dlt.p, ws.rb_active.p, ws.delta.p, ws.chi0.p, ws.ainv.p, ws.rss.p,
-                                       ws.a00L.p);
+      constexpr int kCols = kRbThreads / GW / 2;
+      rb_advance_kernel<GW><<<static_cast<unsigned>((C + kCols - 1) / kCols), kRbThreads, 0, st>>>(
+          C, p, df, ws.rb_A.p, ws.rb_B.p, ws.rb_ld.p, ws.rb_ydy.p, state, ws.rb_dlt.p, ws.rb_active.p);
       EQTL_CUDA(cudaGetLastError());
-      // the golden phase runs the same number of rounds for every column;
-      // from the Newton phase on, stop once no column is left
       if (round >= 40) {
         unsigned int left = 0;
         ws.rb_active.download(&left, 1, st);
@@ -1901,6 +2103,12 @@ static void reml_batched(eqtl_ctx* ctx, int n, int p, int G) {
         if (left == 0) break;
       }
     }
+    sums();
+    ++ctx->launches;
+    constexpr int kGroups = kRbThreads / GW;
+    rb_final_kernel<GW><<<static_cast<unsigned>((C + kGroups - 1) / kGroups), kRbThreads, 0, st>>>(
+        C, g0, p, ws.rb_A.p, ws.rb_B.p, ws.rb_ydy.p, state, ws.delta.p, ws.chi0.p, ws.ainv.p, ws.rss.p, ws.a00L.p);
+    EQTL_CUDA(cudaGetLastError());
   }
 }
 
@@ -1942,7 +2150,10 @@ void lmm_prep(eqtl_ctx* ctx, const PhenoDev& ph, bool y_rotated) {
     EQTL_CUDA(cudaGetLastError());
     return;
   }
-  reml_batched(ctx, n, p, G);
+  // lanes per factorisation: the smallest group that holds p rows
+  if (p <= 8) reml_batched<8>(ctx, n, p, G);
+  else if (p <= 16) reml_batched<16>(ctx, n, p, G);
+  else reml_batched<kMaxPLmm>(ctx, n, p, G);
 }
 
 // ------------------------------------------------------------------- scan
