@@ -50,6 +50,8 @@ struct GeneAcc {
   float chunk_acat = 0.0f;
   float chunk_key = -1.0f;
   uint32_t chunk_snp = 0;
+  // no pair with u below this can be the gene's best (screen16_fast)
+  float u_floor = 0.0f;
   int chrom = -1;
   int64_t lo = 0, hi = -1;
 
@@ -60,6 +62,11 @@ struct GeneAcc {
     best = ~0ull;
     chunk_acat = 0.0f;
     chunk_key = -1.0f;
+  }
+  // Starts from the best that any block has published for the gene (a stale
+  // one is only a lower floor).
+  __device__ __forceinline__ void load_best(const GeneOut& out, int g) {
+    u_floor = __uint_as_float(~static_cast<uint32_t>(__ldcg(out.best + g) >> 32));
   }
   __device__ __forceinline__ void load_window(const Windows& w, int g) {
     if (w.mode != kWinNone) {
@@ -223,6 +230,60 @@ __device__ __forceinline__ void screen16_cubic(const TTable& tt, const float (&u
     acc.chunk_snp = static_cast<uint32_t>(s0 + bj);
   }
   acc.end_chunk();
+}
+
+// The same screen of 16 pairs that are all tested (no SNP of the block gated,
+// none out of scope), for tables in shared memory: u_of(j) gives u = t^2 of
+// pair j, computed without the guards of the general form. Returns false,
+// with acc untouched, unless every u lies in [u_tiny, u_hi), u_hi =
+// min(u_cand, u_defer): a pair near 0, a candidate, a NaN, and whatever the
+// guards would have caught (a vanishing denominator gives u < 0, NaN or inf)
+// are left to the general form.
+//
+// The scans' epilogues are bound by instruction issue, and ~97 % of the
+// 16-pair chunks hold nothing but ordinary pairs, so the per-pair flags, the
+// candidate test, the counts and the best-SNP index leave the loop: the counts
+// are 16, the extremes decide for the chunk, and the index is looked for only
+// where the chunk's largest u reaches the best published for the gene. The
+// terms and the order of their sum are those of screen16_cubic.
+template <class U>
+__device__ __forceinline__ bool screen16_fast(const TTable& tt, uint32_t tab, float u_hi, U&& u_of, int64_t s0,
+                                              GeneAcc& acc) {
+  float sum = 0.0f, umin = INFINITY, umax = 0.0f;
+#pragma unroll
+  for (int j = 0; j < 16; j += 2) {
+    const float ua = u_of(j), ub = u_of(j + 1);
+    umin = min3(umin, ua, ub);
+    umax = max3_nan(umax, ua, ub);
+    sum += cubic_term(ua, tt, tab);
+    sum += cubic_term(ub, tt, tab);
+  }
+  if (!(umin >= tt.u_tiny && umax < u_hi)) return false;
+  acc.tested += 16;
+  acc.used += 16;
+  acc.acat += static_cast<double>(sum);
+  if (umax >= acc.u_floor) {
+    uint32_t bj = 0;
+#pragma unroll
+    for (int j = 15; j >= 0; --j) bj = u_of(j) == umax ? j : bj;  // the first pair with the largest u
+    const unsigned long long k = best_key(umax, static_cast<uint32_t>(s0) + bj);
+    acc.best = k < acc.best ? k : acc.best;
+    acc.u_floor = umax;
+  }
+  return true;
+}
+
+// Whether all 16 flag bytes (0 or 1) are set.
+__device__ __forceinline__ bool all_flags16(const uint32_t (&w)[4]) {
+  return (w[0] & w[1] & w[2] & w[3]) == 0x01010101u;
+}
+
+// Whether every pair of the block of 16 SNPs at s0 is in scope for every gene
+// of the warp's active lanes: a gw scan, or a trans scan on a block clear of
+// all their windows (the vote keeps the warp on one path).
+__device__ __forceinline__ bool chunk_in_scope(const Windows& w, const GeneAcc& acc, int64_t s0) {
+  if (w.mode == kWinNone) return true;
+  return w.mode == kWinExclude && __all_sync(__activemask(), acc.chunk_clear(w, s0));
 }
 
 }  // namespace dev

@@ -58,12 +58,14 @@ struct LmEpi {
   bool gvalid = false;
   float w = 0;   // gscale^2 / yty
   float u_cand;  // t_cand^2
+  uint32_t tab = 0;  // cubic_base of the tables in shared memory
   GeneAcc acc;
 
   __device__ LmEpi(const Params& p, const TileShape&, uint8_t* smem)
       : P(p), tsm(reinterpret_cast<float*>(smem)), tt(p.tt), u_cand(p.t_cand * p.t_cand) {}
   __device__ void init(int tid, int nthr) {
-    if (tsm) tt = screen_to_smem(P.tt, tsm, tid, nthr);
+    tt = screen_to_smem(P.tt, tsm, tid, nthr);
+    tab = cubic_base(smem_u32(tsm));
   }
   __device__ void begin_tile(int g, int64_t s0) {
     gene = g;
@@ -74,6 +76,7 @@ struct LmEpi {
       const float gs = P.gscale[g];
       w = gs * gs * static_cast<float>(P.inv_yty[g]);
       acc.load_window(P.win, g);
+      acc.load_best(P.out, g);
     }
   }
   // t^2 = df r / (1 - r), r = gty^2 / (gtg yty) = acc^2 (a^2 / gtg) (gscale^2 / yty)
@@ -95,15 +98,19 @@ struct LmEpi {
       igv[4 * q + 3] = v4.w;
     }
     if (tt.lt_u) {  // uniform across the launch
-      // a gw scan (no windows), and a trans scan on a chunk clear of every
-      // lane's gene window, skip the per-pair window test; the vote keeps
-      // the warp on one path
-      if (P.win.mode == kWinNone)
-        chunk_cubic<false>(s0, v[0], igv);
-      else if (P.win.mode == kWinExclude && __all_sync(__activemask(), acc.chunk_clear(P.win, s0)))
-        chunk_cubic<false>(s0, v[0], igv);
-      else
-        chunk_cubic<true>(s0, v[0], igv);
+      float ig_min = igv[0];
+#pragma unroll
+      for (int j = 1; j < 15; j += 2) ig_min = min3(ig_min, igv[j], igv[j + 1]);
+      ig_min = fminf(ig_min, igv[15]);
+      // every SNP tested and with a residual variance, every pair in scope
+      if (ig_min > 0.0f && chunk_in_scope(P.win, acc, s0)) {
+        auto u_of = [&](int j) {
+          const float r = v[0][j] * v[0][j] * (igv[j] * w);
+          return P.df * (r * rcp_ftz(1.0f - r));
+        };
+        if (screen16_fast(P.tt, tab, fminf(u_cand, P.tt.u_defer), u_of, s0, acc)) return;
+      }
+      chunk_cubic(s0, v[0], igv);
       return;
     }
 #pragma unroll
@@ -122,13 +129,12 @@ struct LmEpi {
   }
   // The same screen with the per-interval cubics (screen16_cubic): u is
   // never NaN here (a pair outside the scan or with p = 1 has u = 0).
-  template <bool WIN>
   __device__ void chunk_cubic(int64_t s0, const float (&v)[16], const float (&igv)[16]) {
     float u[16];
     bool valid[16];
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
-      valid[j] = igv[j] >= 0.0f && (!WIN || acc.in_scope(P.win, s0 + j));
+      valid[j] = igv[j] >= 0.0f && acc.in_scope(P.win, s0 + j);
       const float ig = valid[j] ? igv[j] * w : 0.0f;
       const float r = v[j] * v[j] * ig;
       const float omr = 1.0f - r;

@@ -24,7 +24,9 @@ constexpr int kTTableNa = 512;   // central intervals (TTableHost::na)
 constexpr int kTTableNb = 4096;  // tail intervals (TTableHost::nb)
 constexpr int kTTableNq = 1024;  // tail intervals of the per-interval cubics (TTableHost::nq)
 constexpr int kTTableNodeBytes = (kTTableNa + 4 + kTTableNb + 4) * 4;
-constexpr int kTTableCubicBytes = (kTTableNa + kTTableNq) * 16;
+// one entry more after each region: a value that rounds onto the region's end
+// still reads an entry of it
+constexpr int kTTableCubicBytes = (kTTableNa + 1 + kTTableNq + 1) * 16;
 constexpr int kTTableSmemBytes = kTTableNodeBytes > kTTableCubicBytes ? kTTableNodeBytes : kTTableCubicBytes;
 
 struct TTable {
@@ -188,6 +190,11 @@ __device__ __forceinline__ ScreenOut acat_screen(float t, const TTable& T) {
   return o;
 }
 
+// the constant that continues an interval's cubic past its end
+__device__ __forceinline__ float4 cubic_end(const float4& a) {
+  return make_float4(((a.w + a.z) + a.y) + a.x, 0.0f, 0.0f, 0.0f);
+}
+
 // Copies the screening tables into shared memory (cooperatively, by `nthr`
 // threads) and returns a view of them; the caller synchronises before use.
 // (With lt_u the per-interval cubics, else the node tables; `sm` 16-byte
@@ -196,10 +203,11 @@ __device__ __forceinline__ TTable screen_to_smem(const TTable& T, float* sm, int
   TTable o = T;
   if (T.lt_u) {
     float4* q = reinterpret_cast<float4*>(sm);
-    for (int i = tid; i < T.na; i += nthr) q[i] = T.c1q[i];
-    for (int i = tid; i < T.nq; i += nthr) q[T.na + i] = T.ltq[i];
+    float4* r = q + T.na + 1;
+    for (int i = tid; i <= T.na; i += nthr) q[i] = i < T.na ? T.c1q[i] : cubic_end(T.c1q[i - 1]);
+    for (int i = tid; i <= T.nq; i += nthr) r[i] = i < T.nq ? T.ltq[i] : cubic_end(T.ltq[i - 1]);
     o.c1q = q;
-    o.ltq = q + T.na;
+    o.ltq = r;
     return o;
   }
   const int nc = T.na + 4, nl = T.nb + 4;
@@ -208,6 +216,54 @@ __device__ __forceinline__ TTable screen_to_smem(const TTable& T, float* sm, int
   o.c1 = sm;
   o.lt = sm + nc;
   return o;
+}
+
+__device__ __forceinline__ float rcp_ftz(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float rsqrt_ftz(float x) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float min3(float a, float b, float c) {
+  float r;
+  asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+// NaN if any of the three is
+__device__ __forceinline__ float max3_nan(float a, float b, float c) {
+  float r;
+  asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+
+// 2^23: adding a float in [0, 2^23) to it, rounding down, leaves the float's
+// integer part in the sum's low bits (no float <-> int conversions, which
+// issue at an eighth of the rate of an add)
+constexpr float kFloorMagic = 8388608.0f;
+
+// Address operand of cubic_term for tables that screen_to_smem laid out at
+// the shared-memory address `sm`.
+__device__ __forceinline__ uint32_t cubic_base(uint32_t sm) { return sm - (0x4B000000u << 4); }
+
+// The ACAT term of one u in [u_tiny, u_defer), as the lt_u branch of
+// acat_screen_u forms it (the same bits; outside that range a meaningless
+// value, without reading past the tables). tab: cubic_base.
+__device__ __forceinline__ float cubic_term(float u, const TTable& T, uint32_t tab) {
+  const float up = fminf(fabsf(u), T.u_defer);  // NaN: u_defer
+  const bool central = up < T.uq0;
+  const float x = central ? up * T.dqc_inv : (up - T.uq0) * T.dq_inv;
+  const float magic = central ? kFloorMagic : kFloorMagic + static_cast<float>(kTTableNa + 1);
+  const float y = __fadd_rd(x, magic);
+  const float f = x - (y - magic);
+  const uint32_t addr = tab + (__float_as_uint(y) << 4);
+  float a0, a1, a2, a3;
+  asm("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(a0), "=f"(a1), "=f"(a2), "=f"(a3) : "r"(addr));
+  const float v = fmaf(fmaf(fmaf(a3, f, a2), f, a1), f, a0);
+  return central ? v * rsqrt_ftz(up) : v;
 }
 
 // Copies the t_tail tables into shared memory (cooperatively, by `nthr`
