@@ -1976,7 +1976,10 @@ void lmm_rotate(eqtl_ctx* ctx) {
     const __half* bh[1] = {g.gc_hi.p};
     const __half* bl[1] = {g.gc_lo.p};
     const int bsel[1] = {0}, prod[1] = {7};
-    launch_tile_n<256, 1>(ctx, bf16, ep, ah, al, n, bh, bl, m, k_pad, bsel, prod);
+    if (!bf16 && tile_pairs(n))
+      launch_tile_n<256, 1, RotEpiParams, dev::kBLoStage, 2>(ctx, false, ep, ah, al, n, bh, bl, m, k_pad, bsel, prod);
+    else
+      launch_tile_n<256, 1>(ctx, bf16, ep, ah, al, n, bh, bl, m, k_pad, bsel, prod);
   }
   if (ctx->precision == EQTL_PREC_FP32_SIMT && m > 0) {
     // the FP32 form keeps its SNP-side operands in FP32

@@ -85,6 +85,16 @@ inline int64_t expected_candidates(const eqtl_scan_params* prm, int64_t m) {
   return static_cast<int64_t>(std::min(e, static_cast<double>(1 << 26)));
 }
 
+// Whether a dense launch over rows_a gene-side rows runs on SM pairs (256-row
+// tiles): an even number of 128-row tiles, or at least seven, where the half
+// tile that an odd number leaves idle costs less than pairing gains (LM scan at
+// n = 1000, 200,000 SNPs and 4,000 genes: 3.3 ms at CG = 1 with the epilogue's
+// chunk form 2.7, here 2.46; rotation of 60,000 SNPs at n = 1,201 0.56 -> 0.50).
+inline bool tile_pairs(int64_t rows_a) {
+  const int64_t t = (rows_a + dev::kTileM - 1) / dev::kTileM;
+  return t % 2 == 0 || t >= 7;
+}
+
 void make_map_2d(CUtensorMap* map, const void* base, uint64_t rows, uint64_t k_pad, uint32_t box_rows, bool bf16);
 int sm_count(eqtl_ctx* ctx);
 
@@ -106,7 +116,9 @@ struct TileK {
 // operands, no product may have bit 2, and more ring stages fit). kc_sub:
 // K chunks per sub-range (0: none; single-group epilogues only). tk:
 // per-accumulator K ranges (TileK; null: every accumulator over all of K).
-template <int NT, int NACC, class EpiParams, int BL = dev::kBLoStage>
+// CG: SMs per tile (tile lists then hold tiles of CG * 128 gene-side rows; FP16
+// only).
+template <int NT, int NACC, class EpiParams, int BL = dev::kBLoStage, int CG = 1>
 void launch_tile_n(eqtl_ctx* ctx, bool bf16, const EpiParams& ep, const __half* const* a_hi,
                    const __half* const* a_lo, int64_t rows_a, const __half* const* b_hi, const __half* const* b_lo,
                    int64_t rows_b, int k_pad, const int* bsel, const int* prod, const int2* tile_list = nullptr,
@@ -121,13 +133,13 @@ namespace eqtl {
 template <class EpiParams>
 struct EpiOf;
 
-template <int NT, int NACC, class EpiParams, int BL>
+template <int NT, int NACC, class EpiParams, int BL, int CG>
 void launch_tile_n(eqtl_ctx* ctx, bool bf16, const EpiParams& ep, const __half* const* a_hi,
                    const __half* const* a_lo, int64_t rows_a, const __half* const* b_hi, const __half* const* b_lo,
                    int64_t rows_b, int k_pad, const int* bsel, const int* prod, const int2* tile_list,
                    int n_tile_list, int ksplit, int n_acc, int kc_sub, const TileK* tk) {
   using Epi = typename EpiOf<EpiParams>::type;
-  using C = dev::TileCfg<NT, NACC, BL>;
+  using C = dev::TileCfg<NT, NACC, BL, CG>;
   dev::TileMaps maps;
   std::memset(&maps, 0, sizeof(maps));
   EQTL_CHECK(n_acc >= 1 && n_acc <= dev::kMaxAcc && (n_acc == NACC || Epi::kGrouped), EQTL_E_INTERNAL,
@@ -141,8 +153,8 @@ void launch_tile_n(eqtl_ctx* ctx, bool bf16, const EpiParams& ep, const __half* 
   for (int j = 0; j < n_acc; ++j) npairs = std::max(npairs, bsel[j] + 1);
   for (int b = 0; b < npairs; ++b) {
     const int kb = tk && tk->k_b[b] > 0 ? tk->k_b[b] : k_pad;
-    make_map_2d(&maps.b[2 * b], b_hi[b], rows_b, kb, NT, bf16);
-    make_map_2d(&maps.b[2 * b + 1], b_lo[b], rows_b, kb, NT, bf16);
+    make_map_2d(&maps.b[2 * b], b_hi[b], rows_b, kb, C::NB, bf16);
+    make_map_2d(&maps.b[2 * b + 1], b_lo[b], rows_b, kb, C::NB, bf16);
   }
   for (int b = npairs; b < 2; ++b) {
     maps.b[2 * b] = maps.b[0];
@@ -173,7 +185,8 @@ void launch_tile_n(eqtl_ctx* ctx, bool bf16, const EpiParams& ep, const __half* 
     EQTL_CHECK(BL != dev::kBLoNone || !(sh.prod[j] & 2), EQTL_E_INTERNAL,
                "tile kernel: hi*lo product without SNP-side lo parts");
   }
-  sh.tiles_a = static_cast<int>((rows_a + dev::kTileM - 1) / dev::kTileM);
+  constexpr int rows_tile = CG * dev::kTileM;
+  sh.tiles_a = static_cast<int>((rows_a + rows_tile - 1) / rows_tile);
   sh.tiles_b = static_cast<int>((rows_b + NT - 1) / NT);
   sh.tile_list = tile_list;
   sh.ksplit = std::max(1, std::min(ksplit, sh.kchunks));
@@ -186,24 +199,37 @@ void launch_tile_n(eqtl_ctx* ctx, bool bf16, const EpiParams& ep, const __half* 
   // gene-side tiles per raster group: keep the group's A operands (hi+lo of
   // every accumulator) within ~48 MB of L2
   {
-    const double a_bytes = static_cast<double>(n_acc) * 2.0 * dev::kTileM * k_pad * 2.0;
+    const double a_bytes = static_cast<double>(n_acc) * 2.0 * rows_tile * k_pad * 2.0;
     sh.group_a = std::max(1, std::min(sh.tiles_a, static_cast<int>(48e6 / a_bytes)));
   }
   sh.status = ctx->d_status;
   if (sh.n_tiles == 0) return;
   EQTL_CUDA(cudaMemsetAsync(ctx->d_status, 0, sizeof(uint32_t), ctx->stream));
-  const int grid = std::min(sh.n_tiles, sm_count(ctx));
+  const int grid = CG * std::min(sh.n_tiles, sm_count(ctx) / CG);
   ++ctx->launches;
   const int smem = C::SMEM_BYTES + Epi::kSmemBytes;
   EQTL_CHECK(smem <= 232448, EQTL_E_INTERNAL, "tile kernel shared memory over the 227 KB limit");
-  if (bf16) {
-    auto kern = dev::tile_kernel<NT, NACC, 1u, Epi, BL>;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(static_cast<unsigned>(grid));
+  cfg.blockDim = dim3(dev::kTileThreads);
+  cfg.dynamicSmemBytes = static_cast<size_t>(smem);
+  cfg.stream = ctx->stream;
+  cudaLaunchAttribute cluster{};
+  cluster.id = cudaLaunchAttributeClusterDimension;
+  cluster.val.clusterDim.x = CG;
+  cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
+  cfg.attrs = &cluster;
+  cfg.numAttrs = CG > 1 ? 1 : 0;
+  auto launch = [&](auto kern) {
     EQTL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    kern<<<grid, dev::kTileThreads, smem, ctx->stream>>>(maps, sh, ep);
+    EQTL_CUDA(cudaLaunchKernelEx(&cfg, kern, maps, sh, ep));
+  };
+  if constexpr (CG == 1) {
+    if (bf16) launch(dev::tile_kernel<NT, NACC, 1u, Epi, BL>);
+    else launch(dev::tile_kernel<NT, NACC, 0u, Epi, BL>);
   } else {
-    auto kern = dev::tile_kernel<NT, NACC, 0u, Epi, BL>;
-    EQTL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    kern<<<grid, dev::kTileThreads, smem, ctx->stream>>>(maps, sh, ep);
+    EQTL_CHECK(!bf16, EQTL_E_INTERNAL, "tile kernel: SM pairs run FP16 operands");
+    launch(dev::tile_kernel<NT, NACC, 0u, Epi, BL, CG>);
   }
   EQTL_CUDA(cudaGetLastError());
   check_tile_status(ctx, "tile kernel");

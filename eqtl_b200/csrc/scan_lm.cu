@@ -507,13 +507,19 @@ void scan_trans_lm(eqtl_ctx* ctx, const eqtl_scan_params* prm, const double* Y, 
       if (raw) {
         const __half* bh[1] = {ctx->rot.raw.p};
         const int prod[1] = {5};
-        launch_tile_n<256, 1, LmEpiParams, dev::kBLoNone>(ctx, false, ep, ah, al, G, bh, bh, m, k_pad, bsel, prod,
-                                                          tiles, n_tiles);
+        if (!tiles && tile_pairs(G))
+          launch_tile_n<256, 1, LmEpiParams, dev::kBLoNone, 2>(ctx, false, ep, ah, al, G, bh, bh, m, k_pad, bsel, prod);
+        else
+          launch_tile_n<256, 1, LmEpiParams, dev::kBLoNone>(ctx, false, ep, ah, al, G, bh, bh, m, k_pad, bsel, prod,
+                                                            tiles, n_tiles);
       } else {
         const __half* bh[1] = {g.gc_hi.p};
         const __half* bl[1] = {g.gc_lo.p};
         const int prod[1] = {7};
-        launch_tile_n<256, 1>(ctx, bf16, ep, ah, al, G, bh, bl, m, k_pad, bsel, prod, tiles, n_tiles);
+        if (!bf16 && !tiles && tile_pairs(G))
+          launch_tile_n<256, 1, LmEpiParams, dev::kBLoStage, 2>(ctx, false, ep, ah, al, G, bh, bl, m, k_pad, bsel, prod);
+        else
+          launch_tile_n<256, 1>(ctx, bf16, ep, ah, al, G, bh, bl, m, k_pad, bsel, prod, tiles, n_tiles);
       }
     });
   }

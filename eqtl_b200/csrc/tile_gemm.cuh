@@ -25,6 +25,18 @@
 // in whichever slots the epilogue has already read, so the epilogue of tile
 // i overlaps the MMAs of tile i+1 (fully when 2 * NACC <= slots, for its
 // first accumulators otherwise).
+// CG = 2 pairs two SMs on one tile (a cluster of two CTAs, tcgen05
+// cta_group::2): 256 gene-side rows x NT SNP-side rows, of which each CTA holds
+// 128 gene-side rows and half of the SNP-side rows in its shared memory and
+// reads its own 128 rows of the accumulators. What bounds these kernels is the
+// shared memory's 128 bytes a cycle, shared by the operand reads of the MMAs,
+// the TMA writes and the epilogue's table gathers: at CG = 1 an MMA of K = 16
+// reads 4 KB of A and NT * 32 bytes of B for its N NT / 128 * 64 cycles (128
+// bytes a cycle at NT = 128, 96 at 256), at CG = 2 half of the B bytes (96 and 64), and the
+// B writes per tile halve too. Only the first CTA of the pair issues MMAs; the
+// operands of both CTAs are counted on its `full` barriers, its commits release
+// stages and publish accumulators in both CTAs, and both epilogues release the
+// slots on its `sempty` barriers.
 // A tile may need more accumulators than TMEM holds at once (the LMM with p
 // covariates needs p + 2): they then run in groups of NACC, one after the
 // other on the same CTA, and a grouped epilogue (Epi::kGrouped) receives each
@@ -72,7 +84,7 @@ struct TileShape {
   int n_groups;           // ceil(n_acc / NACC): TMEM holds one group at a time
   int bsel[kMaxAcc];      // SNP-side pair used by accumulator j (0 or 1)
   int prod[kMaxAcc];      // 1 = hi*hi, 2 = hi*lo, 4 = lo*hi (a lo part no product reads is not loaded)
-  int tiles_a;            // ceil(rows_a / 128)
+  int tiles_a;            // ceil(rows_a / (128 CG))
   int tiles_b;            // ceil(rows_b / NT)
   int n_tiles;            // work items: (tiles_a * tiles_b or the tile-list length) * ksplit
   int ksplit;             // K ranges per output tile (split-K); 1 = whole K
@@ -93,10 +105,11 @@ struct TileShape {
 //              stage holds three parts and more stages fit.
 constexpr int kBLoStage = 0, kBLoNone = 1;
 
-template <int NT, int NACC, int BL = kBLoStage>
+template <int NT, int NACC, int BL = kBLoStage, int CG = 1>
 struct TileCfg {
   static constexpr int A_BYTES = kTileM * kChunkK * 2;
-  static constexpr int B_BYTES = NT * kChunkK * 2;
+  static constexpr int NB = NT / CG;  // SNP-side rows in one CTA's shared memory
+  static constexpr int B_BYTES = NB * kChunkK * 2;
   static constexpr int STAGE_BYTES = 2 * A_BYTES + (BL == kBLoStage ? 2 : 1) * B_BYTES;
   static constexpr int STAGES = (196608 / STAGE_BYTES) < 2 ? 2 : (196608 / STAGE_BYTES > 6 ? 6 : 196608 / STAGE_BYTES);
   // TMEM is split into NSLOTS slots of NT columns; accumulator j of work
@@ -145,11 +158,11 @@ __device__ __forceinline__ void tile_coords(const TileShape& sh, int t, int& ta,
   k1 = min(sh.kchunks, k0 + sh.kc_per_split);
 }
 
-template <int NT, int NACC, uint32_t AB_FMT, class Epi, int BL = kBLoStage>
+template <int NT, int NACC, uint32_t AB_FMT, class Epi, int BL = kBLoStage, int CG = 1>
 __global__ void __launch_bounds__(kTileThreads, 1)
     tile_kernel(const __grid_constant__ TileMaps maps, const TileShape sh,
                 const __grid_constant__ typename Epi::Params ep) {
-  using C = TileCfg<NT, NACC, BL>;
+  using C = TileCfg<NT, NACC, BL, CG>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + C::STAGES * C::STAGE_BYTES);
@@ -163,6 +176,8 @@ __global__ void __launch_bounds__(kTileThreads, 1)
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
+  const uint32_t rank = CG == 2 ? cluster_ctarank() : 0u;  // 0: leads the pair
+  const int unit0 = static_cast<int>(blockIdx.x) / CG, units = static_cast<int>(gridDim.x) / CG;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::STAGES; ++s) {
@@ -171,7 +186,7 @@ __global__ void __launch_bounds__(kTileThreads, 1)
     }
     for (int k = 0; k < C::NSLOTS; ++k) {
       mbar_init(&sfull[k], 1);
-      mbar_init(&sempty[k], 32 * kEpiWarps);
+      mbar_init(&sempty[k], CG * kEpiWarps);
     }
     mbar_init(drain, 1);
     *abort_flag = 0u;
@@ -182,11 +197,12 @@ __global__ void __launch_bounds__(kTileThreads, 1)
     for (int j = 0; j < 4; ++j) tma_prefetch_map(&maps.b[j]);
   }
   if (warp == 1) {
-    tmem_alloc(tmem_slot, C::TMEM_COLS);
-    tmem_relinquish();
+    tmem_alloc<CG>(tmem_slot, C::TMEM_COLS);
+    tmem_relinquish<CG>();
   }
   tc_fence_before();
   __syncthreads();
+  if constexpr (CG == 2) cluster_sync();  // both CTAs' barriers and TMEM are ready
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   uint32_t* status = sh.status;
@@ -199,10 +215,10 @@ __global__ void __launch_bounds__(kTileThreads, 1)
       uint32_t issued_phase[6] = {0, 0, 0, 0, 0, 0};
       bool issued[6] = {false, false, false, false, false, false};
       bool ok = true;
-      for (int t = blockIdx.x; t < sh.n_tiles && ok; t += gridDim.x) {
+      for (int t = unit0; t < sh.n_tiles && ok; t += units) {
         int ta, tb, k0, k1;
         tile_coords(sh, t, ta, tb, k0, k1);
-        const int ra = ta * kTileM, rb = tb * NT;
+        const int ra = (ta * CG + static_cast<int>(rank)) * kTileM, rb = tb * NT + static_cast<int>(rank) * C::NB;
         const int ksub = sh.kc_sub > 0 ? sh.kc_sub : k1 - k0;
         for (int q0 = k0; q0 < k1 && ok; q0 += ksub)
         for (int j = 0; j < sh.n_acc && ok; ++j) {
@@ -219,12 +235,17 @@ __global__ void __launch_bounds__(kTileThreads, 1)
               break;
             }
             uint8_t* sb = smem + stage * C::STAGE_BYTES;
-            mbar_arrive_expect_tx(&full[stage], bytes);
-            tma_load_2d(sb, &maps.a[2 * j], &full[stage], kc * kChunkK, ra);
-            if (a_lo) tma_load_2d(sb + C::A_BYTES, &maps.a[2 * j + 1], &full[stage], kc * kChunkK, ra);
-            tma_load_2d(sb + 2 * C::A_BYTES, &maps.b[2 * bp], &full[stage], kc * kChunkK, rb);
-            if (b_lo)
-              tma_load_2d(sb + 2 * C::A_BYTES + C::B_BYTES, &maps.b[2 * bp + 1], &full[stage], kc * kChunkK, rb);
+            // both CTAs' bytes are expected on the leader's barrier
+            if (rank == 0) mbar_arrive_expect_tx(&full[stage], CG * bytes);
+            const uint32_t fbar = CG == 2 ? map_to_cta(&full[stage], 0) : 0u;
+            auto load = [&](uint8_t* dst, const CUtensorMap* map, int y) {
+              if constexpr (CG == 1) tma_load_2d(dst, map, &full[stage], kc * kChunkK, y);
+              else tma_load_2d_pair(dst, map, fbar, kc * kChunkK, y);
+            };
+            load(sb, &maps.a[2 * j], ra);
+            if (a_lo) load(sb + C::A_BYTES, &maps.a[2 * j + 1], ra);
+            load(sb + 2 * C::A_BYTES, &maps.b[2 * bp], rb);
+            if (b_lo) load(sb + 2 * C::A_BYTES + C::B_BYTES, &maps.b[2 * bp + 1], rb);
             issued[stage] = true;
             issued_phase[stage] = phase;
             if (++stage == C::STAGES) {
@@ -235,28 +256,34 @@ __global__ void __launch_bounds__(kTileThreads, 1)
         }
       }
       // Drain: every load issued into a ring slot must land before the CTA
-      // may exit (bounded; normally already complete).
-      for (int s = 0; s < C::STAGES; ++s) {
-        if (!issued[s]) continue;
+      // may exit, and with CG = 2 (where the leader's barriers count the peer's
+      // loads too) every release of a stage that a commit sends to both CTAs
+      // (bounded; normally already complete).
+      auto drained = [&](uint64_t* bar, uint32_t parity) {
         const long long t0 = clock64();
-        while (!mbar_test(&full[s], issued_phase[s])) {
+        while (!mbar_test(bar, parity)) {
           if (clock64() - t0 > kWaitCycles) {
             set_status(status, kDevTimeoutDrain);
-            break;
+            return;
           }
         }
+      };
+      for (int s = 0; s < C::STAGES; ++s) {
+        if (!issued[s]) continue;
+        if (rank == 0) drained(&full[s], issued_phase[s]);
+        if (CG == 2 && ok) drained(&empty[s], issued_phase[s]);
       }
     }
   } else if (warp == 1) {
     // ---------------------------------------------------------- MMA issuer
-    if (elect_one()) {
-      constexpr uint32_t idesc = idesc_f16(kTileM, NT, AB_FMT);
+    if (rank == 0 && elect_one()) {
+      constexpr uint32_t idesc = idesc_f16(CG * kTileM, NT, AB_FMT);
       int stage = 0;
       uint32_t phase = 0;
       uint32_t eph = 0;   // bit k: parity of slot k's next release
       int slot0 = 0;      // ring slot of the current unit's first accumulator
       bool ok = true;
-      for (int t = blockIdx.x; t < sh.n_tiles && ok; t += gridDim.x) {
+      for (int t = unit0; t < sh.n_tiles && ok; t += units) {
         int ta, tb, k0, k1;
         tile_coords(sh, t, ta, tb, k0, k1);
         const int ksub = sh.kc_sub > 0 ? sh.kc_sub : k1 - k0;
@@ -294,18 +321,18 @@ __global__ void __launch_bounds__(kTileThreads, 1)
                 // every later one adds
                 uint32_t accum = (kc > qa || k > 0) ? 1u : 0u;
                 if (pm & 1) {
-                  umma_f16(d, smem_desc_sw128(sa0 + off), smem_desc_sw128(sb0 + off), idesc, accum);
+                  umma_f16<CG>(d, smem_desc_sw128(sa0 + off), smem_desc_sw128(sb0 + off), idesc, accum);
                   accum = 1u;
                 }
                 if (BL == kBLoStage && (pm & 2)) {
-                  umma_f16(d, smem_desc_sw128(sa0 + off), smem_desc_sw128(sb1 + off), idesc, accum);
+                  umma_f16<CG>(d, smem_desc_sw128(sa0 + off), smem_desc_sw128(sb1 + off), idesc, accum);
                   accum = 1u;
                 }
                 if (pm & 4) {
-                  umma_f16(d, smem_desc_sw128(sa1 + off), smem_desc_sw128(sb0 + off), idesc, accum);
+                  umma_f16<CG>(d, smem_desc_sw128(sa1 + off), smem_desc_sw128(sb0 + off), idesc, accum);
                 }
               }
-              umma_commit(&empty[stage]);
+              umma_commit<CG>(&empty[stage]);
               if (++stage == C::STAGES) {
                 stage = 0;
                 phase ^= 1u;
@@ -313,11 +340,11 @@ __global__ void __launch_bounds__(kTileThreads, 1)
             }
           }
           if (!ok) break;
-          umma_commit(&sfull[last]);  // completes when every MMA issued so far has
+          umma_commit<CG>(&sfull[last]);  // completes when every MMA issued so far has
         }
       }
       // Drain: all issued MMAs complete before TMEM is released (bounded).
-      umma_commit(drain);
+      umma_commit<CG, true>(drain);
       const long long t0 = clock64();
       while (!mbar_test(drain, 0u)) {
         if (clock64() - t0 > kWaitCycles) {
@@ -338,10 +365,21 @@ __global__ void __launch_bounds__(kTileThreads, 1)
     uint32_t fph = 0;   // bit k: parity of slot k's next completion
     int slot0 = 0;      // ring slot of the current unit's first accumulator
     const uint32_t lanes = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
-    for (int t = blockIdx.x; t < sh.n_tiles; t += gridDim.x) {
+    // accumulators [j0, j1) of the unit have been read by this warp
+    auto release = [&](int j0, int j1) {
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0)
+        for (int jj = j0; jj < j1; ++jj) {
+          uint64_t* bar = &sempty[(slot0 + jj) % C::NSLOTS];
+          if constexpr (CG == 1) mbar_arrive(bar);
+          else mbar_arrive_cluster(map_to_cta(bar, 0));
+        }
+    };
+    for (int t = unit0; t < sh.n_tiles; t += units) {
       int ta, tb, k0, k1;
       tile_coords(sh, t, ta, tb, k0, k1);
-      epi.begin_tile(ta * kTileM + row, tb * NT);
+      epi.begin_tile((ta * CG + static_cast<int>(rank)) * kTileM + row, tb * NT);
       bool eok = true;
       const int ksub = sh.kc_sub > 0 ? sh.kc_sub : k1 - k0;
       for (int q0 = k0; q0 < k1 && eok; q0 += ksub)
@@ -383,8 +421,7 @@ __global__ void __launch_bounds__(kTileThreads, 1)
             tmem_wait_ld();
             epi.template pre_chunk<N1>(ci, c, v);
           }
-          tc_fence_before();
-          for (int jj = 0; jj < N1; ++jj) mbar_arrive(&sempty[(slot0 + jj) % C::NSLOTS]);
+          release(0, N1);
 #pragma unroll 1
           for (int ci = 0; ci < NCH; ++ci) {
             const int c = 16 * sub + 16 * kSub * ci;
@@ -394,8 +431,7 @@ __global__ void __launch_bounds__(kTileThreads, 1)
             tmem_wait_ld();
             epi.template post_chunk<NACC - N1>(ci, c, v);
           }
-          tc_fence_before();
-          for (int jj = N1; jj < nv; ++jj) mbar_arrive(&sempty[(slot0 + jj) % C::NSLOTS]);
+          release(N1, nv);
           continue;  // slots released above
         } else if constexpr (HasChunkIdx<Epi>::value) {
           constexpr int NCH = NT / (16 * kSub);
@@ -419,8 +455,7 @@ __global__ void __launch_bounds__(kTileThreads, 1)
             epi.template chunk<NACC>(c, v);
           }
         }
-        tc_fence_before();
-        for (int jj = 0; jj < nv; ++jj) mbar_arrive(&sempty[(slot0 + jj) % C::NSLOTS]);
+        release(0, nv);
       }
       if (!eok) break;
       epi.end_tile();
@@ -429,9 +464,12 @@ __global__ void __launch_bounds__(kTileThreads, 1)
   }
 
   __syncthreads();
+  // neither CTA of a pair leaves while the other may still read its shared
+  // memory, arrive on its barriers or write its TMEM
+  if constexpr (CG == 2) cluster_sync();
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, C::TMEM_COLS);
+    tmem_dealloc<CG>(tmem_base, C::TMEM_COLS);
   }
 }
 
