@@ -257,6 +257,11 @@ dev::Windows upload_windows(eqtl_ctx* ctx, const eqtl_scan_params* prm, int64_t 
   ws.win_gc.upload(prm->gene_chrom, prm->n_genes, ctx->stream);
   ws.win_glo.upload(prm->gene_lo, prm->n_genes, ctx->stream);
   ws.win_ghi.upload(prm->gene_hi, prm->n_genes, ctx->stream);
+  // 16-SNP blocks, up to one 256-SNP tile past the last padded tile; the
+  // padding's values are not used (its SNPs are not tested)
+  const int64_t nb = ((m + 255) / 256 + 1) * 16;
+  ws.win_sc.alloc(static_cast<size_t>(nb * 16));
+  ws.win_sp.alloc(static_cast<size_t>(nb * 16));
   ws.win_sc.upload(prm->snp_chrom, m, ctx->stream);
   ws.win_sp.upload(prm->snp_pos, m, ctx->stream);
   w.mode = mode;
@@ -265,8 +270,6 @@ dev::Windows upload_windows(eqtl_ctx* ctx, const eqtl_scan_params* prm, int64_t 
   w.gene_hi = ws.win_ghi.p;
   w.snp_chrom = ws.win_sc.p;
   w.snp_pos = ws.win_sp.p;
-  // 16-SNP block bounds, up to one 256-SNP tile past the last padded tile
-  const int64_t nb = ((m + 255) / 256 + 1) * 16;
   std::vector<int32_t> bc(static_cast<size_t>(nb), -1);
   std::vector<int64_t> blo(static_cast<size_t>(nb), 0), bhi(static_cast<size_t>(nb), -1);
   for (int64_t b = 0; b * 16 < m; ++b) {

@@ -1055,11 +1055,16 @@ struct LmmRawEpiParams : LmmEpiParams<P> {};
 template <int P>
 struct LmmLrEpiParams : LmmEpiParams<P> {};
 
-// Accumulator order of the tile: [gg, a_0 .. a_{P-1}, NUM] (the gene-side
-// operands w, w o X~_k, w o r~ against Gt^2, Gt, Gt). The epilogue is
-// two-phase: S = gg - a' A00^-1 a of every pair of the warp's chunks first,
-// which frees the gg and a slots for the next tile's MMAs, then NUM and the
-// rest of the statistic.
+// P = 1: accumulator order [NUM, gg, a_0] (the gene-side operands w o r~, w,
+// w o X~_0 against Gt, Gt^2, Gt), all three read chunk by chunk. TMEM's fourth
+// slot takes the next tile's NUM, whose MMAs (K = n) then run under this
+// epilogue, and nothing is kept in registers from chunk to chunk. (The order
+// [gg, a_0, NUM] in two phases, which P = 2 uses, kept 32 values of S per thread
+// and spilled: 600 bytes of spill loads a tile.)
+// P = 2: order [gg, a_0, a_1, NUM] in two phases, since four accumulators fill
+// TMEM: S = gg - a' A00^-1 a of every pair of the warp's chunks first, which
+// frees the gg and a slots for the next tile's MMAs, then NUM and the rest of
+// the statistic.
 //
 // GLM = true is the NB-GLM score test on the same accumulators (unrotated
 // centred dosages gc against w, w o x_k and r of the gene's null fit):
@@ -1078,7 +1083,7 @@ struct LmmEpi {
   static_assert(!(GLM && RAW), "the exact-operand form is the LMM scan's");
   static_assert(!LR || RAW, "the interpolated form reads NUM from the exact operand");
   static constexpr bool kGrouped = false;
-  static constexpr bool kTwoPhase = true;
+  static constexpr bool kTwoPhase = P > 1;
   static constexpr int kPhase1 = P + 1;  // gg and a_k
   static constexpr int kMaxChunks = 2;   // 16-column chunks per warp and tile
   using Params = std::conditional_t<
@@ -1087,7 +1092,6 @@ struct LmmEpi {
   static constexpr int kSmemBytes = kTTableSmemBytes;
   const Params& Pr;
   float* tsm;
-  TTable tt;
   int gene = 0;
   int64_t snp0 = 0;
   bool gvalid = false;
@@ -1095,15 +1099,16 @@ struct LmmEpi {
   float ai[P][P];
   float inv_rss = 0;
   float rs = 0;  // GLM: sum_i r_i of the gene
-  // S per pair of the warp's two chunks (0 where gg < 1e-12); two named
+  // P = 2: S per pair of the warp's two chunks (0 where gg < 1e-12); two named
   // arrays picked by a select, so they stay in registers for a runtime ci
   float S0[16], S1[16];
   float u_cand;  // t_cand^2
+  uint32_t tab = 0;  // screen_tables (0: none)
   GeneAcc acc;
   __device__ LmmEpi(const Params& p, const TileShape&, uint8_t* smem)
-      : Pr(p), tsm(reinterpret_cast<float*>(smem)), tt(p.tt), u_cand(p.t_cand * p.t_cand) {}
+      : Pr(p), tsm(reinterpret_cast<float*>(smem)), u_cand(p.t_cand * p.t_cand) {}
   __device__ void init(int tid, int nthr) {
-    if (tsm) tt = screen_to_smem(Pr.tt, tsm, tid, nthr);
+    if (tsm && Pr.tt.lt_u) tab = screen_tables(Pr.tt, tsm, tid, nthr);
   }
   __device__ void begin_tile(int g, int64_t s0) {
     gene = g;
@@ -1124,11 +1129,72 @@ struct LmmEpi {
         inv_rss = r > 0 ? static_cast<float>(1.0 / r) : 0.0f;
       }
       acc.load_window(Pr.win, g);
+      acc.load_best(Pr.out, g);
     }
   }
   // Screening arithmetic in FP32 (the accumulators carry ~1e-7 relative
   // error already); printed statistics come from the FP64 refinement.
-  // Phase 1: v = [gg, a_0 .. a_{P-1}] of 16 pairs.
+  // S of one pair from its accumulators [gg, a_0 .. a_{P-1}] (0 where gg <
+  // 1e-12: p = 1, S fails the S > 1e-15 test). us: alpha of the SNP (RAW).
+  template <class V>
+  __device__ __forceinline__ float schur(V&& v, float us) {
+    const float gg = v(0) * u[P + 1];
+    float S = gg;
+    float a[P];
+#pragma unroll
+    for (int k = 0; k < P; ++k) a[k] = v(1 + k) * (us * u[1 + k]);
+#pragma unroll
+    for (int x = 0; x < P; ++x)
+#pragma unroll
+      for (int y = 0; y < P; ++y) S = fmaf(-a[x] * ai[x][y], a[y], S);
+    return gg < 1e-12f ? 0.0f : S;
+  }
+  // The screen of 16 pairs from NUM's accumulators and S.
+  __device__ __forceinline__ void screen(int64_t s0, const float (&num_acc)[16], const float (&S)[16]) {
+    const float4* al4 = reinterpret_cast<const float4*>(Pr.snp_alpha + s0);  // RAW (padded past the last tile)
+    uint32_t okw[4];
+    load_flags16(Pr.snp_ok + s0, okw);
+    float s_min = INFINITY;
+#pragma unroll
+    for (int j = 0; j < 16; j += 2) s_min = min3(s_min, S[j], S[j + 1]);
+    auto num_of = [&](int j) {
+      float num = num_acc[j] * u[0];
+      if constexpr (RAW) {
+        const float4 a = __ldg(al4 + (j >> 2));
+        num *= (j & 3) == 0 ? a.x : (j & 3) == 1 ? a.y : (j & 3) == 2 ? a.z : a.w;
+      }
+      return num;
+    };
+    screen_chunk(
+        Pr.tt, tab, u_cand, Pr.win, Pr.out, gene, s0, all_flags16(okw) && s_min > 1e-15f,
+        [&](int j) {
+          const float num = num_of(j);
+          if constexpr (GLM) {
+            const float U = fmaf(__ldg(Pr.snp_mean + s0 + j), rs, num);
+            return U * U * rcp_ftz(S[j]);  // z^2
+          } else {
+            const float r = num * (num * rcp_ftz(S[j])) * inv_rss;
+            return Pr.df * (r * rcp_ftz(1.0f - r));  // t^2
+          }
+        },
+        [&](int j, bool& tested) {
+          tested = flag16(okw, j);  // zero past the last kept SNP
+          const float num = num_of(j);
+          float t2;
+          if constexpr (GLM) {
+            const float U = fmaf(__ldg(Pr.snp_mean + s0 + j), rs, num);
+            t2 = S[j] > 1e-15f ? __fdividef(U * U, S[j]) : 0.0f;
+            if (!(t2 == t2)) t2 = 0.0f;
+          } else {
+            const float r = num * __fdividef(num, S[j]) * inv_rss;
+            const float omr = 1.0f - r;
+            t2 = S[j] > 1e-15f && omr > 0.0f ? Pr.df * __fdividef(r, omr) : 0.0f;
+          }
+          return t2;
+        },
+        acc);
+  }
+  // P = 2, phase 1: v = [gg, a_0, a_1] of 16 pairs.
   template <int N>
   __device__ void pre_chunk(int ci, int c, const float (&v)[N][16]) {
     static_assert(N == P + 1, "phase-1 accumulators");
@@ -1136,107 +1202,61 @@ struct LmmEpi {
     if constexpr (RAW && !LR) load16(Pr.snp_alpha + snp0 + c, al);
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
-      const float gg = v[0][j] * u[P + 1];
-      float S = gg;
-      float a[P];
       float us = 1.0f;
       if constexpr (RAW && !LR) us = al[j];
-#pragma unroll
-      for (int k = 0; k < P; ++k) a[k] = v[1 + k][j] * (us * u[1 + k]);
-#pragma unroll
-      for (int x = 0; x < P; ++x)
-#pragma unroll
-        for (int y = 0; y < P; ++y) S = fmaf(-a[x] * ai[x][y], a[y], S);
-      const float Sj = gg < 1e-12f ? 0.0f : S;  // gg < 1e-12: p = 1 (S fails the S > 1e-15 test)
+      const float Sj = schur([&](int k) { return v[k][j]; }, us);
       if (ci == 0) S0[j] = Sj;
       else S1[j] = Sj;
     }
   }
-  // Phase 2: v = [NUM] of the same 16 pairs. The 16 pairs share one
-  // branch-free tail evaluation, so their table lookups overlap.
+  // Phase 2: v = [NUM] of the same 16 pairs.
   template <int N>
   __device__ void post_chunk(int ci, int c, const float (&v)[N][16]) {
     static_assert(N == 1, "phase-2 accumulators");
     const int64_t s0 = snp0 + c;
     if (!gvalid || s0 >= Pr.m) return;
-    uint32_t okw[4];
-    load_flags16(Pr.snp_ok + s0, okw);
-    float al[16];
-    if constexpr (RAW) load16(Pr.snp_alpha + s0, al);
-    if (!GLM && tt.lt_u) {  // uniform across the launch
-      // a gw scan (no windows), and a trans scan on a chunk clear of every
-      // lane's gene window, skip the per-pair window test; the vote keeps
-      // the warp on one path
-      if (Pr.win.mode == kWinNone)
-        post_cubic<false>(ci, s0, v[0], okw, al);
-      else if (Pr.win.mode == kWinExclude && __all_sync(__activemask(), acc.chunk_clear(Pr.win, s0)))
-        post_cubic<false>(ci, s0, v[0], okw, al);
-      else
-        post_cubic<true>(ci, s0, v[0], okw, al);
-      return;
-    }
+    float S[16];
 #pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      const int64_t s = s0 + j;
-      const bool valid = flag16(okw, j) && s < Pr.m && acc.in_scope(Pr.win, s);
-      float num = v[0][j] * u[0];
-      if constexpr (RAW) num *= al[j];
-      const float S = ci == 0 ? S0[j] : S1[j];
-      float u;
-      if constexpr (GLM) {
-        const float U = fmaf(__ldg(Pr.snp_mean + s), rs, num);
-        u = S > 1e-15f ? __fdividef(U * U, S) : 0.0f;  // z^2
-      } else {
-        const float r = num * __fdividef(num, S) * inv_rss;
-        const float omr = 1.0f - r;
-        const bool ok_stat = S > 1e-15f && omr > 0.0f;
-        u = ok_stat ? Pr.df * __fdividef(r, omr) : 0.0f;  // t^2
-      }
-      const ScreenOut o = acat_screen_u(u, tt);
-      acc.add_screen(o, s, valid);
-      if (valid && (u >= u_cand || o.deferred)) emit_candidate(Pr.out, gene, s, o.deferred, o.tiny);
-    }
-    acc.end_chunk();
+    for (int j = 0; j < 16; ++j) S[j] = ci == 0 ? S0[j] : S1[j];
+    screen(s0, v[0], S);
   }
-  // Phase 2 with the per-interval cubics (screen16_cubic). The SNP flags are
-  // zero past the last kept SNP, so they also mask the padding.
-  template <bool WIN>
-  __device__ void post_cubic(int ci, int64_t s0, const float (&v)[16], const uint32_t (&okw)[4],
-                             const float (&al)[16]) {
-    float uu[16];
-    bool valid[16];
-#pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      valid[j] = flag16(okw, j) && (!WIN || acc.in_scope(Pr.win, s0 + j));
-      float num = v[j] * u[0];
-      if constexpr (RAW) num *= al[j];
-      const float S = ci == 0 ? S0[j] : S1[j];
-      const float r = num * __fdividef(num, S) * inv_rss;
-      const float omr = 1.0f - r;
-      uu[j] = S > 1e-15f && omr > 0.0f ? Pr.df * __fdividef(r, omr) : 0.0f;  // t^2, never NaN
-      if (!valid[j]) uu[j] = 0.0f;
-    }
-    screen16_cubic(tt, uu, valid, u_cand, Pr.out, gene, s0, acc);
-  }
-  // Both phases at once (the CUDA-core comparator): v in the tile's order.
+  // All accumulators of 16 pairs at once: P = 1 in its order [NUM, gg, a_0].
   template <int NACC>
   __device__ void chunk(int c, const float (&v)[NACC][16]) {
     static_assert(NACC == P + 2, "accumulators");
-    float v1[P + 1][16];
+    all_at_once<0, 1>(c, v);
+  }
+  template <int NUM, int GG, int NACC>
+  __device__ __forceinline__ void all_at_once(int c, const float (&v)[NACC][16]) {
+    const int64_t s0 = snp0 + c;
+    if (!gvalid || s0 >= Pr.m) return;
+    float S[16];
+    {
+      float al[16];
+      if constexpr (RAW && !LR) load16(Pr.snp_alpha + s0, al);
 #pragma unroll
-    for (int k = 0; k < P + 1; ++k)
-#pragma unroll
-      for (int j = 0; j < 16; ++j) v1[k][j] = v[k][j];
-    pre_chunk<P + 1>(0, c, v1);
-    float v2[1][16];
-#pragma unroll
-    for (int j = 0; j < 16; ++j) v2[0][j] = v[P + 1][j];
-    post_chunk<1>(0, c, v2);
+      for (int j = 0; j < 16; ++j) {
+        float us = 1.0f;
+        if constexpr (RAW && !LR) us = al[j];
+        S[j] = schur([&](int k) { return v[GG + k][j]; }, us);
+      }
+    }
+    screen(s0, v[NUM], S);
   }
   __device__ void end_tile() {
     if (gvalid) acc.flush(Pr.out, gene);
   }
   __device__ void finish() {}
+};
+
+// The CUDA-core comparator hands over its accumulators as [gg, a_0 .., NUM].
+template <int P>
+struct LmmSimtEpi : LmmEpi<P> {
+  using LmmEpi<P>::LmmEpi;
+  template <int NACC>
+  __device__ void chunk(int c, const float (&v)[NACC][16]) {
+    this->template all_at_once<P + 1, 0>(c, v);
+  }
 };
 
 // ------------------------------------- node-interpolated gg and a_k (p <= 2)
@@ -1529,7 +1549,6 @@ struct LmmGroupEpiT {
   static constexpr int kSmemBytes = kTTableSmemBytes;
   const Params& Pr;
   float* tsm;
-  TTable tt;
   int gene = 0;
   int64_t snp0 = 0;
   bool gvalid = false;
@@ -1537,11 +1556,12 @@ struct LmmGroupEpiT {
   float rs = 0;  // GLM: sum_i r_i of the gene
   float num[16], S[16];
   float u_cand;  // t_cand^2
+  uint32_t tab = 0;  // screen_tables (0: none)
   GeneAcc acc;
   __device__ LmmGroupEpiT(const Params& p, const TileShape&, uint8_t* smem)
-      : Pr(p), tsm(reinterpret_cast<float*>(smem)), tt(p.tt), u_cand(p.t_cand * p.t_cand) {}
+      : Pr(p), tsm(reinterpret_cast<float*>(smem)), u_cand(p.t_cand * p.t_cand) {}
   __device__ void init(int tid, int nthr) {
-    if (tsm) tt = screen_to_smem(Pr.tt, tsm, tid, nthr);
+    if (Pr.tt.lt_u) tab = screen_tables(Pr.tt, tsm, tid, nthr);
   }
   __device__ void begin_tile(int g, int64_t s0) {
     gene = g;
@@ -1557,6 +1577,7 @@ struct LmmGroupEpiT {
         inv_rss = r > 0 ? static_cast<float>(1.0 / r) : 0.0f;
       }
       acc.load_window(Pr.win, g);
+      acc.load_best(Pr.out, g);
     }
   }
   // accumulator j of this tile for the 16 columns at c
@@ -1581,25 +1602,35 @@ struct LmmGroupEpiT {
     if (!gvalid || s0 >= Pr.m) return;
     uint32_t okw[4];
     load_flags16(Pr.snp_ok + s0, okw);
+    float s_min = INFINITY;
 #pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      const int64_t s = s0 + j;
-      const bool valid = flag16(okw, j) && s < Pr.m && acc.in_scope(Pr.win, s);
-      float u;
-      if constexpr (GLM) {
-        const float U = fmaf(__ldg(Pr.snp_mean + s), rs, num[j]);
-        u = S[j] > 1e-15f ? __fdividef(U * U, S[j]) : 0.0f;  // z^2
-      } else {
-        const float r = num[j] * __fdividef(num[j], S[j]) * inv_rss;
-        const float omr = 1.0f - r;
-        const bool ok_stat = S[j] > 1e-15f && omr > 0.0f;
-        u = ok_stat ? Pr.df * __fdividef(r, omr) : 0.0f;  // t^2
-      }
-      const ScreenOut o = acat_screen_u(u, tt);
-      acc.add_screen(o, s, valid);
-      if (valid && (u >= u_cand || o.deferred)) emit_candidate(Pr.out, gene, s, o.deferred, o.tiny);
-    }
-    acc.end_chunk();
+    for (int j = 0; j < 16; j += 2) s_min = min3(s_min, S[j], S[j + 1]);
+    screen_chunk(
+        Pr.tt, tab, u_cand, Pr.win, Pr.out, gene, s0, all_flags16(okw) && s_min > 1e-15f,
+        [&](int j) {
+          if constexpr (GLM) {
+            const float U = fmaf(__ldg(Pr.snp_mean + s0 + j), rs, num[j]);
+            return U * U * rcp_ftz(S[j]);  // z^2
+          } else {
+            const float r = num[j] * (num[j] * rcp_ftz(S[j])) * inv_rss;
+            return Pr.df * (r * rcp_ftz(1.0f - r));  // t^2
+          }
+        },
+        [&](int j, bool& tested) {
+          tested = flag16(okw, j);  // zero past the last kept SNP
+          float t2;
+          if constexpr (GLM) {
+            const float U = fmaf(__ldg(Pr.snp_mean + s0 + j), rs, num[j]);
+            t2 = S[j] > 1e-15f ? __fdividef(U * U, S[j]) : 0.0f;
+            if (!(t2 == t2)) t2 = 0.0f;
+          } else {
+            const float r = num[j] * __fdividef(num[j], S[j]) * inv_rss;
+            const float omr = 1.0f - r;
+            t2 = S[j] > 1e-15f && omr > 0.0f ? Pr.df * __fdividef(r, omr) : 0.0f;
+          }
+          return t2;
+        },
+        acc);
   }
   __device__ void end_tile() {
     if (gvalid) acc.flush(Pr.out, gene);
@@ -2211,6 +2242,13 @@ static void lmm_launch_simt(eqtl_ctx* ctx, const LmmEpiParams<P>& ep, const __ha
                             const __half* const* al, int G, const __half* const* bh, const __half* const* bl,
                             const int* bsel, const Rotated& R);
 
+// Gene-ops index (0 NUM, 1 .. p a_k, p + 1 gg) of the tile's accumulator j
+// (LmmEpi): [NUM, gg, a_0] on the tensor cores with p = 1, else [gg, a_0 .., NUM].
+static int lmm_acc_op(int p, int j, bool tensor) {
+  if (tensor && p == 1) return j == 0 ? 0 : (j == 1 ? 2 : 1);
+  return j == 0 ? p + 1 : (j == p + 1 ? 0 : j);
+}
+
 template <int P, class EP>
 static void lmm_launch(eqtl_ctx* ctx, const EP& ep, const __half* const* ah, const __half* const* al, int G,
                        bool simt, const int2* tiles, int n_tiles, const Rotated& R) {
@@ -2219,16 +2257,17 @@ static void lmm_launch(eqtl_ctx* ctx, const EP& ep, const __half* const* ah, con
   constexpr bool raw = std::is_same_v<EP, LmmRawEpiParams<P>>;
   const __half* bh[2] = {raw ? R.raw.p : R.gt_hi.p, R.gt2_hi.p};
   const __half* bl[2] = {raw ? R.raw.p : R.gt_lo.p, R.gt2_lo.p};
-  // tile order [gg, a_0 .. a_{P-1}, NUM] from the gene-ops order [NUM, a.., gg]
+  // the tile's accumulators [NUM, gg, a_0] (p = 1, tensor cores) or [gg, a_0 ..
+  // a_{P-1}, NUM] from the gene-ops order [NUM, a.., gg]
   const __half* oh[P + 2];
   const __half* ol[P + 2];
   int bsel[P + 2], prod[P + 2];
   for (int j = 0; j < P + 2; ++j) {
-    const int op = j == 0 ? P + 1 : (j == P + 1 ? 0 : j);
+    const int op = lmm_acc_op(P, j, !simt);
     oh[j] = ah[op];
     ol[j] = al[op];
-    bsel[j] = j == 0 ? 1 : 0;  // gg reads Gt^2
-    prod[j] = raw && j > 0 ? 5 : 7;
+    bsel[j] = op == P + 1 ? 1 : 0;  // gg reads Gt^2
+    prod[j] = raw && op != P + 1 ? 5 : 7;
   }
   ah = oh;
   al = ol;
@@ -2265,7 +2304,7 @@ static void lmm_launch_simt(eqtl_ctx* ctx, const LmmEpiParams<P>& ep, const __ha
   dptr.upload(ptrs, P + 2, st);
   TileShape sh{};
   using Cfg = SimtCfg<P + 2>;
-  auto kern = simt_tile_kernel<P + 2, LmmEpi<P>>;
+  auto kern = simt_tile_kernel<P + 2, LmmSimtEpi<P>>;
   EQTL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES));
   dim3 grid(static_cast<unsigned>((R.m + kSimtBN - 1) / kSimtBN), static_cast<unsigned>((G + kSimtBM - 1) / kSimtBM));
   ++ctx->launches;
@@ -2543,7 +2582,7 @@ static bool lmm_lr_prepare(eqtl_ctx* ctx, int n, int G, float s2) {
   }
 }
 
-// The scan with interpolated gg and a_k: tile order [gg, a_0 .., NUM]; gg
+// The scan with interpolated gg and a_k, in LmmEpi's accumulator order: gg
 // and a_k read their kind's node columns of both interpolated operands
 // (K chunks [kind c, (kind + 1) c), c = kn / 64), NUM reads u hi + lo
 // against the exact raw operand over all of K. ah / al: the gene-ops order
@@ -2557,19 +2596,24 @@ static void lmm_launch_lr(eqtl_ctx* ctx, const LmmLrEpiParams<P>& ep, const __ha
   const __half* ol[P + 2];
   int bsel[P + 2], prod[P + 2];
   TileK tk;
-  for (int j = 0; j <= P; ++j) {
+  for (int j = 0; j < P + 2; ++j) {
+    const int op = lmm_acc_op(P, j, true);
+    if (op == 0) {
+      oh[j] = ah[0];
+      ol[j] = al[0];
+      bsel[j] = 0;
+      prod[j] = 5;
+      continue;
+    }
+    const int kind = op == P + 1 ? 0 : op;  // lr_coef_kernel's order: gg, a_0 ..
     oh[j] = ws.lr_chi.p;
     ol[j] = ws.lr_clo.p;
     bsel[j] = 1;
     prod[j] = 7;
-    tk.beg[j] = j * c;
-    tk.end[j] = (j + 1) * c;
+    tk.beg[j] = kind * c;
+    tk.end[j] = (kind + 1) * c;
     tk.k_a[j] = kb;
   }
-  oh[P + 1] = ah[0];
-  ol[P + 1] = al[0];
-  bsel[P + 1] = 0;
-  prod[P + 1] = 5;
   tk.k_b[1] = kb;
   const __half* bh[2] = {R.raw.p, ws.lr_phi.p};
   const __half* bl[2] = {R.raw.p, ws.lr_plo.p};

@@ -29,7 +29,7 @@ struct Windows {
   const int32_t* gene_chrom;
   const int64_t* gene_lo;
   const int64_t* gene_hi;
-  const int32_t* snp_chrom;
+  const int32_t* snp_chrom;  // padded as the blocks below
   const int64_t* snp_pos;
   // per block of 16 kept SNPs (b = s / 16, covering the padded tiles): the
   // block's chromosome (-1 where it mixes chromosomes or lies past the last
@@ -45,11 +45,6 @@ struct GeneAcc {
   int used = 0;
   int tested = 0;
   unsigned long long best = ~0ull;
-  // FP32 sum of the ACAT terms of the current chunk of add_screen pairs, and
-  // its best key and SNP (end_chunk folds them into acat and best)
-  float chunk_acat = 0.0f;
-  float chunk_key = -1.0f;
-  uint32_t chunk_snp = 0;
   // no pair with u below this can be the gene's best (screen16_fast)
   float u_floor = 0.0f;
   int chrom = -1;
@@ -60,8 +55,6 @@ struct GeneAcc {
     used = 0;
     tested = 0;
     best = ~0ull;
-    chunk_acat = 0.0f;
-    chunk_key = -1.0f;
   }
   // Starts from the best that any block has published for the gene (a stale
   // one is only a lower floor).
@@ -84,64 +77,43 @@ struct GeneAcc {
     const int32_t c = __ldg(w.blk_chrom + b);
     return c >= 0 && (c != chrom || __ldg(w.blk_hi + b) < lo || __ldg(w.blk_lo + b) > hi);
   }
-  // true if the (gene, snp) pair is part of this scope
-  __device__ __forceinline__ bool in_scope(const Windows& w, int64_t s) const {
-    if (w.mode == kWinNone) return true;
-    const bool inwin = chrom >= 0 && __ldg(w.snp_chrom + s) == chrom && __ldg(w.snp_pos + s) >= lo &&
-                       __ldg(w.snp_pos + s) <= hi;
-    return w.mode == kWinExclude ? !inwin : inwin;
+  // true if every SNP of that block lies in this gene's window
+  __device__ __forceinline__ bool chunk_inside(const Windows& w, int64_t s0) const {
+    const int64_t b = s0 >> 4;
+    return chrom >= 0 && __ldg(w.blk_chrom + b) == chrom && __ldg(w.blk_lo + b) >= lo && __ldg(w.blk_hi + b) <= hi;
   }
-  // Update for one (gene, SNP) pair; `valid` masks pairs outside the scan
-  // (SNP gate, window, padding). Kept as predicated branches: the
-  // select form `acat += u ? term : 0.0` produced zero sums on sm_100a.
-  __device__ __forceinline__ void add_masked(const TailOut& o, int64_t s, bool valid) {
-    if (valid) {
-      ++tested;
-      if (o.use_acat) {
-        acat += o.term;
-        ++used;
-      }
-      const unsigned long long k = best_key(o.neglog10p, static_cast<uint32_t>(s));
+  // Bit j: SNP s0 + j of the block of 16 at s0 lies in this gene's window. The
+  // positions come with eight 16-byte loads that do not wait for one another
+  // (the arrays are padded to the block bounds' range); one at a time behind
+  // the chromosome test, as the lanes' genes decide, they took thousands of
+  // cycles a block.
+  __device__ __forceinline__ uint32_t window_mask(const Windows& w, int64_t s0) const {
+    const longlong2* p2 = reinterpret_cast<const longlong2*>(w.snp_pos + s0);
+    const int4* c4 = reinterpret_cast<const int4*>(w.snp_chrom + s0);
+    uint32_t m = 0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int4 c = __ldg(c4 + q);
+      const longlong2 a = __ldg(p2 + 2 * q), b = __ldg(p2 + 2 * q + 1);
+      m |= (c.x == chrom && a.x >= lo && a.x <= hi) ? 1u << (4 * q) : 0u;
+      m |= (c.y == chrom && a.y >= lo && a.y <= hi) ? 2u << (4 * q) : 0u;
+      m |= (c.z == chrom && b.x >= lo && b.x <= hi) ? 4u << (4 * q) : 0u;
+      m |= (c.w == chrom && b.y >= lo && b.y <= hi) ? 8u << (4 * q) : 0u;
+    }
+    return chrom >= 0 ? m : 0u;
+  }
+  // Adds a chunk of 16 pairs: its counts, the FP32 sum of its ACAT terms (the
+  // error is ~1e-6 of the chunk's largest term, below the screen's own) and its
+  // best pair (score < 0: none). A chunk's best is its first pair with the
+  // largest score; the 64-bit key breaks ties by SNP index across chunks.
+  __device__ __forceinline__ void add_chunk(int n_tested, int n_used, float sum, float score, uint32_t snp) {
+    tested += n_tested;
+    used += n_used;
+    acat += static_cast<double>(sum);
+    if (score >= 0.0f) {
+      const unsigned long long k = best_key(score, snp);
       best = k < best ? k : best;
     }
-  }
-  // The same for the epilogues' ACAT screen (best SNP keyed on the screen's
-  // key, t^2 in the scans). Pairs come in chunks of up to 16 SNPs; the terms
-  // of a chunk are summed in FP32 (the error is ~1e-6 of the chunk's largest
-  // term, below the screen's own) and added to the FP64 total by end_chunk.
-  // A chunk's pairs come in increasing SNP order, so its best is the first
-  // pair with the largest key (strict >), and the 64-bit key that breaks ties
-  // by SNP index across chunks is formed once per chunk.
-  __device__ __forceinline__ void add_screen(const ScreenOut& o, int64_t s, bool valid) {
-    if (valid) {
-      ++tested;
-      if (o.use_acat) {
-        chunk_acat += o.term;
-        ++used;
-      }
-      if (o.key > chunk_key) {
-        chunk_key = o.key;
-        chunk_snp = static_cast<uint32_t>(s);
-      }
-    }
-  }
-  __device__ __forceinline__ void end_chunk() {
-    acat += static_cast<double>(chunk_acat);
-    chunk_acat = 0.0f;
-    if (chunk_key >= 0.0f) {
-      const unsigned long long k = best_key(chunk_key, chunk_snp);
-      best = k < best ? k : best;
-      chunk_key = -1.0f;
-    }
-  }
-  __device__ __forceinline__ void add(const TailOut& o, int64_t s) {
-    ++tested;
-    if (o.use_acat) {
-      acat += o.term;  // 0 for deferred terms
-      ++used;
-    }
-    const unsigned long long k = best_key(o.neglog10p, static_cast<uint32_t>(s));
-    best = k < best ? k : best;
   }
   __device__ __forceinline__ void flush(const GeneOut& out, int g) const {
     if (tested == 0) return;
@@ -187,68 +159,89 @@ __device__ __forceinline__ void emit_candidate(const GeneOut& out, int g, int64_
                                                   (tiny ? kCandTiny : 0u)));
 }
 
-// The ACAT screen of one gene's 16 pairs s0 .. s0 + 15 with the per-interval
-// cubics (acat_screen_u's lt_u branch, T.lt_u set), for epilogues whose u =
-// t^2 is never NaN (a pair outside the scan, or with p = 1, has u = 0). With
-// u_tiny > 0:
+// What a chunk of 16 pairs adds to its gene (GeneAcc::add_chunk).
+struct ChunkSums {
+  float sum, score;
+  int tested, used, j;
+};
+
+// The ACAT screen of one gene's 16 pairs s0 .. s0 + 15, the general form: u =
+// t^2 of each (0 outside the scan and where p = 1), the bits of `valid` mark
+// the pairs that are tested. With u_tiny > 0:
 //   tiny      0 < u < u_tiny         deferred   tiny or u >= u_defer
 //   ACAT      u_tiny <= u < u_defer  candidate  u >= min(u_cand, u_defer) or tiny
-// The counts, the FP32 term sum and the chunk's best go into acc without
-// per-pair flag structs; candidates are emitted as they are found.
-__device__ __forceinline__ void screen16_cubic(const TTable& tt, const float (&u)[16], const bool (&valid)[16],
-                                               float u_cand, const GeneOut& out, int gene, int64_t s0,
-                                               GeneAcc& acc) {
+// Candidates are emitted as they are found. Out of line: it serves the chunks
+// that screen16_fast leaves, and inlined it cost the epilogues the registers that
+// their common path needs. Unrolled, since a tile's accumulators are released by
+// its slowest warp, so the latency of the rare chunk counts (a rolled loop here
+// took the LM scan from 64 to 72 ms). tab: screen_tables (0: the tables in
+// global memory).
+__device__ __noinline__ inline ChunkSums screen16_general(const TTable& tt, uint32_t tab, const float* u,
+                                                          uint32_t valid, float u_cand, const GeneOut& out, int gene,
+                                                          int64_t s0) {
+  ChunkSums r{0.0f, -1.0f, __popc(valid), 0, 0};
   const float uc = fminf(u_cand, tt.u_defer);
-  const float cmax = static_cast<float>(tt.na) - 1e-3f, tmax = static_cast<float>(tt.nq) - 1e-3f;
-  float sum = 0.0f, bkey = -1.0f;
-  int ntest = 0, nused = 0, bj = 0;
+  if (tt.lt_u && tab) {
+    const float u_tiny = tt.u_tiny, u_defer = tt.u_defer;
+    float uv[16];
 #pragma unroll
+    for (int j = 0; j < 16; ++j) uv[j] = u[j];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      const float uj = uv[j];
+      const bool v = (valid >> j) & 1u;
+      const float term = cubic_term(uj, tt, tab);
+      const bool lo = uj < u_tiny;
+      const bool use = v && !lo && uj < u_defer;
+      r.sum += use ? term : 0.0f;
+      r.used += use ? 1 : 0;
+      const float key = v ? uj : -1.0f;
+      r.j = key > r.score ? j : r.j;
+      r.score = fmaxf(key, r.score);
+    }
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      const bool lo = uv[j] < u_tiny;
+      if (((valid >> j) & 1u) && (uv[j] >= uc || (lo && uv[j] > 0.0f)))
+        emit_candidate(out, gene, s0 + j, lo || uv[j] >= u_defer, lo);
+    }
+    return r;
+  }
   for (int j = 0; j < 16; ++j) {
+    if (!((valid >> j) & 1u)) continue;
     const float uj = u[j];
-    const bool central = uj <= tt.uq0;
-    const float x = fminf(central ? uj * tt.dqc_inv : (uj - tt.uq0) * tt.dq_inv, central ? cmax : tmax);
-    const int i = static_cast<int>(x);
-    const float f = x - static_cast<float>(i);
-    const float4 a = (central ? tt.c1q : tt.ltq)[i];
-    const float y = fmaf(fmaf(fmaf(a.w, f, a.z), f, a.y), f, a.x);
-    const float term = central ? y * rsqrtf(uj) : y;
-    const bool lo = uj < tt.u_tiny;
-    const bool use = !lo && uj < tt.u_defer;
-    sum += use ? term : 0.0f;
-    nused += use ? 1 : 0;
-    ntest += valid[j] ? 1 : 0;
-    const float key = valid[j] ? uj : -1.0f;
-    bj = key > bkey ? j : bj;
-    bkey = fmaxf(key, bkey);
-    if (uj >= uc || (lo && uj > 0.0f)) emit_candidate(out, gene, s0 + j, lo || uj >= tt.u_defer, lo);
+    const ScreenOut o = acat_screen_u(uj, tt);
+    if (o.use_acat) {
+      r.sum += o.term;
+      ++r.used;
+    }
+    if (o.key > r.score) {
+      r.score = o.key;
+      r.j = j;
+    }
+    if (uj >= uc || o.deferred) emit_candidate(out, gene, s0 + j, o.deferred, o.tiny);
   }
-  acc.tested += ntest;
-  acc.used += nused;
-  acc.chunk_acat += sum;
-  if (bkey >= 0.0f && bkey > acc.chunk_key) {
-    acc.chunk_key = bkey;
-    acc.chunk_snp = static_cast<uint32_t>(s0 + bj);
-  }
-  acc.end_chunk();
+  return r;
 }
 
 // The same screen of 16 pairs that are all tested (no SNP of the block gated,
 // none out of scope), for tables in shared memory: u_of(j) gives u = t^2 of
 // pair j, computed without the guards of the general form. Returns false,
-// with acc untouched, unless every u lies in [u_tiny, u_hi), u_hi =
-// min(u_cand, u_defer): a pair near 0, a candidate, a NaN, and whatever the
-// guards would have caught (a vanishing denominator gives u < 0, NaN or inf)
-// are left to the general form.
+// with acc untouched, unless every u lies in [u_tiny, u_defer): a pair near 0 or
+// deferred, a NaN, and whatever the guards would have caught (a vanishing
+// denominator gives u < 0, NaN or inf) are left to the general form. u_of is
+// called twice for the pairs of a chunk with a candidate or with what may be the
+// gene's best.
 //
-// The scans' epilogues are bound by instruction issue, and ~97 % of the
+// The scans' epilogues are bound by instruction issue, and ~99 % of the
 // 16-pair chunks hold nothing but ordinary pairs, so the per-pair flags, the
 // candidate test, the counts and the best-SNP index leave the loop: the counts
 // are 16, the extremes decide for the chunk, and the index is looked for only
 // where the chunk's largest u reaches the best published for the gene. The
-// terms and the order of their sum are those of screen16_cubic.
+// terms and the order of their sum are those of the general form.
 template <class U>
-__device__ __forceinline__ bool screen16_fast(const TTable& tt, uint32_t tab, float u_hi, U&& u_of, int64_t s0,
-                                              GeneAcc& acc) {
+__device__ __forceinline__ bool screen16_fast(const TTable& tt, uint32_t tab, float u_cand, U&& u_of,
+                                              const GeneOut& out, int gene, int64_t s0, GeneAcc& acc) {
   float sum = 0.0f, umin = INFINITY, umax = 0.0f;
 #pragma unroll
   for (int j = 0; j < 16; j += 2) {
@@ -258,18 +251,20 @@ __device__ __forceinline__ bool screen16_fast(const TTable& tt, uint32_t tab, fl
     sum += cubic_term(ua, tt, tab);
     sum += cubic_term(ub, tt, tab);
   }
-  if (!(umin >= tt.u_tiny && umax < u_hi)) return false;
-  acc.tested += 16;
-  acc.used += 16;
-  acc.acat += static_cast<double>(sum);
-  if (umax >= acc.u_floor) {
-    uint32_t bj = 0;
+  if (!(umin >= tt.u_tiny && umax < tt.u_defer)) return false;
+  float score = -1.0f;
+  uint32_t bj = 0;
+  if (umax >= fminf(acc.u_floor, u_cand)) {
 #pragma unroll
-    for (int j = 15; j >= 0; --j) bj = u_of(j) == umax ? j : bj;  // the first pair with the largest u
-    const unsigned long long k = best_key(umax, static_cast<uint32_t>(s0) + bj);
-    acc.best = k < acc.best ? k : acc.best;
-    acc.u_floor = umax;
+    for (int j = 15; j >= 0; --j) {
+      const float u = u_of(j);
+      bj = u == umax ? j : bj;  // the first pair with the largest u
+      if (u >= u_cand) emit_candidate(out, gene, s0 + j, false, false);
+    }
+    score = umax;
+    acc.u_floor = fmaxf(acc.u_floor, umax);
   }
+  acc.add_chunk(16, 16, sum, score, static_cast<uint32_t>(s0) + bj);
   return true;
 }
 
@@ -278,12 +273,49 @@ __device__ __forceinline__ bool all_flags16(const uint32_t (&w)[4]) {
   return (w[0] & w[1] & w[2] & w[3]) == 0x01010101u;
 }
 
-// Whether every pair of the block of 16 SNPs at s0 is in scope for every gene
-// of the warp's active lanes: a gw scan, or a trans scan on a block clear of
-// all their windows (the vote keeps the warp on one path).
-__device__ __forceinline__ bool chunk_in_scope(const Windows& w, const GeneAcc& acc, int64_t s0) {
-  if (w.mode == kWinNone) return true;
-  return w.mode == kWinExclude && __all_sync(__activemask(), acc.chunk_clear(w, s0));
+// Scope of the block of 16 SNPs at s0 for the genes of the warp's active
+// lanes (the vote keeps the warp on one path): kAll (a gw scan; a trans scan on
+// a block clear of all their windows; a cis scan on a block inside all of them),
+// kNone (the reverse) or kMixed (decided per pair).
+enum ChunkScope : int { kScopeAll, kScopeNone, kScopeMixed };
+__device__ __forceinline__ ChunkScope chunk_scope(const Windows& w, const GeneAcc& acc, int64_t s0) {
+  if (w.mode == kWinNone) return kScopeAll;
+  const uint32_t m = __activemask();
+  const bool clear = __all_sync(m, acc.chunk_clear(w, s0));
+  if (clear) return w.mode == kWinExclude ? kScopeAll : kScopeNone;
+  const bool inside = __all_sync(m, acc.chunk_inside(w, s0));
+  if (inside) return w.mode == kWinExclude ? kScopeNone : kScopeAll;
+  return kScopeMixed;
+}
+
+// One chunk of 16 pairs through the two forms. ok: every SNP of the chunk is
+// tested and the fast form's denominators are sound; tab: cubic_base of the
+// tables in shared memory (0: none); u_fast(j): u without guards; u_gen(j, valid)
+// sets whether pair j is tested (its scope aside) and gives u with guards, never
+// NaN.
+template <class UF, class UG>
+__device__ __forceinline__ void screen_chunk(const TTable& tt, uint32_t tab, float u_cand, const Windows& win,
+                                             const GeneOut& out, int gene, int64_t s0, bool ok, UF&& u_fast,
+                                             UG&& u_gen, GeneAcc& acc) {
+  const ChunkScope sc = chunk_scope(win, acc, s0);
+  if (sc == kScopeNone) return;
+  if (ok && sc == kScopeAll && tab && tt.lt_u &&  // (tt.lt_u: uniform across the launch)
+      screen16_fast(tt, tab, u_cand, u_fast, out, gene, s0, acc))
+    return;
+  float u[16];
+  uint32_t valid = 0;
+#pragma unroll
+  for (int j = 0; j < 16; ++j) {
+    bool v = true;
+    u[j] = u_gen(j, v);
+    valid |= v ? 1u << j : 0u;
+  }
+  if (sc == kScopeMixed) {
+    const uint32_t in = acc.window_mask(win, s0);
+    valid &= win.mode == kWinExclude ? ~in : in;
+  }
+  const ChunkSums r = screen16_general(tt, tab, u, valid, u_cand, out, gene, s0);
+  acc.add_chunk(r.tested, r.used, r.sum, r.score, static_cast<uint32_t>(s0 + r.j));
 }
 
 }  // namespace dev

@@ -52,7 +52,6 @@ struct LmEpi {
   static constexpr int kSmemBytes = kTTableSmemBytes;
   const Params& P;
   float* tsm;
-  TTable tt;
   int gene = 0;
   int64_t snp0 = 0;
   bool gvalid = false;
@@ -62,10 +61,9 @@ struct LmEpi {
   GeneAcc acc;
 
   __device__ LmEpi(const Params& p, const TileShape&, uint8_t* smem)
-      : P(p), tsm(reinterpret_cast<float*>(smem)), tt(p.tt), u_cand(p.t_cand * p.t_cand) {}
+      : P(p), tsm(reinterpret_cast<float*>(smem)), u_cand(p.t_cand * p.t_cand) {}
   __device__ void init(int tid, int nthr) {
-    tt = screen_to_smem(P.tt, tsm, tid, nthr);
-    tab = cubic_base(smem_u32(tsm));
+    if (P.tt.lt_u) tab = screen_tables(P.tt, tsm, tid, nthr);
   }
   __device__ void begin_tile(int g, int64_t s0) {
     gene = g;
@@ -97,50 +95,25 @@ struct LmEpi {
       igv[4 * q + 2] = v4.z;
       igv[4 * q + 3] = v4.w;
     }
-    if (tt.lt_u) {  // uniform across the launch
-      float ig_min = igv[0];
+    float ig_min = igv[0];
 #pragma unroll
-      for (int j = 1; j < 15; j += 2) ig_min = min3(ig_min, igv[j], igv[j + 1]);
-      ig_min = fminf(ig_min, igv[15]);
-      // every SNP tested and with a residual variance, every pair in scope
-      if (ig_min > 0.0f && chunk_in_scope(P.win, acc, s0)) {
-        auto u_of = [&](int j) {
+    for (int j = 1; j < 15; j += 2) ig_min = min3(ig_min, igv[j], igv[j + 1]);
+    ig_min = fminf(ig_min, igv[15]);
+    // ig_min > 0: every SNP tested and with a residual variance
+    screen_chunk(
+        P.tt, tab, u_cand, P.win, P.out, gene, s0, ig_min > 0.0f,
+        [&](int j) {
           const float r = v[0][j] * v[0][j] * (igv[j] * w);
           return P.df * (r * rcp_ftz(1.0f - r));
-        };
-        if (screen16_fast(P.tt, tab, fminf(u_cand, P.tt.u_defer), u_of, s0, acc)) return;
-      }
-      chunk_cubic(s0, v[0], igv);
-      return;
-    }
-#pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      const int64_t s = s0 + j;
-      const bool valid = igv[j] >= 0.0f && acc.in_scope(P.win, s);
-      const float ig = valid ? igv[j] * w : 0.0f;
-      const float r = v[0][j] * v[0][j] * ig;
-      const float omr = 1.0f - r;
-      const float u = (ig > 0.0f && omr > 0.0f) ? P.df * __fdividef(r, omr) : 0.0f;  // t^2
-      const ScreenOut o = acat_screen_u(u, tt);
-      acc.add_screen(o, s, valid);
-      if (valid && (u >= u_cand || o.deferred)) emit_candidate(P.out, gene, s, o.deferred, o.tiny);
-    }
-    acc.end_chunk();
-  }
-  // The same screen with the per-interval cubics (screen16_cubic): u is
-  // never NaN here (a pair outside the scan or with p = 1 has u = 0).
-  __device__ void chunk_cubic(int64_t s0, const float (&v)[16], const float (&igv)[16]) {
-    float u[16];
-    bool valid[16];
-#pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      valid[j] = igv[j] >= 0.0f && acc.in_scope(P.win, s0 + j);
-      const float ig = valid[j] ? igv[j] * w : 0.0f;
-      const float r = v[j] * v[j] * ig;
-      const float omr = 1.0f - r;
-      u[j] = (ig > 0.0f && omr > 0.0f) ? P.df * __fdividef(r, omr) : 0.0f;  // t^2
-    }
-    screen16_cubic(tt, u, valid, u_cand, P.out, gene, s0, acc);
+        },
+        [&](int j, bool& tested) {
+          tested = igv[j] >= 0.0f;
+          const float ig = tested ? igv[j] * w : 0.0f;
+          const float r = v[0][j] * v[0][j] * ig;
+          const float omr = 1.0f - r;
+          return ig > 0.0f && omr > 0.0f ? P.df * __fdividef(r, omr) : 0.0f;  // t^2, never NaN
+        },
+        acc);
   }
   __device__ void end_tile() {
     if (gvalid) acc.flush(P.out, gene);

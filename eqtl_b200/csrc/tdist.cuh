@@ -245,13 +245,9 @@ __device__ __forceinline__ float max3_nan(float a, float b, float c) {
 // issue at an eighth of the rate of an add)
 constexpr float kFloorMagic = 8388608.0f;
 
-// Address operand of cubic_term for tables that screen_to_smem laid out at
-// the shared-memory address `sm`.
-__device__ __forceinline__ uint32_t cubic_base(uint32_t sm) { return sm - (0x4B000000u << 4); }
-
 // The ACAT term of one u in [u_tiny, u_defer), as the lt_u branch of
 // acat_screen_u forms it (the same bits; outside that range a meaningless
-// value, without reading past the tables). tab: cubic_base.
+// value, without reading past the tables). tab: screen_tables.
 __device__ __forceinline__ float cubic_term(float u, const TTable& T, uint32_t tab) {
   const float up = fminf(fabsf(u), T.u_defer);  // NaN: u_defer
   const bool central = up < T.uq0;
@@ -264,6 +260,14 @@ __device__ __forceinline__ float cubic_term(float u, const TTable& T, uint32_t t
   asm("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(a0), "=f"(a1), "=f"(a2), "=f"(a3) : "r"(addr));
   const float v = fmaf(fmaf(fmaf(a3, f, a2), f, a1), f, a0);
   return central ? v * rsqrt_ftz(up) : v;
+}
+
+// Copies the screen's cubics (T.lt_u) into shared memory as screen_to_smem does
+// and returns the address operand of cubic_term (never 0); the caller
+// synchronises before use.
+__device__ __forceinline__ uint32_t screen_tables(const TTable& T, float* sm, int tid, int nthr) {
+  screen_to_smem(T, sm, tid, nthr);
+  return static_cast<uint32_t>(__cvta_generic_to_shared(sm)) - (0x4B000000u << 4);
 }
 
 // Copies the t_tail tables into shared memory (cooperatively, by `nthr`

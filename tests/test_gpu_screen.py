@@ -71,3 +71,45 @@ def test_lm_screen_gate_in_chunk(gated):
     ora, ref = oracle_scan.trans_lm(dec.dosage[:, sub], Y[sub], X[sub], 1e-2)
     assert np.all(res[0]["n_tested"] == m - 1)
     check_scan(res, ora, ref, 1e-2, len(sub) - 2)
+
+
+@pytest.mark.parametrize("scope", [1, 2])
+@pytest.mark.parametrize("model,p", [("lm", 2), ("lmm", 1), ("lmm", 2), ("lmm", 4)])
+def test_screen_window_blocks(model, p, scope):
+    """Blocks of 16 SNPs inside every gene's window, clear of all of them, and
+    mixed (window edges and a chromosome's end inside a block), for genes with a
+    window over the whole chromosome, a part of it, one SNP, nothing, and no
+    location."""
+    from eqtl_b200 import capi, synth
+    n, G = 75, 70
+    rng = np.random.default_rng(7 + p)
+    per = [150, 89, 40]                      # chromosomes that end inside blocks
+    m = sum(per)
+    schrom = np.repeat(np.arange(3), per).astype(np.int32)
+    spos = np.concatenate([np.sort(rng.choice(np.arange(1, 4000), k, replace=False)) for k in per])
+    codes = rng.binomial(2, rng.uniform(0.15, 0.85, (m, 1)), (m, n)).astype(np.int8)
+    codes[:, :3] = [0, 1, 2]
+    gchrom = rng.integers(-1, 3, G).astype(np.int32)
+    lo = rng.integers(1, 4000, G)
+    hi = lo + rng.integers(0, 2500, G)
+    gchrom[:34], lo[:34], hi[:34] = 0, 1, 4000          # a warp whose genes share a window
+    hi[40] = lo[40] = spos[200]
+    gchrom[40] = schrom[200]
+    gchrom[41], lo[41], hi[41] = 1, 3990, 100
+    X = np.column_stack([np.ones(n), rng.standard_normal((n, p - 1))])
+    Y = rng.standard_normal((n, G))
+    win = (gchrom, lo, hi, schrom, spos, scope)
+    mask = oracle_scan.windows_mask(schrom, spos, gchrom, lo, hi)
+    excl = mask if scope == 1 else ~mask
+    with capi.Context(0) as c:
+        c.load_bed(synth.pack_bed_rows(codes), n, np.arange(n))
+        if model == "lm":
+            res = c.scan_trans_lm(Y, X, pthr=1e-2, windows=win)
+            ora, ref = oracle_scan.trans_lm(codes.astype(float), Y, X, 1e-2, excl=excl)
+        else:
+            Q, _ = np.linalg.qr(rng.standard_normal((n, n)))
+            lam = np.sort(rng.gamma(0.5, 2.0, n))
+            c.set_basis(Q, lam)
+            res = c.scan_trans_lmm(Y, X, pthr=1e-2, windows=win)
+            ora, ref = oracle_scan.trans_lmm(codes.astype(float), Y, X, Q, lam, 1e-2, excl=excl, deltas=res[3])
+    check_scan(res[:3], ora, ref, 1e-2, n - p - 1, rel=1e-9 if model == "lm" else 1e-6)
