@@ -294,11 +294,65 @@ dev::Windows upload_windows(eqtl_ctx* ctx, const eqtl_scan_params* prm, int64_t 
   return w;
 }
 
-// Banded tile list of a cis scan (scope 2): for every tile of 128 genes, the
+// Scans with windows (trans, cis) lay their genes out by window position, so
+// that the 32 genes of a warp and the 128 of a tile have windows close together:
+// a warp's 16-SNP blocks are then mostly in or out for all of its genes
+// (chunk_scope), and a cis tile's band covers few SNP tiles. In the caller's
+// order the windows of 32 genes scattered over the genome make over a quarter of
+// the blocks mixed, and the bands of 128 cover nearly every SNP. Consecutive
+// genes with the same window (permuted columns) stay together. Scans of genes in
+// random order, before and after: cis LMM (p = 16, 500 genes, 45,000 SNPs) 2.07 ->
+// 0.74 ms, cis LM (1,000 genes, 20,000 SNPs) 0.156 -> 0.093 ms, trans LM on dosages
+// (1.8e8 tests) 1.13 -> 0.79 ms. The order changes no pair's arithmetic.
+GeneOrder gene_order(eqtl_ctx* ctx, const eqtl_scan_params* prm) {
+  GeneOrder go;
+  const int G = prm->n_genes;
+  if (prm->exclude_cis == 0 || !prm->gene_chrom || !prm->gene_lo || !prm->gene_hi || !prm->snp_chrom ||
+      !prm->snp_pos)
+    return go;
+  struct Run {
+    uint32_t chrom;  // genes without a location (-1) last
+    int64_t lo;
+    int first, count;
+  };
+  std::vector<Run> runs;
+  for (int g = 0; g < G; ++g) {
+    const uint32_t c = static_cast<uint32_t>(prm->gene_chrom[g]);
+    if (g > 0 && prm->gene_chrom[g] == prm->gene_chrom[g - 1] && prm->gene_lo[g] == prm->gene_lo[g - 1] &&
+        prm->gene_hi[g] == prm->gene_hi[g - 1])
+      ++runs.back().count;
+    else
+      runs.push_back({c, prm->gene_lo[g], g, 1});
+  }
+  auto before = [](const Run& a, const Run& b) {
+    if (a.chrom != b.chrom) return a.chrom < b.chrom;
+    if (a.lo != b.lo) return a.lo < b.lo;
+    return a.first < b.first;
+  };
+  if (std::is_sorted(runs.begin(), runs.end(), before)) return go;
+  std::sort(runs.begin(), runs.end(), before);
+  Workspace& ws = ctx->ws;
+  std::vector<int> gene(static_cast<size_t>(G));
+  ws.gene_row_h.resize(static_cast<size_t>(G));
+  int r = 0;
+  for (const Run& run : runs)
+    for (int k = 0; k < run.count; ++k, ++r) {
+      gene[static_cast<size_t>(r)] = run.first + k;
+      ws.gene_row_h[static_cast<size_t>(run.first + k)] = r;
+    }
+  ws.row_gene.upload(gene.data(), gene.size(), ctx->stream);
+  ws.gene_row.upload(ws.gene_row_h.data(), ws.gene_row_h.size(), ctx->stream);
+  go.row = ws.gene_row.p;
+  go.gene = ws.row_gene.p;
+  return go;
+}
+
+// Banded tile list of a cis scan (scope 2): for every tile of 128 operand rows, the
 // SNP tiles of NT kept SNPs that hold some gene's window. Needs the kept
 // SNPs grouped by chromosome in position order (as in a sorted .bim); returns
 // false otherwise, and the caller runs the full grid masked to the windows.
-bool cis_tile_list(eqtl_ctx* ctx, const eqtl_scan_params* prm, int64_t m, int NT, const int2*& list, int& n_list) {
+bool cis_tile_list(eqtl_ctx* ctx, const eqtl_scan_params* prm, const GeneOrder& go, int64_t m, int NT,
+                   const int2*& list, int& n_list) {
   list = nullptr;
   n_list = 0;
   if (prm->exclude_cis != 2 || !prm->gene_chrom || !prm->snp_chrom || !prm->snp_pos || m == 0) return false;
@@ -326,7 +380,8 @@ bool cis_tile_list(eqtl_ctx* ctx, const eqtl_scan_params* prm, int64_t m, int NT
     const int64_t k_lo = std::lower_bound(p0, p1, prm->gene_lo[g]) - prm->snp_pos;
     const int64_t k_hi = std::upper_bound(p0, p1, prm->gene_hi[g]) - prm->snp_pos;  // exclusive
     if (k_hi <= k_lo) continue;
-    uint8_t* row = &mark[static_cast<size_t>(g / dev::kTileM) * tiles_b];
+    const int r = go.row ? ctx->ws.gene_row_h[static_cast<size_t>(g)] : g;
+    uint8_t* row = &mark[static_cast<size_t>(r / dev::kTileM) * tiles_b];
     for (int64_t tb = k_lo / NT; tb <= (k_hi - 1) / NT; ++tb) row[tb] = 1;
   }
   std::vector<int2> tl;

@@ -221,6 +221,8 @@ struct Workspace {
   DevBuf<eqtl_pair> refined;
   DevBuf<double> tiny_p;
   DevBuf<int2> tile_list;
+  DevBuf<int> gene_row, row_gene;      // GeneOrder of the current scan
+  std::vector<int> gene_row_h;
   DevBuf<__half> q_hi, q_lo;  // rotation: split eigenvector operand
   DevBuf<int> ref_snps, ref_col;
   DevBuf<int2> ref_pairs;

@@ -869,10 +869,12 @@ __global__ void __launch_bounds__(kRbThreads)
 // the accumulators back into NUM, a_k, gg.
 __global__ void lmm_gene_ops_kernel(const double* __restrict__ Ytil, const double* __restrict__ Xtil,
                                     const double* __restrict__ lam, const double* __restrict__ delta,
-                                    const double* __restrict__ chi0, int n, int p, int G, int k_pad, float s1,
-                                    float s2, __half* const* hi, __half* const* lo, float* unscale) {
+                                    const double* __restrict__ chi0, int n, int p, int G,
+                                    const int* __restrict__ gene_row, int k_pad, float s1, float s2,
+                                    __half* const* hi, __half* const* lo, float* unscale) {
   const int g = blockIdx.x;
   if (g >= G) return;
+  const int64_t row = gene_row ? gene_row[g] : g;  // operand row
   const int nops = p + 2;
   __shared__ double mx[kMaxPLmm + 2][8];
   __shared__ double sc[kMaxPLmm + 2];
@@ -916,8 +918,8 @@ __global__ void lmm_gene_ops_kernel(const double* __restrict__ Ytil, const doubl
     for (int i = threadIdx.x; i < k_pad; i += blockDim.x) {
       const double v = value(op, i) * s;
       const __half h = __double2half(v);
-      hi[op][static_cast<int64_t>(g) * k_pad + i] = h;
-      lo[op][static_cast<int64_t>(g) * k_pad + i] = __double2half(v - static_cast<double>(__half2float(h)));
+      hi[op][row * k_pad + i] = h;
+      lo[op][row * k_pad + i] = __double2half(v - static_cast<double>(__half2float(h)));
     }
   }
 }
@@ -957,10 +959,12 @@ __global__ void lmm_uv_w_kernel(const double* __restrict__ Ytil, const double* _
 // SNP operand holds its imputed mean, which centres each SNP inside the
 // contraction.
 __global__ void lmm_gene_ops_raw_kernel(const double* __restrict__ UV, const double* __restrict__ lam,
-                                        const double* __restrict__ delta, int n, int p, int G, int k_pad, float s2,
-                                        __half* const* hi, __half* const* lo, float* unscale) {
+                                        const double* __restrict__ delta, int n, int p, int G,
+                                        const int* __restrict__ gene_row, int k_pad, float s2, __half* const* hi,
+                                        __half* const* lo, float* unscale) {
   const int g = blockIdx.x;
   if (g >= G) return;
+  const int64_t row = gene_row ? gene_row[g] : g;  // operand row
   const int nops = p + 2;
   __shared__ double mx[kMaxPLmm + 2][8];
   __shared__ double sc[kMaxPLmm + 2];
@@ -995,8 +999,8 @@ __global__ void lmm_gene_ops_raw_kernel(const double* __restrict__ UV, const dou
   __syncthreads();
   for (int op = 0; op < nops; ++op) {
     const double s = sc[op];
-    __half* h_row = hi[op] + static_cast<int64_t>(g) * k_pad;
-    __half* l_row = lo[op] + static_cast<int64_t>(g) * k_pad;
+    __half* h_row = hi[op] + row * k_pad;
+    __half* l_row = lo[op] + row * k_pad;
     double sum = 0.0;
     for (int i = threadIdx.x; i < k_pad; i += blockDim.x) {
       const double v = value(op, i) * s;
@@ -1025,6 +1029,7 @@ __global__ void lmm_gene_ops_raw_kernel(const double* __restrict__ UV, const dou
 template <int P>
 struct LmmEpiParams {
   int G;
+  const int* order;         // GeneOrder::gene
   int64_t m;
   const float* unscale;     // [G][P+2]
   const double* ainv;       // [G][P][P]
@@ -1110,10 +1115,10 @@ struct LmmEpi {
   __device__ void init(int tid, int nthr) {
     if (tsm && Pr.tt.lt_u) tab = screen_tables(Pr.tt, tsm, tid, nthr);
   }
-  __device__ void begin_tile(int g, int64_t s0) {
-    gene = g;
+  __device__ void begin_tile(int row, int64_t s0) {
     snp0 = s0;
-    gvalid = g < Pr.G;
+    gvalid = row < Pr.G;
+    const int g = gene = gvalid && Pr.order ? __ldg(Pr.order + row) : row;
     if constexpr (GLM) gvalid = gvalid && Pr.gene_ok[g];  // a failed null fit tests nothing
     acc.reset();
     if (gvalid) {
@@ -1402,7 +1407,7 @@ constexpr double kLrSpan = 3.0;  // longest interval of ln(delta)
 // inverse as the unscale of gg (kind 0) and a_k (kind 1 + k).
 __global__ void lr_coef_kernel(const double* __restrict__ delta, int G, const double* __restrict__ node_a,
                                double a0, double h, int nint, const float* __restrict__ sigma, int kn, int kb,
-                               int P, __half* hi, __half* lo, float* unscale) {
+                               int P, const int* __restrict__ gene_row, __half* hi, __half* lo, float* unscale) {
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= G) return;
   double a = log(fmax(delta[g], 1e-300));
@@ -1426,8 +1431,9 @@ __global__ void lr_coef_kernel(const double* __restrict__ delta, int G, const do
     for (int j = 0; j < kLrNodes; ++j)
       if (sg[j] != 0.0f) mx = fmax(mx, fabs(l[j] / static_cast<double>(sg[j])));
     const double sc = mx > 0.0 ? ldexp(1.0, 10 - ilogb(mx)) : 1.0;
-    __half* hr = hi + static_cast<int64_t>(g) * kb + kind * kn + base;
-    __half* lr = lo + static_cast<int64_t>(g) * kb + kind * kn + base;
+    const int64_t row = gene_row ? gene_row[g] : g;
+    __half* hr = hi + row * kb + kind * kn + base;
+    __half* lr = lo + row * kb + kind * kn + base;
 #pragma unroll
     for (int j = 0; j < kLrNodes; ++j) {
       const double y = sg[j] != 0.0f ? l[j] / static_cast<double>(sg[j]) * sc : 0.0;
@@ -1450,10 +1456,11 @@ __global__ void lr_coef_kernel(const double* __restrict__ delta, int G, const do
 __global__ void lmm_gene_ops_orth_kernel(const double* __restrict__ Ytil, const double* __restrict__ Xtil,
                                          const double* __restrict__ lam, const double* __restrict__ delta,
                                          const double* __restrict__ chi0, const double* __restrict__ ainv, int n,
-                                         int p, int G, int k_pad, float s1, float s2, __half* const* hi,
-                                         __half* const* lo, float* unscale) {
+                                         int p, int G, const int* __restrict__ gene_row, int k_pad, float s1,
+                                         float s2, __half* const* hi, __half* const* lo, float* unscale) {
   const int g = blockIdx.x;
   if (g >= G) return;
+  const int64_t row = gene_row ? gene_row[g] : g;  // operand row
   const int nops = p + 2;
   __shared__ double mx[kMaxPLmm + 2][8];
   __shared__ double sc[kMaxPLmm + 2];
@@ -1516,14 +1523,15 @@ __global__ void lmm_gene_ops_orth_kernel(const double* __restrict__ Ytil, const 
     for (int i = threadIdx.x; i < k_pad; i += blockDim.x) {
       const double v = value(op, i) * s;
       const __half h = __double2half(v);
-      hi[op][static_cast<int64_t>(g) * k_pad + i] = h;
-      lo[op][static_cast<int64_t>(g) * k_pad + i] = __double2half(v - static_cast<double>(__half2float(h)));
+      hi[op][row * k_pad + i] = h;
+      lo[op][row * k_pad + i] = __double2half(v - static_cast<double>(__half2float(h)));
     }
   }
 }
 
 struct LmmGroupEpiParams {
   int G;
+  const int* order;         // GeneOrder::gene
   int64_t m;
   int n_acc;                // p + 2
   const float* unscale;     // [G][n_acc]: NUM, gg, a~_0 .. a~_{p-1}
@@ -1563,10 +1571,10 @@ struct LmmGroupEpiT {
   __device__ void init(int tid, int nthr) {
     if (Pr.tt.lt_u) tab = screen_tables(Pr.tt, tsm, tid, nthr);
   }
-  __device__ void begin_tile(int g, int64_t s0) {
-    gene = g;
+  __device__ void begin_tile(int row, int64_t s0) {
     snp0 = s0;
-    gvalid = g < Pr.G;
+    gvalid = row < Pr.G;
+    const int g = gene = gvalid && Pr.order ? __ldg(Pr.order + row) : row;
     if constexpr (GLM) gvalid = gvalid && Pr.gene_ok[g];
     acc.reset();
     if (gvalid) {
@@ -2433,7 +2441,7 @@ static bool lmm_lr_wanted(int G) {
 // ws.unscale of gg and a_k). Returns false, leaving the direct form, when
 // the intervals would be longer than kLrSpan.
 template <int P>
-static bool lmm_lr_build(eqtl_ctx* ctx, int n, int G, float s2) {
+static bool lmm_lr_build(eqtl_ctx* ctx, int n, int G, const int* gene_row, float s2) {
   Workspace& ws = ctx->ws;
   const Geno& g = ctx->geno;
   const Rotated& R = ctx->rot;
@@ -2502,8 +2510,8 @@ static bool lmm_lr_build(eqtl_ctx* ctx, int n, int G, float s2) {
   ws.lr_ops_ptr.upload(nptr, 2 * nops, st);
   ws.lr_unscale.alloc(static_cast<size_t>(nn) * nops);
   ++ctx->launches;
-  lmm_gene_ops_raw_kernel<<<nn, 256, 0, st>>>(ws.lr_uv.p, ctx->basis.lambda.p, ws.lr_delta.p, n, P, nn, k_pad, s2,
-                                              ws.lr_ops_ptr.p, ws.lr_ops_ptr.p + nops, ws.lr_unscale.p);
+  lmm_gene_ops_raw_kernel<<<nn, 256, 0, st>>>(ws.lr_uv.p, ctx->basis.lambda.p, ws.lr_delta.p, n, P, nn, nullptr, k_pad,
+                                              s2, ws.lr_ops_ptr.p, ws.lr_ops_ptr.p + nops, ws.lr_unscale.p);
   EQTL_CUDA(cudaGetLastError());
 
   // node pass: accumulators [gg, a_0 ..] against Gt^2 and the raw operand
@@ -2556,7 +2564,7 @@ static bool lmm_lr_build(eqtl_ctx* ctx, int n, int G, float s2) {
   ws.lr_clo.zero(st);
   ++ctx->launches;
   lr_coef_kernel<<<(G + 127) / 128, 128, 0, st>>>(ws.delta.p, G, ws.lr_a.p, lo, h, nint, ws.lr_sigma.p, kn, kb, P,
-                                                  ws.lr_chi.p, ws.lr_clo.p, ws.unscale.p);
+                                                  gene_row, ws.lr_chi.p, ws.lr_clo.p, ws.unscale.p);
   EQTL_CUDA(cudaGetLastError());
   return true;
 }
@@ -2564,9 +2572,9 @@ static bool lmm_lr_build(eqtl_ctx* ctx, int n, int G, float s2) {
 // lmm_lr_build, or the direct form when its tables do not fit in device
 // memory beside the scan's operands (their large buffers are given back).
 template <int P>
-static bool lmm_lr_prepare(eqtl_ctx* ctx, int n, int G, float s2) {
+static bool lmm_lr_prepare(eqtl_ctx* ctx, int n, int G, const int* gene_row, float s2) {
   try {
-    return lmm_lr_build<P>(ctx, n, G, s2);
+    return lmm_lr_build<P>(ctx, n, G, gene_row, s2);
   } catch (const Error& e) {
     if (e.code != EQTL_E_NOMEM) throw;
     EQTL_CUDA(cudaStreamSynchronize(ctx->stream));
@@ -2661,6 +2669,7 @@ static void scan_trans_lmm_impl(eqtl_ctx* ctx, const eqtl_scan_params* prm, cons
   lmm_prep(ctx, ph, prm->y_rotated != 0);
 
   // gene-side operands
+  const GeneOrder go = gene_order(ctx, prm);
   const int k_pad = g.k_pad;
   const int nops = p + 2;
   float s1, s2;
@@ -2689,15 +2698,15 @@ static void scan_trans_lmm_impl(eqtl_ctx* ctx, const eqtl_scan_params* prm, cons
                            ctx->basis.Q.p, n, ws.lmm_w.p, n, &zero, ws.lmm_uv.p, n) == CUBLAS_STATUS_SUCCESS,
                EQTL_E_CUDA, "Q (w o [r~, X~]) failed");
     ctx->launches += 1;
-    lmm_gene_ops_raw_kernel<<<G, 256, 0, st>>>(ws.lmm_uv.p, ctx->basis.lambda.p, ws.delta.p, n, p, G, k_pad, s2,
-                                               ws.ops_ptr.p, ws.ops_ptr.p + nops, unscale.p);
+    lmm_gene_ops_raw_kernel<<<G, 256, 0, st>>>(ws.lmm_uv.p, ctx->basis.lambda.p, ws.delta.p, n, p, G, go.row, k_pad,
+                                               s2, ws.ops_ptr.p, ws.ops_ptr.p + nops, unscale.p);
   } else if (grouped) {
     lmm_gene_ops_orth_kernel<<<G, 256, 0, st>>>(ws.Ytil.p, ws.Xtil.p, ctx->basis.lambda.p, ws.delta.p, ws.chi0.p,
-                                                ws.ainv.p, n, p, G, k_pad, s1, s2, ws.ops_ptr.p,
+                                                ws.ainv.p, n, p, G, go.row, k_pad, s1, s2, ws.ops_ptr.p,
                                                 ws.ops_ptr.p + nops, unscale.p);
   } else {
     lmm_gene_ops_kernel<<<G, 256, 0, st>>>(ws.Ytil.p, ws.Xtil.p, ctx->basis.lambda.p, ws.delta.p, ws.chi0.p, n, p, G,
-                                           k_pad, s1, s2, ws.ops_ptr.p, ws.ops_ptr.p + nops, unscale.p);
+                                           go.row, k_pad, s1, s2, ws.ops_ptr.p, ws.ops_ptr.p + nops, unscale.p);
   }
   EQTL_CUDA(cudaGetLastError());
   // dense scans with the exact operand: gg and a_k interpolated between node
@@ -2705,7 +2714,7 @@ static void scan_trans_lmm_impl(eqtl_ctx* ctx, const eqtl_scan_params* prm, cons
   bool lr = false;
   ws.lr_nodes = 0;
   if (raw && prm->exclude_cis != 2 && lmm_lr_wanted(G))
-    lr = p == 1 ? lmm_lr_prepare<1>(ctx, n, G, s2) : lmm_lr_prepare<2>(ctx, n, G, s2);
+    lr = p == 1 ? lmm_lr_prepare<1>(ctx, n, G, go.row, s2) : lmm_lr_prepare<2>(ctx, n, G, go.row, s2);
   if (simt) {
     // the FP32 form's gene-side operands, in the tile's accumulator order
     // [gg, a_0 .. a_{p-1}, NUM] (the gene-ops order is [NUM, a.., gg])
@@ -2730,12 +2739,13 @@ static void scan_trans_lmm_impl(eqtl_ctx* ctx, const eqtl_scan_params* prm, cons
   ScanOutputs so(ctx, G, m, expected_candidates(prm, m));
   const int2* tiles = nullptr;  // cis: banded tile list (NT of the kernel that runs)
   int n_tiles = 0;
-  if (!simt) cis_tile_list(ctx, prm, m, grouped ? LmmGroupEpi::kTileN : 128, tiles, n_tiles);
+  if (!simt) cis_tile_list(ctx, prm, go, m, grouped ? LmmGroupEpi::kTileN : 128, tiles, n_tiles);
   std::unique_ptr<StageScope> scan_timer(new StageScope(ctx, EQTL_STAGE_SCAN));
   if (m > 0 && grouped) {
     Rotated& Rt = ctx->rot;
     LmmGroupEpiParams ep{};
     ep.G = G;
+    ep.order = go.gene;
     ep.m = m;
     ep.n_acc = nops;
     ep.unscale = unscale.p;
@@ -2771,6 +2781,7 @@ static void scan_trans_lmm_impl(eqtl_ctx* ctx, const eqtl_scan_params* prm, cons
     const __half* al[4] = {oph[nops + 0], oph[nops + 1], oph[nops + 2], nops > 3 ? oph[nops + 3] : oph[nops + 2]};
     auto fill = [&](auto& ep) {
       ep.G = G;
+      ep.order = go.gene;
       ep.m = m;
       ep.unscale = unscale.p;
       ep.ainv = ws.ainv.p;
@@ -3075,10 +3086,11 @@ __global__ void __launch_bounds__(kGlmThreads)
 // (X'WX)^-1; each scaled to a power of two and split into FP16 hi + lo.
 __global__ void glm_gene_ops_kernel(const double* __restrict__ W, const double* __restrict__ Rr,
                                     const double* __restrict__ X, const double* __restrict__ ainv, int n, int p, int G,
-                                    int k_pad, float s1, float s2, int grouped, __half* const* hi, __half* const* lo,
-                                    float* unscale) {
+                                    const int* __restrict__ gene_row, int k_pad, float s1, float s2, int grouped,
+                                    __half* const* hi, __half* const* lo, float* unscale) {
   const int g = blockIdx.x;
   if (g >= G) return;
+  const int64_t row = gene_row ? gene_row[g] : g;  // operand row
   const int nops = p + 2;
   __shared__ double mx[kMaxPLmm + 2][8];
   __shared__ double sc[kMaxPLmm + 2];
@@ -3135,8 +3147,8 @@ __global__ void glm_gene_ops_kernel(const double* __restrict__ W, const double* 
     for (int i = threadIdx.x; i < k_pad; i += blockDim.x) {
       const double v = value(op, i) * sv;
       const __half h = __double2half(v);
-      hi[op][static_cast<int64_t>(g) * k_pad + i] = h;
-      lo[op][static_cast<int64_t>(g) * k_pad + i] = __double2half(v - static_cast<double>(__half2float(h)));
+      hi[op][row * k_pad + i] = h;
+      lo[op][row * k_pad + i] = __double2half(v - static_cast<double>(__half2float(h)));
     }
   }
 }
@@ -3336,8 +3348,9 @@ void scan_glm(eqtl_ctx* ctx, const eqtl_scan_params* prm, const double* Y, const
   }
   ws.ops_ptr.upload(oph.data(), oph.size(), st);
   ws.unscale.alloc(static_cast<size_t>(G) * nops);
+  const GeneOrder go = gene_order(ctx, prm);
   ++ctx->launches;
-  glm_gene_ops_kernel<<<G, 256, 0, st>>>(ws.glm_w.p, ws.glm_r.p, ph.X.p, ws.ainv.p, n, p, G, k_pad, s1, s2,
+  glm_gene_ops_kernel<<<G, 256, 0, st>>>(ws.glm_w.p, ws.glm_r.p, ph.X.p, ws.ainv.p, n, p, G, go.row, k_pad, s1, s2,
                                          grouped ? 1 : 0, ws.ops_ptr.p, ws.ops_ptr.p + nops, ws.unscale.p);
   EQTL_CUDA(cudaGetLastError());
   lmm_gate(ctx);
@@ -3351,11 +3364,12 @@ void scan_glm(eqtl_ctx* ctx, const eqtl_scan_params* prm, const double* Y, const
   ScanOutputs so(ctx, G, m, expected_candidates(prm, m));
   const int2* tiles = nullptr;
   int n_tiles = 0;
-  cis_tile_list(ctx, prm, m, grouped ? GlmGroupEpi::kTileN : 128, tiles, n_tiles);
+  cis_tile_list(ctx, prm, go, m, grouped ? GlmGroupEpi::kTileN : 128, tiles, n_tiles);
   std::unique_ptr<StageScope> scan_timer(new StageScope(ctx, EQTL_STAGE_SCAN));
   if (m > 0 && grouped) {
     GlmGroupEpiParams ep{};
     ep.G = G;
+    ep.order = go.gene;
     ep.m = m;
     ep.n_acc = nops;
     ep.unscale = ws.unscale.p;
@@ -3380,6 +3394,7 @@ void scan_glm(eqtl_ctx* ctx, const eqtl_scan_params* prm, const double* Y, const
     const __half* al[4] = {oph[nops + 0], oph[nops + 1], oph[nops + 2], nops > 3 ? oph[nops + 3] : oph[nops + 2]};
     auto fill = [&](auto& ep) {
       ep.G = G;
+      ep.order = go.gene;
       ep.m = m;
       ep.unscale = ws.unscale.p;
       ep.ainv = ws.ainv.p;

@@ -35,7 +35,16 @@ dev::Windows upload_windows(eqtl_ctx* ctx, const eqtl_scan_params* prm, int64_t 
 // Device tables of the two-sided t tail with `df` residual degrees of
 // freedom, or of the normal tail (normal = true; df is then ignored).
 dev::TTable device_ttable(eqtl_ctx* ctx, double df, bool normal = false);
-bool cis_tile_list(eqtl_ctx* ctx, const eqtl_scan_params* prm, int64_t m, int NT, const int2*& list, int& n_list);
+// The order in which a scan's genes take the gene-side operand rows (device
+// arrays; null: gene g has row g).
+struct GeneOrder {
+  const int* row = nullptr;   // [G] operand row of a gene
+  const int* gene = nullptr;  // [G] gene of an operand row
+};
+GeneOrder gene_order(eqtl_ctx* ctx, const eqtl_scan_params* prm);
+
+bool cis_tile_list(eqtl_ctx* ctx, const eqtl_scan_params* prm, const GeneOrder& go, int64_t m, int NT,
+                   const int2*& list, int& n_list);
 
 // Resolves the phenotypes of a scan call: uploads (Y, X) when given,
 // otherwise checks the resident ones match the call's shape.

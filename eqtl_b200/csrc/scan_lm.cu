@@ -31,6 +31,7 @@ namespace dev {
 
 struct LmEpiParams {
   int G;
+  const int* order;        // GeneOrder::gene
   int64_t m;
   const double* inv_yty;   // [G] 1 / yty (0 when yty == 0)
   const float* gscale;     // [G] gene-side factor of the accumulator -> gty
@@ -65,10 +66,10 @@ struct LmEpi {
   __device__ void init(int tid, int nthr) {
     if (P.tt.lt_u) tab = screen_tables(P.tt, tsm, tid, nthr);
   }
-  __device__ void begin_tile(int g, int64_t s0) {
-    gene = g;
+  __device__ void begin_tile(int row, int64_t s0) {
     snp0 = s0;
-    gvalid = g < P.G;
+    gvalid = row < P.G;
+    const int g = gene = gvalid && P.order ? __ldg(P.order + row) : row;
     acc.reset();
     if (gvalid) {
       const float gs = P.gscale[g];
@@ -140,10 +141,12 @@ __global__ void lm_igs_kernel(const double* __restrict__ inv_gtg, const uint8_t*
 // ---------------------------------------------------------------- prep
 // One block per gene: yty, power-of-two scale, FP16/BF16 hi/lo rows.
 template <class T>
-__global__ void gene_split_kernel(const double* __restrict__ Ys, int n, int k_pad, int G, T* hi, T* lo,
+__global__ void gene_split_kernel(const double* __restrict__ Ys, int n, int k_pad, int G,
+                                  const int* __restrict__ gene_row, T* hi, T* lo,
                                   float* gscale, double* yty_out, double* inv_yty, float snp_scale) {
   const int g = blockIdx.x;
   if (g >= G) return;
+  const int64_t row = gene_row ? gene_row[g] : g;  // operand row
   const double* y = Ys + static_cast<int64_t>(g) * n;
   __shared__ double red[32];
   __shared__ double redm[32];
@@ -189,8 +192,8 @@ __global__ void gene_split_kernel(const double* __restrict__ Ys, int n, int k_pa
       h = __double2bfloat16(v);
       l = __double2bfloat16(v - static_cast<double>(__bfloat162float(h)));
     }
-    hi[static_cast<int64_t>(g) * k_pad + k] = h;
-    lo[static_cast<int64_t>(g) * k_pad + k] = l;
+    hi[row * k_pad + k] = h;
+    lo[row * k_pad + k] = l;
   }
   if (threadIdx.x == 0) {
     gscale[g] = static_cast<float>(1.0 / (sc * snp_scale));
@@ -410,6 +413,7 @@ void scan_trans_lm(eqtl_ctx* ctx, const eqtl_scan_params* prm, const double* Y, 
   ws.XtY.alloc(static_cast<size_t>(p) * G);
   residualize_genes(ctx, ph.X.p, ws.XtXinv.p, n, p, G, ws.Ys.p, ws.XtY.p);  // Ys <- Y - X beta
 
+  const GeneOrder go = gene_order(ctx, prm);
   const int k_pad = g.k_pad;
   DevBuf<__half>& a_hi = ws.ops_hi[0];
   DevBuf<__half>& a_lo = ws.ops_lo[0];
@@ -426,12 +430,12 @@ void scan_trans_lm(eqtl_ctx* ctx, const eqtl_scan_params* prm, const double* Y, 
   const bool raw = !bf16 && geno_raw_operand(ctx);
   ++ctx->launches;
   if (bf16)
-    gene_split_kernel<__nv_bfloat16><<<G, 256, 0, st>>>(ws.Ys.p, n, k_pad, G,
+    gene_split_kernel<__nv_bfloat16><<<G, 256, 0, st>>>(ws.Ys.p, n, k_pad, G, go.row,
                                                         reinterpret_cast<__nv_bfloat16*>(a_hi.p),
                                                         reinterpret_cast<__nv_bfloat16*>(a_lo.p), ws.gscale.p,
                                                         ws.yty.p, ws.inv_yty.p, kGcScale);
   else
-    gene_split_kernel<__half><<<G, 256, 0, st>>>(ws.Ys.p, n, k_pad, G, a_hi.p, a_lo.p, ws.gscale.p, ws.yty.p,
+    gene_split_kernel<__half><<<G, 256, 0, st>>>(ws.Ys.p, n, k_pad, G, go.row, a_hi.p, a_lo.p, ws.gscale.p, ws.yty.p,
                                                  ws.inv_yty.p, raw ? 1.0f : kGcScale);
   EQTL_CUDA(cudaGetLastError());
 
@@ -449,6 +453,7 @@ void scan_trans_lm(eqtl_ctx* ctx, const eqtl_scan_params* prm, const double* Y, 
   if (prm->perm_thr > 0) t_cand = std::min(t_cand, t_critical(prm->perm_thr, df));
   LmEpiParams ep{};
   ep.G = G;
+  ep.order = go.gene;
   ep.m = m;
   ep.inv_yty = ws.inv_yty.p;
   ep.gscale = ws.gscale.p;
@@ -469,7 +474,7 @@ void scan_trans_lm(eqtl_ctx* ctx, const eqtl_scan_params* prm, const double* Y, 
   ScanOutputs so(ctx, G, m, expected_candidates(prm, m));
   const int2* tiles = nullptr;  // cis: banded tile list
   int n_tiles = 0;
-  cis_tile_list(ctx, prm, m, 256, tiles, n_tiles);
+  cis_tile_list(ctx, prm, go, m, 256, tiles, n_tiles);
   std::unique_ptr<StageScope> scan_timer(new StageScope(ctx, EQTL_STAGE_SCAN));
   if (m > 0) {
     so.run([&](GeneOut out) {
@@ -544,7 +549,7 @@ void test_pairs_lm(eqtl_ctx* ctx, const eqtl_scan_params* prm, const double* Y, 
   ws.inv_yty.alloc(G);
   ws.yty.alloc(G);
   ++ctx->launches;
-  gene_split_kernel<__half><<<G, 256, 0, st>>>(ws.Ys.p, n, k_pad, G, ws.ops_hi[0].p, ws.ops_lo[0].p, ws.gscale.p,
+  gene_split_kernel<__half><<<G, 256, 0, st>>>(ws.Ys.p, n, k_pad, G, nullptr, ws.ops_hi[0].p, ws.ops_lo[0].p, ws.gscale.p,
                                                ws.yty.p, ws.inv_yty.p, kGcScale);
   EQTL_CUDA(cudaGetLastError());
   const int64_t m = g.m;
