@@ -225,6 +225,7 @@ struct Workspace {
   std::vector<int> gene_row_h;
   DevBuf<__half> q_hi, q_lo;  // rotation: split eigenvector operand
   DevBuf<int> ref_snps, ref_col;
+  DevBuf<__half> qg_dose, qg_mask;  // exact_qg: dosages of the listed SNPs, mask of their missing calls
   DevBuf<int2> ref_pairs;
   // batched REML (p > 3): covariate pair products, per-round weights and sums
   DevBuf<double> rb_P, rb_dlt, rb_W, rb_WY, rb_A, rb_B, rb_ld, rb_ydy;
@@ -284,6 +285,10 @@ struct LmmBasisDev {
   DevBuf<double> Q;        // [n, n] column-major (column j = eigenvector j)
   DevBuf<double> lambda;   // [n]
   std::vector<double> Q_h, lambda_h;
+  // the digits of Q (exact_qg) and their scales, made when first needed
+  bool sliced = false;
+  DevBuf<__half> digits;
+  DevBuf<double> digit_scale;
 };
 
 }  // namespace eqtl

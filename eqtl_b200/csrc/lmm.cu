@@ -1682,6 +1682,144 @@ __global__ void raw_dosage_kernel(GenoRows src, const int32_t* __restrict__ col,
   }
 }
 
+// ------------------------------------- exact Q'g on the tensor cores
+// Gt = Q'g of the listed SNPs in FP64, for 2-bit rows: the dosages are 0, 1 or
+// 2, so with each eigenvector cut into digits of 12 bits
+//     q_i 2^s = d_1 + d_2 / 4096 + ... + d_5 / 4096^4,   d_k integers, |d_k| <= 2048
+// every sum over i of d_k g_i is an integer of at most 4096 n < 2^24 (n <=
+// kQgMaxN) and therefore exact in the tensor cores' FP32 accumulators. The five
+// sums of an eigenvector meet in FP64. The digits cover 2^-60 of the
+// eigenvector's largest entry, so the result is at least as close to the exact
+// sum as a DGEMM's, whose products and partial sums round. Missing calls are 0
+// in g; a second pass contracts the 0 / 1 mask of missing calls and adds mu
+// times its sums. The DGEMM this replaces was half of the refinement: n = 2000,
+// 52,000 SNPs QG_FIGS.
+// Digit rows: eigenvector j has rows 16 (j / 3) + 5 (j % 3) + k, so 16 rows hold
+// three whole eigenvectors (and one zero row).
+constexpr int kQgDigits = 5;
+constexpr int kQgMaxN = 4095;
+// From this n^2 u on (a DGEMM of 0.6 ms): below, the digits, the passes' launches
+// and their status checks cost what they save (n = 1,201, 2,400 SNPs: refinement
+// 0.74 ms with the DGEMM, 0.76 without).
+constexpr int64_t kQgMinWork = int64_t(10) << 30;
+__host__ __device__ constexpr int64_t qg_rows(int n) { return static_cast<int64_t>((n + 2) / 3) * 16; }
+
+__global__ void __launch_bounds__(256)
+    q_digits_kernel(const double* __restrict__ Q, int n, int k_pad, __half* out, double* scale) {
+  __shared__ double red[8];
+  const int j = blockIdx.x;
+  const double* q = Q + static_cast<int64_t>(j) * n;
+  double mx = 0.0;
+  for (int i = threadIdx.x; i < n; i += 256) mx = fmax(mx, fabs(q[i]));
+  for (int o = 16; o; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
+  __syncthreads();
+  mx = red[0];
+  for (int w = 1; w < 8; ++w) mx = fmax(mx, red[w]);
+  const int e = mx > 0 ? 10 - ilogb(mx) : 0;  // the largest entry times 2^e lies in [1024, 2048)
+  if (threadIdx.x == 0) scale[j] = ldexp(1.0, -e);
+  __half* rows = out + (static_cast<int64_t>(j / 3) * 16 + (j % 3) * kQgDigits) * k_pad;
+  for (int i = threadIdx.x; i < k_pad; i += 256) {
+    double x = i < n ? ldexp(q[i], e) : 0.0;
+#pragma unroll
+    for (int k = 0; k < kQgDigits; ++k) {
+      const double d = rint(x);
+      rows[static_cast<int64_t>(k) * k_pad + i] = __double2half(d);
+      x = (x - d) * 4096.0;  // exact
+    }
+  }
+}
+
+// Dosages of the listed kept SNPs as FP16 rows (missing calls 0) and the mask
+// of missing calls (mask null: not wanted), one warp per SNP.
+__global__ void __launch_bounds__(256)
+    listed_dosage_kernel(GenoRows src, const int32_t* __restrict__ col, int n, int k_pad,
+                         const int64_t* __restrict__ kept, const int* __restrict__ snps, int u, __half* dose,
+                         __half* mask) {
+  const int lane = threadIdx.x & 31;
+  const int c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (c >= u) return;
+  const int64_t s = kept[snps[c]];
+  for (int k0 = lane * 8; k0 < k_pad; k0 += 256) {
+    uint32_t dw[4] = {0, 0, 0, 0}, mw[4] = {0, 0, 0, 0};
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int k = k0 + j;
+      const double d = k < n ? src.dosage(s, __ldg(col + k)) : 0.0;
+      if (isnan(d)) mw[j / 2] |= 0x3C00u << (16 * (j & 1));  // 1.0
+      else dw[j / 2] |= static_cast<uint32_t>(__half_as_ushort(__double2half(d))) << (16 * (j & 1));
+    }
+    const int64_t o = static_cast<int64_t>(c) * k_pad + k0;
+    *reinterpret_cast<uint4*>(dose + o) = make_uint4(dw[0], dw[1], dw[2], dw[3]);
+    if (mask) *reinterpret_cast<uint4*>(mask + o) = make_uint4(mw[0], mw[1], mw[2], mw[3]);
+  }
+}
+
+// Rows = digit rows, columns = listed SNPs; out[c * n + j] = the five digit sums
+// of eigenvector j, or += mu_c times them (the mask's pass). The digits of an eigenvector lie in five neighbouring lanes,
+// so a warp passes its 32 x 16 accumulators through shared memory and each lane
+// forms three outputs, consecutive lanes those of consecutive eigenvectors: no
+// conversion to FP64 (8 issue cycles a warp) is done twice, and a column is
+// stored as 48 contiguous bytes.
+struct QgEpiParams {
+  int n, u;
+  const double* scale;  // [n]
+  const double* mu;     // [m_all] imputation means (null: the dosages' pass)
+  const int64_t* kept;
+  const int* snps;
+  double* out;
+};
+
+struct QgEpi {
+  static constexpr bool kGrouped = false;
+  static constexpr int kWarpFloats = 32 * 16;  // row r, column i at 16 r + (i ^ (r % 16))
+  static constexpr int kSmemBytes = kEpiWarps * kWarpFloats * 4;
+  using Params = QgEpiParams;
+  const Params& P;
+  float* buf;
+  int64_t c0 = 0;
+  int j0 = 0;  // the warp's first eigenvector
+  __device__ QgEpi(const Params& p, const TileShape&, uint8_t* smem)
+      : P(p), buf(reinterpret_cast<float*>(smem) + ((threadIdx.x >> 5) - 2) * kWarpFloats) {}
+  __device__ void init(int, int) {}
+  __device__ void begin_tile(int row, int64_t col) {
+    c0 = col;
+    j0 = 3 * (row / 32) * 2;
+  }
+  template <int NACC>
+  __device__ void chunk(int cc, const float (&v)[NACC][16]) {
+    const int lane = threadIdx.x & 31;
+    __syncwarp();  // the previous chunk has been read
+#pragma unroll
+    for (int i = 0; i < 16; ++i) buf[lane * 16 + (i ^ (lane & 15))] = v[0][i];
+    __syncwarp();
+    double* dst[3];
+    double x[3], mu[3], before[3];
+#pragma unroll
+    for (int t = 0; t < 3; ++t) {
+      const int o = lane + 32 * t, i = o / 6, e = o % 6;  // column i, eigenvector j0 + e
+      const int64_t c = c0 + cc + i;
+      dst[t] = c < P.u && j0 + e < P.n ? P.out + c * P.n + j0 + e : nullptr;
+      if (P.mu && dst[t]) {
+        mu[t] = P.mu[P.kept[P.snps[c]]];
+        before[t] = *dst[t];
+      }
+      const float* b = buf + 256 * (e / 3);
+      const int r0 = kQgDigits * (e % 3);
+      auto digit = [&](int k) { return static_cast<double>(b[(r0 + k) * 16 + (i ^ (r0 + k))]); };
+      x[t] = digit(kQgDigits - 1);
+#pragma unroll
+      for (int k = kQgDigits - 2; k >= 0; --k) x[t] = fma(x[t], 1.0 / 4096.0, digit(k));
+      if (dst[t]) x[t] *= P.scale[j0 + e];
+    }
+#pragma unroll
+    for (int t = 0; t < 3; ++t)
+      if (dst[t]) *dst[t] = P.mu ? fma(mu[t], x[t], before[t]) : x[t];
+  }
+  __device__ void end_tile() {}
+  __device__ void finish() {}
+};
+
 // One warp per (gene, snp) pair from the FP64 rotated raw dosage Gt = Q'g:
 // gg = Gt'W Gt, yg = Gt'W y~, a = X~'W Gt with W = diag(1 / (delta lambda + 1)),
 // then the pair's printed statistics (test_lmm_gtil, src/scan_trans_lmm.cpp:11-40).
@@ -1806,6 +1944,10 @@ __global__ void lmm_tiny_kernel(GenoRows src, const int32_t* __restrict__ col, i
 template <>
 struct EpiOf<dev::RotEpiParams> {
   using type = dev::RotEpi;
+};
+template <>
+struct EpiOf<dev::QgEpiParams> {
+  using type = dev::QgEpi;
 };
 template <>
 struct EpiOf<dev::LmmEpiParams<1>> {
@@ -1938,6 +2080,7 @@ void lmm_basis_from_grm(eqtl_ctx* ctx, const double* K_dev, int n, double sparsi
   for (double& l : B.lambda_h) l = std::max(l, 0.0);  // cwiseMax(0.0)
   B.lambda.upload(B.lambda_h.data(), n, st);
   B.Q_h.clear();
+  B.sliced = false;
   ctx->have_basis = true;
   ctx->rot.m = 0;  // rotated genotypes belong to the previous basis
 }
@@ -1955,6 +2098,7 @@ void lmm_set_basis(eqtl_ctx* ctx, const double* Q, const double* lambda, int n) 
   for (double& l : B.lambda_h) l = std::max(l, 0.0);
   B.lambda.upload(B.lambda_h.data(), n, ctx->stream);
   EQTL_CUDA(cudaStreamSynchronize(ctx->stream));
+  B.sliced = false;
   ctx->have_basis = true;
   ctx->rot.m = 0;
 }
@@ -2321,9 +2465,55 @@ static void lmm_launch_simt(eqtl_ctx* ctx, const LmmEpiParams<P>& ep, const __ha
   EQTL_CUDA(cudaStreamSynchronize(st));
 }
 
+// Q'g of the listed SNPs (snps; on the device in ws.ref_snps) from their exact
+// dosages by the digits of Q, into out [u][n].
+static void exact_qg(eqtl_ctx* ctx, const std::vector<int>& snps, double* out) {
+  const Geno& g = ctx->geno;
+  Workspace& ws = ctx->ws;
+  LmmBasisDev& B = ctx->basis;
+  cudaStream_t st = ctx->stream;
+  const int n = g.n, k_pad = g.k_pad, u = static_cast<int>(snps.size());
+  const int64_t rows = qg_rows(n);
+  if (!B.sliced) {
+    B.digits.alloc(static_cast<size_t>(rows) * k_pad);
+    B.digit_scale.alloc(static_cast<size_t>(n));
+    B.digits.zero(st);  // the rows that hold no digit
+    ++ctx->launches;
+    q_digits_kernel<<<n, 256, 0, st>>>(B.Q.p, n, k_pad, B.digits.p, B.digit_scale.p);
+    EQTL_CUDA(cudaGetLastError());
+    B.sliced = true;
+  }
+  // (over the load's samples, of which a view has a part)
+  const bool any_missing = std::any_of(snps.begin(), snps.end(), [&](int r) {
+    return g.n_miss_h[static_cast<size_t>(g.kept_h[static_cast<size_t>(r)])] > 0;
+  });
+  ws.qg_dose.alloc(static_cast<size_t>(u) * k_pad);
+  if (any_missing) ws.qg_mask.alloc(static_cast<size_t>(u) * k_pad);
+  ++ctx->launches;
+  listed_dosage_kernel<<<(u + 7) / 8, 256, 0, st>>>(g.rows(), g.col.p, n, k_pad, g.kept.p, ws.ref_snps.p, u,
+                                                    ws.qg_dose.p, any_missing ? ws.qg_mask.p : nullptr);
+  EQTL_CUDA(cudaGetLastError());
+  QgEpiParams ep{n, u, B.digit_scale.p, nullptr, g.kept.p, ws.ref_snps.p, out};
+  auto pass = [&](const __half* snp_side) {
+    const __half* ap[1] = {B.digits.p};
+    const __half* bp[1] = {snp_side};
+    const int bsel[1] = {0}, prod[1] = {1};
+    if (tile_pairs(rows))
+      launch_tile_n<256, 1, QgEpiParams, dev::kBLoNone, 2>(ctx, false, ep, ap, ap, rows, bp, bp, u, k_pad, bsel, prod);
+    else
+      launch_tile_n<256, 1, QgEpiParams, dev::kBLoNone>(ctx, false, ep, ap, ap, rows, bp, bp, u, k_pad, bsel, prod);
+  };
+  pass(ws.qg_dose.p);
+  if (any_missing) {
+    ep.mu = g.mu.p;
+    pass(ws.qg_mask.p);
+  }
+}
+
 // FP64 statistics of (gene, kept SNP) pairs against the current LMM prep
-// (ws.Ytil, Xtil, delta, chi0, ainv, rss): raw dosages of the SNPs involved,
-// Gt = Q'g by DGEMM, then one warp per pair (lmm_refine_kernel).
+// (ws.Ytil, Xtil, delta, chi0, ainv, rss): Gt = Q'g of the SNPs involved (exactly
+// on the tensor cores for many 2-bit rows, else by DGEMM: FP32 dosages, more than
+// kQgMaxN samples, little work), then one warp per pair (lmm_refine_kernel).
 static std::vector<eqtl_pair> lmm_refine_pairs(eqtl_ctx* ctx, int p, double df, const std::vector<int2>& todo) {
   Geno& g = ctx->geno;
   Workspace& ws = ctx->ws;
@@ -2353,17 +2543,22 @@ static std::vector<eqtl_pair> lmm_refine_pairs(eqtl_ctx* ctx, int p, double df, 
     dpc.upload(pcol.data(), pcol.size(), st);
     dtodo.upload(todo.data(), todo.size(), st);
     tr.mark("host index + upload");
-    DevBuf<double>& graw = ws.graw;
     DevBuf<double>& gt = ws.gt;
-    graw.alloc(static_cast<size_t>(n) * u);
     gt.alloc(static_cast<size_t>(n) * u);
-    ctx->launches += 2;
-    raw_dosage_kernel<<<1184, 256, 0, st>>>(g.rows(), g.col.p, n, g.kept.p, g.mu.p, dsn.p, u, graw.p);
-    EQTL_CUDA(cudaGetLastError());
-    const double one = 1.0, zero = 0.0;
-    EQTL_CHECK(cublasDgemm(blas_of(ctx), CUBLAS_OP_T, CUBLAS_OP_N, n, u, n, &one, ctx->basis.Q.p, n, graw.p, n, &zero,
-                           gt.p, n) == CUBLAS_STATUS_SUCCESS,
-               EQTL_E_CUDA, "Q'g failed");
+    if (!g.dense && n <= kQgMaxN && static_cast<int64_t>(n) * n * u >= kQgMinWork) {
+      exact_qg(ctx, snps, gt.p);
+    } else {
+      DevBuf<double>& graw = ws.graw;
+      graw.alloc(static_cast<size_t>(n) * u);
+      ++ctx->launches;
+      raw_dosage_kernel<<<1184, 256, 0, st>>>(g.rows(), g.col.p, n, g.kept.p, g.mu.p, dsn.p, u, graw.p);
+      EQTL_CUDA(cudaGetLastError());
+      const double one = 1.0, zero = 0.0;
+      EQTL_CHECK(cublasDgemm(blas_of(ctx), CUBLAS_OP_T, CUBLAS_OP_N, n, u, n, &one, ctx->basis.Q.p, n, graw.p, n,
+                             &zero, gt.p, n) == CUBLAS_STATUS_SUCCESS,
+                 EQTL_E_CUDA, "Q'g failed");
+    }
+    ++ctx->launches;
     ws.refined.alloc(todo.size());
     lmm_refine_kernel<<<static_cast<unsigned>((todo.size() + 7) / 8), 256, 0, st>>>(
         gt.p, n, dpc.p, dtodo.p, static_cast<int>(todo.size()), ws.Ytil.p, ws.Xtil.p, p, ctx->basis.lambda.p,
