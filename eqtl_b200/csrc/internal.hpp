@@ -203,8 +203,16 @@ struct PhenoDev {
   std::vector<double> X_h;
 };
 
+// PEER: the table, its factors and loadings, per-gene moments.
+struct PeerWork {
+  DevBuf<double> Yraw, Y, XtY, E2, W, epsW, X, T1, XE2S, W_E2S, W_Xprec, Xcov, Alpha, Eps, b1, b2, part;
+  DevBuf<int> fail;
+};
+
 // Per-call workspaces reused across calls (capacity grows, never shrinks).
 struct Workspace {
+  DevBuf<double> int_y;  // --pheno-norm int: the table
+  PeerWork peer;
   DevBuf<double> Ytil, Xtil, Ys, XtY, XtXinv, delta, chi0, ainv, a00L, rss, gtg, inv_gtg, af_sub, inv_yty, yty;
   DevBuf<__half> ops_hi[34], ops_lo[34];  // gene-side operands, one per accumulator (dev::kMaxAcc)
   DevBuf<__half> opsb_hi[34], opsb_lo[34];  // the same re-split into BF16 hi + lo (split-BF16 LMM scans)

@@ -251,11 +251,14 @@ int peer_factors(eqtl_ctx* ctx, const double* Y_host, int n, int G, int K, int m
   cublasHandle_t h = peer_blas(ctx);
   const int KK = K * K;
   const int64_t nG = static_cast<int64_t>(n) * G;
-  DevBuf<double> Yraw, Y, R, XtY, E2, W, epsW, X, T1, XE2S, W_E2S, W_Xprec, Xcov, Alpha, Eps, b1, b2, part;
-  DevBuf<int> fail;
+  PeerWork& w = ctx->ws.peer;
+  auto &Yraw = w.Yraw, &Y = w.Y, &XtY = w.XtY, &E2 = w.E2, &W = w.W, &epsW = w.epsW, &X = w.X, &T1 = w.T1,
+       &XE2S = w.XE2S, &W_E2S = w.W_E2S, &W_Xprec = w.W_Xprec, &Xcov = w.Xcov, &Alpha = w.Alpha, &Eps = w.Eps,
+       &b1 = w.b1, &b2 = w.b2, &part = w.part;
+  auto& R = w.Yraw;  // the residual takes the place of the uploaded table, which is only centred from
+  DevBuf<int>& fail = w.fail;
   Yraw.upload(Y_host, static_cast<size_t>(nG), st);
   Y.alloc(static_cast<size_t>(nG));
-  R.alloc(static_cast<size_t>(nG));
   XtY.alloc(static_cast<size_t>(K) * G);
   E2.alloc(static_cast<size_t>(G) * KK);
   W.upload(W0, static_cast<size_t>(G) * K, st);

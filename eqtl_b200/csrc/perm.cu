@@ -9,8 +9,9 @@
 // so that no permuted column is built on the host or crosses PCIe: column
 // c = g * B + b gets the keys
 //     key_i = (philox(seed, gene_key[g]; b, i) << 32) | i,   i < n
-// and the permutation is the order of the keys (a segmented radix sort of
-// all columns at once). The 32 random bits make every order equally likely
+// and the permutation is the order of the keys (sorted by one block per column,
+// or for more than 4096 samples by a segmented radix sort of all columns at
+// once). The 32 random bits make every order equally likely
 // up to ties, which the index bits break (a tie among n keys has
 // probability about n^2 / 2^33). The permuted column is then
 //     LM   base_g[perm(i)]
@@ -25,7 +26,9 @@
 #include <cub/device/device_segmented_radix_sort.cuh>
 
 #include <algorithm>
+#include <type_traits>
 
+#include "block_sort.cuh"
 #include "internal.hpp"
 
 namespace eqtl {
@@ -45,6 +48,36 @@ __device__ __forceinline__ U4 philox4x32_10(U4 c, uint32_t k0, uint32_t k1) {
     k1 += 0xBB67AE85u;
   }
   return c;
+}
+
+// One permuted column per block: thread t draws the keys of samples 4 t .. 4 t + 3
+// with one Philox call, the block sorts them in registers and shared memory, and
+// the column is written once. Bound by the sort's instruction issue (figures in
+// block_sort.cuh).
+template <int T>
+__global__ void __launch_bounds__(T)
+    perm_block_kernel(int n, int B, uint64_t seed, const uint64_t* __restrict__ gene_key,
+                      const double* __restrict__ base, const double* __restrict__ xb0,
+                      const double* __restrict__ dinv, double* Y) {
+  __shared__ uint64_t sm[4 * T];
+  const int64_t c = blockIdx.x;
+  const int64_t g = c / B;
+  const uint32_t b = static_cast<uint32_t>(c - g * B);
+  const uint64_t gk = gene_key[g];
+  const U4 w = philox4x32_10(U4{b, threadIdx.x, static_cast<uint32_t>(gk), static_cast<uint32_t>(gk >> 32)},
+                             static_cast<uint32_t>(seed), static_cast<uint32_t>(seed >> 32));
+  const uint32_t rw[4] = {w.x, w.y, w.z, w.w};
+  uint64_t k[4];
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    const uint32_t i = 4 * threadIdx.x + r;
+    k[r] = i < static_cast<uint32_t>(n) ? (static_cast<uint64_t>(rw[r]) << 32) | i : ~0ull;  // padding last
+  }
+  dev::block_sort_u64<T>(k, sm);
+  for (int i = threadIdx.x; i < n; i += T) {
+    const double v = base[g * n + static_cast<uint32_t>(sm[i])];
+    Y[c * n + i] = xb0 ? xb0[g * n + i] + v / sqrt(fmax(dinv[g * n + i], 1e-12)) : v;
+  }
 }
 
 // keys of every column: one Philox call gives the random words of four
@@ -114,9 +147,6 @@ void pheno_permute(eqtl_ctx* ctx, const double* base, const double* xb0, const d
     ws.perm_dinv.upload(dinv, gn, st);
   }
   ws.perm_gkey.upload(gene_key, static_cast<size_t>(G), st);
-  ws.perm_keys.alloc(static_cast<size_t>(total));
-  ws.perm_sorted.alloc(static_cast<size_t>(total));
-  ws.perm_off.alloc(static_cast<size_t>(cols) + 1);
   PhenoDev& P = ctx->pheno;
   P.Y.alloc(static_cast<size_t>(total));
   P.X.upload(X, static_cast<size_t>(n) * p, st);
@@ -124,28 +154,43 @@ void pheno_permute(eqtl_ctx* ctx, const double* base, const double* xb0, const d
   P.n = n;
   P.G = static_cast<int>(cols);
   P.p = p;
-  const int64_t quads = cols * ((n + 3) / 4);
-  const unsigned grid = static_cast<unsigned>(std::min<int64_t>((quads + 255) / 256, int64_t(ctx->sm_count) * 16));
-  const unsigned ogrid = static_cast<unsigned>(std::min<int64_t>((cols + 256) / 256, int64_t(ctx->sm_count) * 16));
-  ctx->launches += 2;
-  perm_keys_kernel<<<grid, 256, 0, st>>>(n, B, cols, seed, ws.perm_gkey.p, ws.perm_keys.p);
-  perm_offsets_kernel<<<ogrid, 256, 0, st>>>(cols, n, ws.perm_off.p);
-  EQTL_CUDA(cudaGetLastError());
-  // the random word is bits 32..63; the radix sort is stable, so equal words
-  // keep the index order of bits 0..31
-  size_t temp_bytes = 0;
-  EQTL_CUDA(cub::DeviceSegmentedRadixSort::SortKeys(nullptr, temp_bytes, ws.perm_keys.p, ws.perm_sorted.p,
-                                                    static_cast<int>(total), static_cast<int>(cols), ws.perm_off.p,
-                                                    ws.perm_off.p + 1, 32, 64, st));
-  ws.perm_temp.alloc(temp_bytes);
-  EQTL_CUDA(cub::DeviceSegmentedRadixSort::SortKeys(ws.perm_temp.p, temp_bytes, ws.perm_keys.p, ws.perm_sorted.p,
-                                                    static_cast<int>(total), static_cast<int>(cols), ws.perm_off.p,
-                                                    ws.perm_off.p + 1, 32, 64, st));
-  ++ctx->launches;
-  const unsigned ggrid = static_cast<unsigned>(std::min<int64_t>((total + 255) / 256, int64_t(ctx->sm_count) * 16));
-  perm_gather_kernel<<<ggrid, 256, 0, st>>>(n, B, cols, ws.perm_sorted.p, ws.perm_base.p,
-                                            xb0 ? ws.perm_xb0.p : nullptr, xb0 ? ws.perm_dinv.p : nullptr, P.Y.p);
-  EQTL_CUDA(cudaGetLastError());
+  const double* d_xb0 = xb0 ? ws.perm_xb0.p : nullptr;
+  const double* d_dinv = xb0 ? ws.perm_dinv.p : nullptr;
+  if (n <= dev::kBlockSortMax) {
+    ++ctx->launches;
+    dev::with_sort_block(n, [&](auto tc) {
+      constexpr int T = decltype(tc)::value;
+      perm_block_kernel<T><<<static_cast<unsigned>(cols), T, 0, st>>>(n, B, seed, ws.perm_gkey.p, ws.perm_base.p,
+                                                                      d_xb0, d_dinv, P.Y.p);
+    });
+    EQTL_CUDA(cudaGetLastError());
+  } else {
+    ws.perm_keys.alloc(static_cast<size_t>(total));
+    ws.perm_sorted.alloc(static_cast<size_t>(total));
+    ws.perm_off.alloc(static_cast<size_t>(cols) + 1);
+    const int64_t quads = cols * ((n + 3) / 4);
+    const unsigned grid = static_cast<unsigned>(std::min<int64_t>((quads + 255) / 256, int64_t(ctx->sm_count) * 16));
+    const unsigned ogrid = static_cast<unsigned>(std::min<int64_t>((cols + 256) / 256, int64_t(ctx->sm_count) * 16));
+    ctx->launches += 2;
+    perm_keys_kernel<<<grid, 256, 0, st>>>(n, B, cols, seed, ws.perm_gkey.p, ws.perm_keys.p);
+    perm_offsets_kernel<<<ogrid, 256, 0, st>>>(cols, n, ws.perm_off.p);
+    EQTL_CUDA(cudaGetLastError());
+    // the random word is bits 32..63; the radix sort is stable, so equal words
+    // keep the index order of bits 0..31
+    size_t temp_bytes = 0;
+    EQTL_CUDA(cub::DeviceSegmentedRadixSort::SortKeys(nullptr, temp_bytes, ws.perm_keys.p, ws.perm_sorted.p,
+                                                      static_cast<int>(total), static_cast<int>(cols), ws.perm_off.p,
+                                                      ws.perm_off.p + 1, 32, 64, st));
+    ws.perm_temp.alloc(temp_bytes);
+    EQTL_CUDA(cub::DeviceSegmentedRadixSort::SortKeys(ws.perm_temp.p, temp_bytes, ws.perm_keys.p, ws.perm_sorted.p,
+                                                      static_cast<int>(total), static_cast<int>(cols), ws.perm_off.p,
+                                                      ws.perm_off.p + 1, 32, 64, st));
+    ++ctx->launches;
+    const unsigned ggrid = static_cast<unsigned>(std::min<int64_t>((total + 255) / 256, int64_t(ctx->sm_count) * 16));
+    perm_gather_kernel<<<ggrid, 256, 0, st>>>(n, B, cols, ws.perm_sorted.p, ws.perm_base.p,
+                                              d_xb0, d_dinv, P.Y.p);
+    EQTL_CUDA(cudaGetLastError());
+  }
   if (Y_out) P.Y.download(Y_out, static_cast<size_t>(total), st);
   EQTL_CUDA(cudaStreamSynchronize(st));
 }

@@ -5,14 +5,17 @@
 // Per column: the finite values are ranked (ties share the average of their
 // 1-based positions), and value i becomes qnorm_inv((rank_i - 1/2) / nf),
 // nf = number of finite values; values that are not finite stay as they are,
-// and a column with at most one finite value is left unchanged. All columns
-// are sorted at once by a segmented radix sort (keys: the values, with every
-// value that is not finite mapped to +inf so that the finite ones lead each
-// segment; items: the sample index); one thread per sorted entry then finds
-// its tie group by binary search in the sorted segment and writes the
-// transformed value back at the sample's position.
+// and a column with at most one finite value is left unchanged. Columns of up
+// to 4096 values are sorted by one block each (block_sort.cuh); longer ones all
+// at once by a segmented radix sort (keys: the values, with every value that is
+// not finite mapped to +inf so that the finite ones lead each segment; items: the
+// sample index). An entry finds its tie group by binary search in its sorted
+// column.
 #include <cub/device/device_segmented_radix_sort.cuh>
 
+#include <type_traits>
+
+#include "block_sort.cuh"
 #include "internal.hpp"
 #include "stats64.hpp"
 
@@ -70,6 +73,50 @@ __global__ void int_apply_kernel(const double* __restrict__ sorted, const int* _
   }
 }
 
+// Integers in the order of the doubles: both zeros alike, +inf above every
+// finite value.
+__device__ __forceinline__ uint64_t ordered_bits(double v) {
+  const uint64_t b = static_cast<uint64_t>(__double_as_longlong(v == 0.0 ? 0.0 : v));
+  return b >> 63 ? ~b : b | 0x8000000000000000ull;
+}
+
+// first position in sorted[0, len) whose key is at least / above k
+__device__ __forceinline__ int key_pos(const uint64_t* s, int len, uint64_t k, bool above) {
+  int lo = 0, hi = len;
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (above ? s[mid] <= k : s[mid] < k) lo = mid + 1;
+    else hi = mid;
+  }
+  return lo;
+}
+
+// One column per block, in place: the keys alone are sorted, since every entry
+// finds its own rank.
+template <int T>
+__global__ void __launch_bounds__(T) int_block_kernel(int n, double* Y) {
+  __shared__ uint64_t sm[4 * T];
+  double* y = Y + static_cast<int64_t>(blockIdx.x) * n;
+  const uint64_t inf = ordered_bits(__longlong_as_double(0x7ff0000000000000LL));
+  uint64_t k[4], mine[4];
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    const int i = static_cast<int>(threadIdx.x) + T * r;
+    const double v = i < n ? y[i] : 0.0;
+    k[r] = mine[r] = i < n && isfinite(v) ? ordered_bits(v) : inf;  // the rest (and padding) last
+  }
+  dev::block_sort_u64<T>(k, sm);
+  const int nf = key_pos(sm, n, inf, false);
+  if (nf <= 1) return;
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    if (mine[r] == inf) continue;  // not finite: unchanged
+    const int first = key_pos(sm, nf, mine[r], false), last = key_pos(sm, nf, mine[r], true);
+    const double rank = 0.5 * static_cast<double>(first + 1 + last);
+    y[static_cast<int>(threadIdx.x) + T * r] = normal_quantile((rank - 0.5) / static_cast<double>(nf));
+  }
+}
+
 }  // namespace
 
 void pheno_int(eqtl_ctx* ctx, double* Y_host, int n, int G) {
@@ -78,9 +125,21 @@ void pheno_int(eqtl_ctx* ctx, double* Y_host, int n, int G) {
              "pheno_int: more than 2^31 values in one call");
   cudaStream_t st = ctx->stream;
   const int64_t total = static_cast<int64_t>(n) * G;
-  DevBuf<double> y, keys, keys_out;
-  DevBuf<int> idx, idx_out, off;
+  DevBuf<double>& y = ctx->ws.int_y;
   y.upload(Y_host, static_cast<size_t>(total), st);
+  if (n <= dev::kBlockSortMax) {
+    ++ctx->launches;
+    dev::with_sort_block(n, [&](auto tc) {
+      constexpr int T = decltype(tc)::value;
+      int_block_kernel<T><<<static_cast<unsigned>(G), T, 0, st>>>(n, y.p);
+    });
+    EQTL_CUDA(cudaGetLastError());
+    y.download(Y_host, static_cast<size_t>(total), st);
+    EQTL_CUDA(cudaStreamSynchronize(st));
+    return;
+  }
+  DevBuf<double> keys, keys_out;
+  DevBuf<int> idx, idx_out, off;
   keys.alloc(static_cast<size_t>(total));
   keys_out.alloc(static_cast<size_t>(total));
   idx.alloc(static_cast<size_t>(total));
