@@ -1450,9 +1450,15 @@ __global__ void lr_coef_kernel(const double* __restrict__ delta, int G, const do
 // a' A00^-1 a = |U' a|^2 and U' a = Gt'(w o X~U): each covariate column
 // becomes one plain accumulator a~_k = Gt'(w o (X~U)_k), and
 //     S = gg - sum_k a~_k^2.
-// The p + 2 accumulators [NUM, gg, a~_0 .. a~_{p-1}] exceed what TMEM holds
-// for one tile, so the tile kernel runs them in groups of four; this
-// epilogue keeps NUM and the running S of its 16 pairs across the groups.
+// The p + 2 accumulators exceed what TMEM holds for one tile, so the tile kernel
+// runs them in groups of two, in the order [gg, a~_0 .. a~_{p-1}, NUM]: this
+// epilogue keeps only the running S of its pairs across the groups, and NUM ends
+// the tile. Tiles are 128 SNPs wide: per K chunk of an accumulator (12 MMAs) an SM
+// then moves 160 KB through shared memory for 128 x 128 pairs, or 120 KB on SM
+// pairs, where the 64-wide tiles that NUM and S of a thread once limited it to
+// moved 120 KB for half as many; shared memory's 128 bytes a cycle is what bounds
+// the kernel. NB-GLM scan (n = 1000, p = 3, 2e8 tests) 6.3 -> 5.2 ms (1.15 PFLOP/s
+// issued), LMM scan (n = 1000, p = 6, 2e8 tests) 10.0 -> 7.8 ms (1.23 PFLOP/s).
 __global__ void lmm_gene_ops_orth_kernel(const double* __restrict__ Ytil, const double* __restrict__ Xtil,
                                          const double* __restrict__ lam, const double* __restrict__ delta,
                                          const double* __restrict__ chi0, const double* __restrict__ ainv, int n,
@@ -1534,7 +1540,7 @@ struct LmmGroupEpiParams {
   const int* order;         // GeneOrder::gene
   int64_t m;
   int n_acc;                // p + 2
-  const float* unscale;     // [G][n_acc]: NUM, gg, a~_0 .. a~_{p-1}
+  const float* unscale;     // [G][n_acc]: NUM, gg, a~_0 .. a~_{p-1} (the gene-ops order)
   const double* rss_null;   // [G]
   const uint8_t* snp_ok;    // [m]
   Windows win;
@@ -1552,7 +1558,9 @@ struct GlmGroupEpiParams : LmmGroupEpiParams {};
 template <bool GLM>
 struct LmmGroupEpiT {
   static constexpr bool kGrouped = true;
-  static constexpr int kTileN = 64;  // one 16-column chunk per epilogue thread
+  static constexpr int kTileN = 128;
+  static constexpr int kGroup = 2;      // accumulators per group: two groups in TMEM
+  static constexpr int kMaxChunks = 2;  // 16-column chunks per warp and tile
   using Params = std::conditional_t<GLM, GlmGroupEpiParams, LmmGroupEpiParams>;
   static constexpr int kSmemBytes = kTTableSmemBytes;
   const Params& Pr;
@@ -1562,7 +1570,9 @@ struct LmmGroupEpiT {
   bool gvalid = false;
   float inv_rss = 0;
   float rs = 0;  // GLM: sum_i r_i of the gene
-  float num[16], S[16];
+  // running S per pair of the warp's two chunks; two named arrays picked by a
+  // select, so they stay in registers for a runtime ci
+  float S0[16], S1[16];
   float u_cand;  // t_cand^2
   uint32_t tab = 0;  // screen_tables (0: none)
   GeneAcc acc;
@@ -1589,50 +1599,56 @@ struct LmmGroupEpiT {
     }
   }
   // accumulator j of this tile for the 16 columns at c
-  __device__ void acc_chunk(int j, int c, const float (&v)[16]) {
+  __device__ void acc_chunk(int j, int ci, int c, const float (&v)[16]) {
     if (!gvalid) return;
-    const float us = Pr.unscale[static_cast<int64_t>(gene) * Pr.n_acc + j];
+    const float* us = Pr.unscale + static_cast<int64_t>(gene) * Pr.n_acc;
+    if (j == Pr.n_acc - 1) {
+      screen(ci, snp0 + c, v, __ldg(us));
+      return;
+    }
+    const float f = __ldg(us + j + 1);
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
-      const float x = v[i] * us;
-      if (j == 0) {
-        num[i] = x;
-      } else if (j == 1) {
-        S[i] = x < 1e-12f ? -INFINITY : x;  // gg < 1e-12: p = 1
-      } else {
-        S[i] = fmaf(-x, x, S[i]);
-      }
+      const float x = v[i] * f;
+      float s;
+      if (j == 0) s = x < 1e-12f ? -INFINITY : x;  // gg < 1e-12: p = 1
+      else s = fmaf(-x, x, ci == 0 ? S0[i] : S1[i]);
+      if (ci == 0) S0[i] = s;
+      else S1[i] = s;
     }
   }
-  // after the last group: the 16 pairs' t, tail and per-gene updates
-  __device__ void finish_chunk(int c) {
-    const int64_t s0 = snp0 + c;
-    if (!gvalid || s0 >= Pr.m) return;
+  // NUM of the 16 pairs, the last accumulator: their t, tail and per-gene updates
+  __device__ __forceinline__ void screen(int ci, int64_t s0, const float (&v)[16], float us) {
+    if (s0 >= Pr.m) return;
     uint32_t okw[4];
     load_flags16(Pr.snp_ok + s0, okw);
-    float s_min = INFINITY;
+    float S[16], s_min = INFINITY;
+#pragma unroll
+    for (int j = 0; j < 16; ++j) S[j] = ci == 0 ? S0[j] : S1[j];
 #pragma unroll
     for (int j = 0; j < 16; j += 2) s_min = min3(s_min, S[j], S[j + 1]);
     screen_chunk(
         Pr.tt, tab, u_cand, Pr.win, Pr.out, gene, s0, all_flags16(okw) && s_min > 1e-15f,
         [&](int j) {
+          const float num = v[j] * us;
           if constexpr (GLM) {
-            const float U = fmaf(__ldg(Pr.snp_mean + s0 + j), rs, num[j]);
+            const float U = fmaf(__ldg(Pr.snp_mean + s0 + j), rs, num);
             return U * U * rcp_ftz(S[j]);  // z^2
           } else {
-            const float r = num[j] * (num[j] * rcp_ftz(S[j])) * inv_rss;
+            const float r = num * (num * rcp_ftz(S[j])) * inv_rss;
             return Pr.df * (r * rcp_ftz(1.0f - r));  // t^2
           }
         },
         [&](int j, bool& tested) {
           tested = flag16(okw, j);  // zero past the last kept SNP
+          const float num = v[j] * us;
           float t2;
           if constexpr (GLM) {
-            const float U = fmaf(__ldg(Pr.snp_mean + s0 + j), rs, num[j]);
+            const float U = fmaf(__ldg(Pr.snp_mean + s0 + j), rs, num);
             t2 = S[j] > 1e-15f ? __fdividef(U * U, S[j]) : 0.0f;
             if (!(t2 == t2)) t2 = 0.0f;
           } else {
-            const float r = num[j] * __fdividef(num[j], S[j]) * inv_rss;
+            const float r = num * __fdividef(num, S[j]) * inv_rss;
             const float omr = 1.0f - r;
             t2 = S[j] > 1e-15f && omr > 0.0f ? Pr.df * __fdividef(r, omr) : 0.0f;
           }
@@ -2824,6 +2840,29 @@ static void lmm_launch_lr(eqtl_ctx* ctx, const LmmLrEpiParams<P>& ep, const __ha
                             &tk);
 }
 
+// The grouped scan (p >= 3): ops = the gene-side hi operands [NUM, gg, a~_0 ..],
+// then their lo parts; bh / bl = [Gt, Gt^2]. Dense scans run on SM pairs.
+template <class EP>
+static void launch_grouped(eqtl_ctx* ctx, bool bf16, const EP& ep, const __half* const* ops, int nops, int G,
+                           const __half* const* bh, const __half* const* bl, int64_t m, int k_pad, const int2* tiles,
+                           int n_tiles) {
+  using E = typename EpiOf<EP>::type;
+  std::vector<const __half*> ah(static_cast<size_t>(nops)), al(static_cast<size_t>(nops));
+  std::vector<int> bsel(static_cast<size_t>(nops)), prod(static_cast<size_t>(nops), 7);
+  for (int j = 0; j < nops; ++j) {
+    const int op = j == nops - 1 ? 0 : j + 1;  // tile order [gg, a~_0 .., NUM]
+    ah[static_cast<size_t>(j)] = ops[op];
+    al[static_cast<size_t>(j)] = ops[nops + op];
+    bsel[static_cast<size_t>(j)] = op == 1 ? 1 : 0;  // gg reads the squares
+  }
+  if (!bf16 && !tiles && tile_pairs(G))
+    launch_tile_n<E::kTileN, E::kGroup, EP, dev::kBLoStage, 2>(ctx, false, ep, ah.data(), al.data(), G, bh, bl, m,
+                                                               k_pad, bsel.data(), prod.data(), nullptr, 0, 1, nops);
+  else
+    launch_tile_n<E::kTileN, E::kGroup>(ctx, bf16, ep, ah.data(), al.data(), G, bh, bl, m, k_pad, bsel.data(),
+                                        prod.data(), tiles, n_tiles, 1, nops);
+}
+
 // Subset gate of every kept SNP on the analysis samples into ws.ok.
 static void lmm_gate(eqtl_ctx* ctx) {
   Geno& g = ctx->geno;
@@ -2952,8 +2991,6 @@ static void scan_trans_lmm_impl(eqtl_ctx* ctx, const eqtl_scan_params* prm, cons
     ep.tt = tt;
     const __half* bh[2] = {Rt.gt_hi.p, Rt.gt2_hi.p};
     const __half* bl[2] = {Rt.gt_lo.p, Rt.gt2_lo.p};
-    std::vector<int> bsel(nops, 0), prod(nops, 7);
-    bsel[1] = 1;  // gg reads Gt^2
     const bool bf16 = ctx->precision == EQTL_PREC_SPLIT_BF16;
     std::vector<const __half*> opb(2 * static_cast<size_t>(nops));
     if (bf16) {
@@ -2968,8 +3005,7 @@ static void scan_trans_lmm_impl(eqtl_ctx* ctx, const eqtl_scan_params* prm, cons
     const __half* const* ops = bf16 ? opb.data() : oph.data();
     so.run([&](GeneOut out) {
       ep.out = out;
-      launch_tile_n<LmmGroupEpi::kTileN, 4>(ctx, bf16, ep, ops, ops + nops, G, bh, bl, Rt.m, Rt.k_pad, bsel.data(),
-                                            prod.data(), tiles, n_tiles, 1, nops);
+      launch_grouped(ctx, bf16, ep, ops, nops, G, bh, bl, Rt.m, Rt.k_pad, tiles, n_tiles);
     });
   } else if (m > 0) {
     const __half* ah[4] = {oph[0], oph[1], oph[2], nops > 3 ? oph[3] : oph[2]};
@@ -3577,12 +3613,9 @@ void scan_glm(eqtl_ctx* ctx, const eqtl_scan_params* prm, const double* Y, const
     ep.gene_ok = ws.glm_ok.p;
     const __half* bh[2] = {S.gt_hi.p, S.gt2_hi.p};
     const __half* bl[2] = {S.gt_lo.p, S.gt2_lo.p};
-    std::vector<int> bsel(nops, 0), prod(nops, 7);
-    bsel[1] = 1;  // gg reads gc^2
     so.run([&](GeneOut out) {
       ep.out = out;
-      launch_tile_n<GlmGroupEpi::kTileN, 4>(ctx, false, ep, oph.data(), oph.data() + nops, G, bh, bl, S.m, S.k_pad,
-                                            bsel.data(), prod.data(), tiles, n_tiles, 1, nops);
+      launch_grouped(ctx, false, ep, oph.data(), nops, G, bh, bl, S.m, S.k_pad, tiles, n_tiles);
     });
   } else if (m > 0) {
     const __half* ah[4] = {oph[0], oph[1], oph[2], nops > 3 ? oph[3] : oph[2]};

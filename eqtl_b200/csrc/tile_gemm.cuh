@@ -395,16 +395,18 @@ __global__ void __launch_bounds__(kTileThreads, 1)
         tc_fence_after();
         auto col = [&](int jj) { return lanes + static_cast<uint32_t>(((slot0 + jj) % C::NSLOTS) * NT); };
         if constexpr (Epi::kGrouped) {
+          constexpr int NCH = NT / (16 * kSub);
+          static_assert(NT % (16 * kSub) == 0 && NCH <= Epi::kMaxChunks, "grouped epilogue: chunks per warp");
 #pragma unroll 1
-          for (int c = 16 * sub; c < NT; c += 16 * kSub) {
+          for (int ci = 0; ci < NCH; ++ci) {
+            const int c = 16 * sub + 16 * kSub * ci;
 #pragma unroll 1
             for (int jj = 0; jj < nv; ++jj) {
               float v[16];
               tmem_ld16(col(jj) + static_cast<uint32_t>(c), v);
               tmem_wait_ld();
-              epi.acc_chunk(j0 + jj, c, v);
+              epi.acc_chunk(j0 + jj, ci, c, v);
             }
-            if (grp == sh.n_groups - 1) epi.finish_chunk(c);
           }
         } else if constexpr (IsTwoPhase<Epi>::value) {
           constexpr int N1 = Epi::kPhase1;
