@@ -150,103 +150,6 @@ void residualize_genes(eqtl_ctx* ctx, const double* dX, const double* dXtXinv, i
 
 
 
-void finish_scan(const eqtl_scan_params* prm, eqtl_gene_result* genes, const std::vector<eqtl_pair>& refined,
-                 std::vector<eqtl_pair>& pairs, std::vector<eqtl_pair>& cands) {
-  pairs.clear();
-  cands.clear();
-  const int G = prm->n_genes;
-  std::vector<const eqtl_pair*> best(G, nullptr);
-  for (const eqtl_pair& q : refined) {
-    if (q.p <= prm->pthr) pairs.push_back(q);
-    if (prm->perm_thr > 0 && std::isfinite(q.p) && q.p < prm->perm_thr) cands.push_back(q);
-    const eqtl_pair*& b = best[q.gene];
-    if (!b || q.p < b->p || (q.p == b->p && q.snp < b->snp)) b = &q;
-  }
-  for (int g = 0; g < G; ++g) {
-    eqtl_gene_result& r = genes[g];
-    if (r.n_tested > 0 && best[g]) {
-      r.best_snp = best[g]->snp;
-      r.best_p = best[g]->p;
-      r.best_beta = best[g]->beta;
-      r.best_se = best[g]->se;
-      r.best_t = best[g]->t;
-      r.best_r2 = best[g]->r2;
-    } else {
-      r.best_snp = -1;
-      r.best_p = 2.0;
-      r.best_beta = r.best_se = r.best_t = r.best_r2 = 0.0;
-    }
-  }
-  {
-    // (snp, gene) order through 64-bit keys: snp < 2^31, gene < 2^31
-    std::vector<uint64_t> key(pairs.size());
-    std::vector<uint32_t> idx(pairs.size());
-    for (size_t i = 0; i < pairs.size(); ++i) {
-      key[i] = (static_cast<uint64_t>(pairs[i].snp) << 32) | static_cast<uint32_t>(pairs[i].gene);
-      idx[i] = static_cast<uint32_t>(i);
-    }
-    radix_sort_u64(key, &idx);
-    std::vector<eqtl_pair> sorted(pairs.size());
-    for (size_t i = 0; i < idx.size(); ++i) sorted[i] = pairs[idx[i]];
-    pairs.swap(sorted);
-  }
-  std::sort(cands.begin(), cands.end(), [](const eqtl_pair& a, const eqtl_pair& b) {
-    if (a.gene != b.gene) return a.gene < b.gene;
-    if (a.p != b.p) return a.p < b.p;
-    return a.snp < b.snp;
-  });
-}
-
-void add_deferred_acat(eqtl_gene_result* genes, const std::vector<eqtl_pair>& refined,
-                       const std::vector<int2>& deferred) {
-  const long double kPiL = 3.14159265358979323846L;
-  // terms on every host thread, then added in pair order (the sums do not
-  // depend on the thread count)
-  std::vector<double> term(deferred.size());
-  std::vector<uint8_t> use(deferred.size());
-  std::vector<uint8_t> found(deferred.size());
-  parallel_for(deferred.size(), [&](size_t i) {
-    const int2 d = deferred[i];
-    auto it = std::lower_bound(refined.begin(), refined.end(), d, [](const eqtl_pair& q, const int2& k) {
-      return q.gene != k.x ? q.gene < k.x : q.snp < static_cast<int64_t>(k.y);
-    });
-    found[i] = it != refined.end() && it->gene == d.x && it->snp == d.y;
-    if (!found[i]) return;
-    double p = it->p;
-    use[i] = !(!std::isfinite(p) || p < 0.0 || p >= 1.0 - 1e-12);  // AcatAcc::add guards
-    if (!use[i]) return;
-    if (p <= 0.0) p = 1e-300;
-    term[i] = static_cast<double>(std::tan((0.5L - static_cast<long double>(p)) * kPiL));
-  });
-  for (size_t i = 0; i < deferred.size(); ++i) {
-    EQTL_CHECK(found[i], EQTL_E_INTERNAL, "deferred ACAT pair was not refined");
-    if (!use[i]) continue;
-    genes[deferred[i].x].acat_tan_sum += term[i];
-    ++genes[deferred[i].x].acat_used;
-  }
-}
-
-void add_acat_terms(eqtl_gene_result* genes, const std::vector<int2>& pairs, const std::vector<double>& p_pairs) {
-  const long double kPiL = 3.14159265358979323846L;
-  // terms on every host thread, then added in pair order (the sums do not
-  // depend on the thread count)
-  std::vector<double> term(pairs.size());
-  std::vector<uint8_t> use(pairs.size());
-  parallel_for(pairs.size(), [&](size_t i) {
-    double p = p_pairs[i];
-    use[i] = !(!std::isfinite(p) || p < 0.0 || p >= 1.0 - 1e-12);  // AcatAcc::add guards
-    if (!use[i]) return;
-    if (p <= 0.0) p = 1e-300;
-    term[i] = static_cast<double>(std::tan((0.5L - static_cast<long double>(p)) * kPiL));
-  });
-  for (size_t i = 0; i < pairs.size(); ++i) {
-    if (!use[i]) continue;
-    eqtl_gene_result& g = genes[pairs[i].x];
-    g.acat_tan_sum += term[i];
-    ++g.acat_used;
-  }
-}
-
 dev::Windows upload_windows(eqtl_ctx* ctx, const eqtl_scan_params* prm, int64_t m, int mode) {
   dev::Windows w{};
   w.mode = dev::kWinNone;
@@ -514,8 +417,8 @@ __global__ void fill_u64(unsigned long long* p, int n, unsigned long long v) {
 }
 }  // namespace
 
-ScanOutputs::ScanOutputs(eqtl_ctx* c, int genes, int64_t m, int64_t cap_hint)
-    : ctx(c), G(genes), acat(c->ws.acat), used(c->ws.used), tested(c->ws.tested), best(c->ws.best),
+ScanOutputs::ScanOutputs(eqtl_ctx* c, int genes, int64_t snps, int64_t cap_hint)
+    : ctx(c), G(genes), m(snps), acat(c->ws.acat), used(c->ws.used), tested(c->ws.tested), best(c->ws.best),
       cand(c->ws.cand), count(c->ws.count) {
   acat.alloc(G);
   used.alloc(G);
@@ -524,7 +427,6 @@ ScanOutputs::ScanOutputs(eqtl_ctx* c, int genes, int64_t m, int64_t cap_hint)
   count.alloc(1);
   cap = static_cast<unsigned int>(std::min<int64_t>(std::max<int64_t>(cap_hint, 1 << 16), 1 << 26));
   cand.alloc(cap);
-  (void)m;
 }
 
 void ScanOutputs::reset() {
@@ -541,7 +443,6 @@ void ScanOutputs::run(const std::function<void(dev::GeneOut)>& launch) {
     reset();
     dev::GeneOut o{acat.p, used.p, tested.p, best.p, cand.p, count.p, cap};
     launch(o);
-    EQTL_CUDA(cudaStreamSynchronize(ctx->stream));
     count.download(&n_cand, 1, ctx->stream);
     EQTL_CUDA(cudaStreamSynchronize(ctx->stream));
     if (n_cand <= cap) return;
@@ -551,49 +452,6 @@ void ScanOutputs::run(const std::function<void(dev::GeneOut)>& launch) {
     cand.alloc(cap);
   }
   throw Error(EQTL_E_INTERNAL, "candidate buffer did not converge");
-}
-
-void ScanOutputs::collect(eqtl_gene_result* genes, std::vector<int2>& todo, std::vector<int2>& deferred,
-                          std::vector<int2>* tiny) {
-  std::vector<double> a(G);
-  std::vector<int> u(G), t(G);
-  std::vector<unsigned long long> b(G);
-  acat.download(a.data(), G, ctx->stream);
-  used.download(u.data(), G, ctx->stream);
-  tested.download(t.data(), G, ctx->stream);
-  best.download(b.data(), G, ctx->stream);
-  std::vector<int2> c(n_cand);
-  cand.download(c.data(), n_cand, ctx->stream);
-  EQTL_CUDA(cudaStreamSynchronize(ctx->stream));
-  todo.clear();
-  deferred.clear();
-  if (tiny) tiny->clear();
-  for (const int2& q : c) {
-    const uint32_t s = static_cast<uint32_t>(q.y);
-    const int2 clean = make_int2(q.x, static_cast<int>(s & ~(dev::kCandDeferred | dev::kCandTiny)));
-    if (tiny && (s & dev::kCandTiny)) {
-      tiny->push_back(clean);
-      continue;
-    }
-    todo.push_back(clean);
-    if (s & dev::kCandDeferred) deferred.push_back(clean);
-  }
-  for (int g = 0; g < G; ++g) {
-    genes[g].n_tested = t[g];
-    genes[g].acat_used = u[g];
-    genes[g].acat_tan_sum = a[g];
-    genes[g].best_snp = -1;
-    if (t[g] > 0 && b[g] != ~0ull) todo.push_back(make_int2(g, static_cast<int>(b[g] & 0xFFFFFFFFull)));
-  }
-  // (gene, snp) order without duplicates, through 64-bit keys
-  std::vector<uint64_t> key(todo.size());
-  for (size_t i = 0; i < todo.size(); ++i)
-    key[i] = (static_cast<uint64_t>(static_cast<uint32_t>(todo[i].x)) << 32) | static_cast<uint32_t>(todo[i].y);
-  radix_sort_u64(key);
-  key.erase(std::unique(key.begin(), key.end()), key.end());
-  todo.resize(key.size());
-  for (size_t i = 0; i < key.size(); ++i)
-    todo[i] = make_int2(static_cast<int>(key[i] >> 32), static_cast<int>(key[i] & 0xFFFFFFFFull));
 }
 
 }  // namespace eqtl
@@ -929,17 +787,14 @@ int eqtl_scan_trans_lmm(eqtl_ctx* ctx, const eqtl_scan_params* prm, const double
                         int64_t* n_pairs, eqtl_pair* cands, int64_t cand_cap, int64_t* n_cands) {
   return guarded(ctx, [&] {
     EQTL_CHECK(prm && genes, EQTL_E_ARG, "null input");
-    std::vector<eqtl_pair> pv, cv;
+    eqtl::PairList pv{pairs, pair_cap, 0}, cv{cands, cand_cap, 0};
     if (ctx->precision == EQTL_PREC_FP32_SIMT)
       eqtl::scan_trans_lmm_simt(ctx, prm, Y, X, delta_out, genes, pv, cv);
     else
       eqtl::scan_trans_lmm(ctx, prm, Y, X, delta_out, genes, pv, cv);
-    if (n_pairs) *n_pairs = static_cast<int64_t>(pv.size());
-    if (n_cands) *n_cands = static_cast<int64_t>(cv.size());
-    EQTL_CHECK(static_cast<int64_t>(pv.size()) <= pair_cap && static_cast<int64_t>(cv.size()) <= cand_cap,
-               EQTL_E_OVERFLOW, "result buffer too small");
-    if (!pv.empty()) std::copy(pv.begin(), pv.end(), pairs);
-    if (!cv.empty()) std::copy(cv.begin(), cv.end(), cands);
+    if (n_pairs) *n_pairs = pv.n;
+    if (n_cands) *n_cands = cv.n;
+    EQTL_CHECK(pv.n <= pair_cap && cv.n <= cand_cap, EQTL_E_OVERFLOW, "result buffer too small");
   });
 }
 
@@ -948,14 +803,11 @@ int eqtl_scan_glm(eqtl_ctx* ctx, const eqtl_scan_params* prm, const double* Y, c
                   int64_t* n_pairs, eqtl_pair* cands, int64_t cand_cap, int64_t* n_cands) {
   return guarded(ctx, [&] {
     EQTL_CHECK(prm && genes, EQTL_E_ARG, "null input");
-    std::vector<eqtl_pair> pv, cv;
+    eqtl::PairList pv{pairs, pair_cap, 0}, cv{cands, cand_cap, 0};
     eqtl::scan_glm(ctx, prm, Y, X, phi_out, converged_out, genes, pv, cv);
-    if (n_pairs) *n_pairs = static_cast<int64_t>(pv.size());
-    if (n_cands) *n_cands = static_cast<int64_t>(cv.size());
-    EQTL_CHECK(static_cast<int64_t>(pv.size()) <= pair_cap && static_cast<int64_t>(cv.size()) <= cand_cap,
-               EQTL_E_OVERFLOW, "result buffer too small");
-    if (!pv.empty()) std::copy(pv.begin(), pv.end(), pairs);
-    if (!cv.empty()) std::copy(cv.begin(), cv.end(), cands);
+    if (n_pairs) *n_pairs = pv.n;
+    if (n_cands) *n_cands = cv.n;
+    EQTL_CHECK(pv.n <= pair_cap && cv.n <= cand_cap, EQTL_E_OVERFLOW, "result buffer too small");
   });
 }
 
@@ -975,14 +827,11 @@ int eqtl_scan_trans_lm(eqtl_ctx* ctx, const eqtl_scan_params* prm, const double*
     EQTL_CHECK(prm && genes, EQTL_E_ARG, "null input");
     EQTL_CHECK(ctx->precision != EQTL_PREC_FP32_SIMT, EQTL_E_UNSUPPORTED,
                "the FP32 CUDA-core comparator is available for the LMM scan only");
-    std::vector<eqtl_pair> pv, cv;
+    eqtl::PairList pv{pairs, pair_cap, 0}, cv{cands, cand_cap, 0};
     eqtl::scan_trans_lm(ctx, prm, Y, X, genes, pv, cv);
-    if (n_pairs) *n_pairs = static_cast<int64_t>(pv.size());
-    if (n_cands) *n_cands = static_cast<int64_t>(cv.size());
-    EQTL_CHECK(static_cast<int64_t>(pv.size()) <= pair_cap && static_cast<int64_t>(cv.size()) <= cand_cap,
-               EQTL_E_OVERFLOW, "result buffer too small");
-    if (!pv.empty()) std::copy(pv.begin(), pv.end(), pairs);
-    if (!cv.empty()) std::copy(cv.begin(), cv.end(), cands);
+    if (n_pairs) *n_pairs = pv.n;
+    if (n_cands) *n_cands = cv.n;
+    EQTL_CHECK(pv.n <= pair_cap && cv.n <= cand_cap, EQTL_E_OVERFLOW, "result buffer too small");
   });
 }
 

@@ -212,6 +212,14 @@ struct PeerWork {
 // Per-call workspaces reused across calls (capacity grows, never shrinks).
 struct Workspace {
   DevBuf<double> int_y;  // --pheno-norm int: the table
+  // a scan's results: sort keys and their histograms, compaction counts, lists
+  DevBuf<uint64_t> res_key[2], res_blk;
+  DevBuf<unsigned> res_hist, res_count;
+  DevBuf<int> res_deferred, res_cand, res_dg, ref_mark;
+  DevBuf<double> res_dp;
+  DevBuf<int2> tiny_pairs;
+  DevBuf<eqtl_gene_result> res_genes;
+  DevBuf<eqtl_pair> res_pairs;
   PeerWork peer;
   DevBuf<double> Ytil, Xtil, Ys, XtY, XtXinv, delta, chi0, ainv, a00L, rss, gtg, inv_gtg, af_sub, inv_yty, yty;
   DevBuf<__half> ops_hi[34], ops_lo[34];  // gene-side operands, one per accumulator (dev::kMaxAcc)
@@ -327,7 +335,6 @@ struct eqtl_ctx {
   eqtl::Workspace ws;
   bool have_basis = false;
   int precision = EQTL_PREC_SPLIT_F16;
-  std::vector<int> host_mark;  // per-kept-SNP scratch of the refinement's index
 };
 
 namespace eqtl {
@@ -361,14 +368,18 @@ void pheno_permute(eqtl_ctx* ctx, const double* base, const double* xb0, const d
                    double* Y_out);
 
 // -- scan drivers
+// A caller's list of pairs: n of them were found; they are there if n <= cap.
+struct PairList {
+  eqtl_pair* p;
+  int64_t cap, n;
+};
 void scan_trans_lm(eqtl_ctx* ctx, const eqtl_scan_params* prm, const double* Y, const double* X,
-                   eqtl_gene_result* genes, std::vector<eqtl_pair>& pairs, std::vector<eqtl_pair>& cands);
+                   eqtl_gene_result* genes, PairList& pairs, PairList& cands);
 
 void scan_trans_lmm(eqtl_ctx* ctx, const eqtl_scan_params* prm, const double* Y, const double* X, double* delta_out,
-                    eqtl_gene_result* genes, std::vector<eqtl_pair>& pairs, std::vector<eqtl_pair>& cands);
+                    eqtl_gene_result* genes, PairList& pairs, PairList& cands);
 void scan_trans_lmm_simt(eqtl_ctx* ctx, const eqtl_scan_params* prm, const double* Y, const double* X,
-                         double* delta_out, eqtl_gene_result* genes, std::vector<eqtl_pair>& pairs,
-                         std::vector<eqtl_pair>& cands);
+                         double* delta_out, eqtl_gene_result* genes, PairList& pairs, PairList& cands);
 
 // -- grm.cu / lmm.cu
 template <class T>
@@ -394,8 +405,7 @@ void test_pairs_lm(eqtl_ctx* ctx, const eqtl_scan_params* prm, const double* Y, 
 // NB-GLM score-test scan (model_glm.cpp) of every (gene, kept SNP) pair in
 // scope; phi_out / converged_out per gene.
 void scan_glm(eqtl_ctx* ctx, const eqtl_scan_params* prm, const double* Y, const double* X, double* phi_out,
-              uint8_t* converged_out, eqtl_gene_result* genes, std::vector<eqtl_pair>& pairs,
-              std::vector<eqtl_pair>& cands);
+              uint8_t* converged_out, eqtl_gene_result* genes, PairList& pairs, PairList& cands);
 void test_pairs_lmm(eqtl_ctx* ctx, const eqtl_scan_params* prm, const double* Y, const double* X,
                     const std::vector<int2>& todo, eqtl_pair* out, double* delta_out);
 

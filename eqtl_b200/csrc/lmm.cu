@@ -2526,72 +2526,47 @@ static void exact_qg(eqtl_ctx* ctx, const std::vector<int>& snps, double* out) {
   }
 }
 
-// FP64 statistics of (gene, kept SNP) pairs against the current LMM prep
-// (ws.Ytil, Xtil, delta, chi0, ainv, rss): Gt = Q'g of the SNPs involved (exactly
-// on the tensor cores for many 2-bit rows, else by DGEMM: FP32 dosages, more than
-// kQgMaxN samples, little work), then one warp per pair (lmm_refine_kernel).
-static std::vector<eqtl_pair> lmm_refine_pairs(eqtl_ctx* ctx, int p, double df, const std::vector<int2>& todo) {
+// FP64 statistics of the first n_pairs of ws.ref_pairs into ws.refined, against the
+// current LMM prep (ws.Ytil, Xtil, delta, chi0, ainv, rss): Gt = Q'g of the SNPs
+// involved (exactly on the tensor cores for many 2-bit rows, else by DGEMM: FP32
+// dosages, more than kQgMaxN samples, little work), then one warp per pair
+// (lmm_refine_kernel).
+static void lmm_refine_pairs(eqtl_ctx* ctx, int p, double df, int n_pairs) {
   Geno& g = ctx->geno;
   Workspace& ws = ctx->ws;
   cudaStream_t st = ctx->stream;
   const int n = g.n;
-  std::vector<eqtl_pair> refined(todo.size());
-  HostTrace tr("lmm_refine_pairs");
-  if (!todo.empty()) {
-    // distinct SNPs in index order and each pair's column among them, by a
-    // marker over the kept SNPs (O(m + pairs), no sort)
-    std::vector<int>& mark = ctx->host_mark;
-    mark.assign(static_cast<size_t>(g.m), -1);
-    for (const int2& q : todo) mark[q.y] = 0;
-    std::vector<int> snps;
-    for (int64_t s = 0; s < g.m; ++s)
-      if (mark[s] == 0) {
-        mark[s] = static_cast<int>(snps.size());
-        snps.push_back(static_cast<int>(s));
-      }
-    std::vector<int> pcol(todo.size());
-    for (size_t i = 0; i < todo.size(); ++i) pcol[i] = mark[todo[i].y];
-    const int u = static_cast<int>(snps.size());
-    DevBuf<int>& dsn = ws.ref_snps;
-    DevBuf<int>& dpc = ws.ref_col;
-    DevBuf<int2>& dtodo = ws.ref_pairs;
-    dsn.upload(snps.data(), u, st);
-    dpc.upload(pcol.data(), pcol.size(), st);
-    dtodo.upload(todo.data(), todo.size(), st);
-    tr.mark("host index + upload");
-    DevBuf<double>& gt = ws.gt;
-    gt.alloc(static_cast<size_t>(n) * u);
-    if (!g.dense && n <= kQgMaxN && static_cast<int64_t>(n) * n * u >= kQgMinWork) {
-      exact_qg(ctx, snps, gt.p);
-    } else {
-      DevBuf<double>& graw = ws.graw;
-      graw.alloc(static_cast<size_t>(n) * u);
-      ++ctx->launches;
-      raw_dosage_kernel<<<1184, 256, 0, st>>>(g.rows(), g.col.p, n, g.kept.p, g.mu.p, dsn.p, u, graw.p);
-      EQTL_CUDA(cudaGetLastError());
-      const double one = 1.0, zero = 0.0;
-      EQTL_CHECK(cublasDgemm(blas_of(ctx), CUBLAS_OP_T, CUBLAS_OP_N, n, u, n, &one, ctx->basis.Q.p, n, graw.p, n,
-                             &zero, gt.p, n) == CUBLAS_STATUS_SUCCESS,
-                 EQTL_E_CUDA, "Q'g failed");
-    }
+  if (n_pairs == 0) return;
+  const std::vector<int> snps = distinct_snps(ctx, n_pairs, g.m);
+  const int u = static_cast<int>(snps.size());
+  DevBuf<double>& gt = ws.gt;
+  gt.alloc(static_cast<size_t>(n) * u);
+  if (!g.dense && n <= kQgMaxN && static_cast<int64_t>(n) * n * u >= kQgMinWork) {
+    exact_qg(ctx, snps, gt.p);
+  } else {
+    DevBuf<double>& graw = ws.graw;
+    graw.alloc(static_cast<size_t>(n) * u);
     ++ctx->launches;
-    ws.refined.alloc(todo.size());
-    lmm_refine_kernel<<<static_cast<unsigned>((todo.size() + 7) / 8), 256, 0, st>>>(
-        gt.p, n, dpc.p, dtodo.p, static_cast<int>(todo.size()), ws.Ytil.p, ws.Xtil.p, p, ctx->basis.lambda.p,
-        ws.delta.p, ws.chi0.p, ws.a00L.p, ws.rss.p, df, ws.refined.p);
+    raw_dosage_kernel<<<1184, 256, 0, st>>>(g.rows(), g.col.p, n, g.kept.p, g.mu.p, ws.ref_snps.p, u, graw.p);
     EQTL_CUDA(cudaGetLastError());
-    tr.mark("launches");
-    ws.refined.download(refined.data(), todo.size(), st);
-    EQTL_CUDA(cudaStreamSynchronize(st));
-    tr.mark("device work + download");
+    const double one = 1.0, zero = 0.0;
+    EQTL_CHECK(cublasDgemm(blas_of(ctx), CUBLAS_OP_T, CUBLAS_OP_N, n, u, n, &one, ctx->basis.Q.p, n, graw.p, n,
+                           &zero, gt.p, n) == CUBLAS_STATUS_SUCCESS,
+               EQTL_E_CUDA, "Q'g failed");
   }
-  return refined;
+  ++ctx->launches;
+  ws.refined.alloc(static_cast<size_t>(n_pairs));
+  lmm_refine_kernel<<<static_cast<unsigned>((n_pairs + 7) / 8), 256, 0, st>>>(
+      gt.p, n, ws.ref_col.p, ws.ref_pairs.p, n_pairs, ws.Ytil.p, ws.Xtil.p, p, ctx->basis.lambda.p, ws.delta.p,
+      ws.chi0.p, ws.a00L.p, ws.rss.p, df, ws.refined.p);
+  EQTL_CUDA(cudaGetLastError());
 }
 
-// FP64 p of tiny-|t| pairs against the current LMM prep (see lmm_tiny_kernel).
+// FP64 p of the n_tiny pairs of ws.tiny_pairs against the current LMM prep (see
+// lmm_tiny_kernel).
 // U_pre (optional): u = Q (w o r~) of gene g at U_pre + g * u_stride, as the
 // exact-operand scan has it already; otherwise it is computed here.
-static std::vector<double> lmm_tiny_p(eqtl_ctx* ctx, int p, double df, const std::vector<int2>& tiny,
+static std::vector<double> lmm_tiny_p(eqtl_ctx* ctx, int p, double df, int n_tiny,
                                       const double* U_pre = nullptr, int64_t u_stride = 0) {
   Geno& g = ctx->geno;
   Workspace& ws = ctx->ws;
@@ -2599,8 +2574,8 @@ static std::vector<double> lmm_tiny_p(eqtl_ctx* ctx, int p, double df, const std
   cudaStream_t st = ctx->stream;
   const int n = g.n;
   const int G = static_cast<int>(ws.delta.n);
-  std::vector<double> out(tiny.size());
-  if (tiny.empty()) return out;
+  std::vector<double> out(static_cast<size_t>(n_tiny));
+  if (n_tiny == 0) return out;
   const double* U = U_pre;
   if (!U) {
     ws.graw.alloc(static_cast<size_t>(n) * G);  // w o r~ per gene
@@ -2619,12 +2594,11 @@ static std::vector<double> lmm_tiny_p(eqtl_ctx* ctx, int p, double df, const std
   ctx->launches += 1;
   float s1, s2;
   output_scales(n, s1, s2);
-  ws.ref_pairs.upload(tiny.data(), tiny.size(), st);
-  ws.tiny_p.alloc(tiny.size());
-  lmm_tiny_kernel<<<static_cast<unsigned>((tiny.size() + 7) / 8), 256, 0, st>>>(
+  ws.tiny_p.alloc(static_cast<size_t>(n_tiny));
+  lmm_tiny_kernel<<<static_cast<unsigned>((n_tiny + 7) / 8), 256, 0, st>>>(
       g.rows(), g.col.p, n, R.k_pad, g.kept.p, g.mu.p, U, u_stride, R.gt_hi.p, R.gt_lo.p, 1.0 / s1,
-      ws.Xtil.p, p, ctx->basis.lambda.p, ws.delta.p, ws.ainv.p, ws.rss.p, df, ws.ref_pairs.p,
-      static_cast<int>(tiny.size()), ws.tiny_p.p);
+      ws.Xtil.p, p, ctx->basis.lambda.p, ws.delta.p, ws.ainv.p, ws.rss.p, df, ws.tiny_pairs.p, n_tiny,
+      ws.tiny_p.p);
   EQTL_CUDA(cudaGetLastError());
   ws.tiny_p.download(out.data(), out.size(), st);
   EQTL_CUDA(cudaStreamSynchronize(st));
@@ -2879,8 +2853,7 @@ static void lmm_gate(eqtl_ctx* ctx) {
 }
 
 static void scan_trans_lmm_impl(eqtl_ctx* ctx, const eqtl_scan_params* prm, const double* Y, const double* X,
-                                double* delta_out, eqtl_gene_result* genes, std::vector<eqtl_pair>& pairs,
-                                std::vector<eqtl_pair>& cands, bool simt) {
+                                double* delta_out, eqtl_gene_result* genes, PairList& pairs, PairList& cands, bool simt) {
   Geno& g = ctx->geno;
   Workspace& ws = ctx->ws;
   const int n = prm->n, G = prm->n_genes, p = prm->p;
@@ -3044,8 +3017,7 @@ static void scan_trans_lmm_impl(eqtl_ctx* ctx, const eqtl_scan_params* prm, cons
   }
   scan_timer.reset();
   HostTrace tr("scan_trans_lmm");
-  std::vector<int2> todo, deferred, tiny;
-  so.collect(genes, todo, deferred, &tiny);
+  so.collect(true);
   tr.mark("collect (waits for the scan)");
 
   // ---- FP64 refinement: rotate raw dosages of the SNPs involved
@@ -3054,30 +3026,29 @@ static void scan_trans_lmm_impl(eqtl_ctx* ctx, const eqtl_scan_params* prm, cons
     ws.delta.download(delta_out, G, st);
     EQTL_CUDA(cudaStreamSynchronize(st));
   }
-  std::vector<eqtl_pair> refined = lmm_refine_pairs(ctx, p, df, todo);
+  lmm_refine_pairs(ctx, p, df, so.n_todo);
   tr.mark("refine pairs");
-  add_deferred_acat(genes, refined, deferred);
-  tr.mark("deferred ACAT");
-  const std::vector<double> tiny_p =
-      raw ? lmm_tiny_p(ctx, p, df, tiny, ws.lmm_uv.p, static_cast<int64_t>(p + 1) * n) : lmm_tiny_p(ctx, p, df, tiny);
+  const std::vector<double> tiny_p = raw ? lmm_tiny_p(ctx, p, df, so.n_tiny, ws.lmm_uv.p, static_cast<int64_t>(p + 1) * n)
+                                         : lmm_tiny_p(ctx, p, df, so.n_tiny);
+  std::vector<int2> tiny(static_cast<size_t>(so.n_tiny));
+  ws.tiny_pairs.download(tiny.data(), tiny.size(), st);
   tr.mark("tiny-|t| pairs");
+  so.finish(prm, genes, pairs, cands);
+  tr.mark("finish");
   add_acat_terms(genes, tiny, tiny_p);
   tr.mark("tiny ACAT terms");
-  finish_scan(prm, genes, refined, pairs, cands);
-  tr.mark("finish");
   if (tr.on)
-    std::fprintf(stderr, "[eqtl trace] scan_trans_lmm counts: candidates %zu deferred %zu tiny %zu\n", todo.size(),
-                 deferred.size(), tiny.size());
+    std::fprintf(stderr, "[eqtl trace] scan_trans_lmm counts: candidates %d deferred %d tiny %d\n", so.n_todo,
+                 so.n_deferred, so.n_tiny);
 }
 
 void scan_trans_lmm(eqtl_ctx* ctx, const eqtl_scan_params* prm, const double* Y, const double* X, double* delta_out,
-                    eqtl_gene_result* genes, std::vector<eqtl_pair>& pairs, std::vector<eqtl_pair>& cands) {
+                    eqtl_gene_result* genes, PairList& pairs, PairList& cands) {
   scan_trans_lmm_impl(ctx, prm, Y, X, delta_out, genes, pairs, cands, false);
 }
 
 void scan_trans_lmm_simt(eqtl_ctx* ctx, const eqtl_scan_params* prm, const double* Y, const double* X,
-                         double* delta_out, eqtl_gene_result* genes, std::vector<eqtl_pair>& pairs,
-                         std::vector<eqtl_pair>& cands) {
+                         double* delta_out, eqtl_gene_result* genes, PairList& pairs, PairList& cands) {
   scan_trans_lmm_impl(ctx, prm, Y, X, delta_out, genes, pairs, cands, true);
 }
 
@@ -3101,11 +3072,12 @@ void test_pairs_lmm(eqtl_ctx* ctx, const eqtl_scan_params* prm, const double* Y,
   lmm_gate(ctx);
   std::vector<uint8_t> ok(static_cast<size_t>(g.m));
   ws.ok.download(ok.data(), static_cast<size_t>(g.m), ctx->stream);
-  const std::vector<eqtl_pair> refined = lmm_refine_pairs(ctx, p, df, todo);
-  for (size_t i = 0; i < todo.size(); ++i) {
-    out[i] = refined[i];
+  ws.ref_pairs.upload(todo.data(), todo.size(), ctx->stream);
+  lmm_refine_pairs(ctx, p, df, static_cast<int>(todo.size()));
+  ws.refined.download(out, todo.size(), ctx->stream);
+  EQTL_CUDA(cudaStreamSynchronize(ctx->stream));
+  for (size_t i = 0; i < todo.size(); ++i)
     if (!ok[todo[i].y]) out[i].p = std::numeric_limits<double>::quiet_NaN();
-  }
   if (delta_out) {
     ws.delta.download(delta_out, G, ctx->stream);
     EQTL_CUDA(cudaStreamSynchronize(ctx->stream));
@@ -3419,7 +3391,8 @@ __global__ void glm_refine_kernel(GenoRows src, const int32_t* __restrict__ col,
                                   const int64_t* __restrict__ kept, const double* __restrict__ mu_imp,
                                   const double* __restrict__ W, const double* __restrict__ Rr,
                                   const double* __restrict__ X, int p, const double* __restrict__ ainv,
-                                  const int2* __restrict__ pairs, int n_pairs, eqtl_pair* out) {
+                                  const uint8_t* __restrict__ gene_ok, const int2* __restrict__ pairs, int n_pairs,
+                                  eqtl_pair* out) {
   const int lane = threadIdx.x & 31;
   const int wid = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (wid >= n_pairs) return;
@@ -3467,39 +3440,28 @@ __global__ void glm_refine_kernel(GenoRows src, const int32_t* __restrict__ col,
   q.gene = g;
   q.reserved = 0;
   glm_stats_fp64(U, gwg, xAx, sd2 / n - mean * mean, q);
+  // a gene whose null fit failed tests nothing (p = NaN, test_glm_nb)
+  if (!gene_ok[g]) q.p = CUDART_NAN;
   out[wid] = q;
 }
 
 }  // namespace dev
 
-static std::vector<eqtl_pair> glm_refine_pairs(eqtl_ctx* ctx, int p, const std::vector<int2>& todo) {
+// FP64 statistics of the first n_pairs of ws.ref_pairs into ws.refined.
+static void glm_refine_pairs(eqtl_ctx* ctx, int p, int n_pairs) {
   Geno& g = ctx->geno;
   Workspace& ws = ctx->ws;
-  cudaStream_t st = ctx->stream;
-  std::vector<eqtl_pair> refined(todo.size());
-  if (todo.empty()) return refined;
-  ws.ref_pairs.upload(todo.data(), todo.size(), st);
-  ws.refined.alloc(todo.size());
-  const int n_pairs = static_cast<int>(todo.size());
+  if (n_pairs == 0) return;
+  ws.refined.alloc(static_cast<size_t>(n_pairs));
   ++ctx->launches;
-  glm_refine_kernel<<<static_cast<unsigned>((n_pairs + 7) / 8), 256, 0, st>>>(
-      g.rows(), g.col.p, g.n, g.kept.p, g.mu.p, ws.glm_w.p, ws.glm_r.p, ctx->pheno.X.p, p, ws.ainv.p,
+  glm_refine_kernel<<<static_cast<unsigned>((n_pairs + 7) / 8), 256, 0, ctx->stream>>>(
+      g.rows(), g.col.p, g.n, g.kept.p, g.mu.p, ws.glm_w.p, ws.glm_r.p, ctx->pheno.X.p, p, ws.ainv.p, ws.glm_ok.p,
       ws.ref_pairs.p, n_pairs, ws.refined.p);
   EQTL_CUDA(cudaGetLastError());
-  ws.refined.download(refined.data(), refined.size(), st);
-  EQTL_CUDA(cudaStreamSynchronize(st));
-  // a gene whose null fit failed tests nothing (p = NaN, test_glm_nb)
-  std::vector<uint8_t> ok(ctx->pheno.G);
-  ws.glm_ok.download(ok.data(), ok.size(), st);
-  EQTL_CUDA(cudaStreamSynchronize(st));
-  for (eqtl_pair& q : refined)
-    if (!ok[q.gene]) q.p = std::numeric_limits<double>::quiet_NaN();
-  return refined;
 }
 
 void scan_glm(eqtl_ctx* ctx, const eqtl_scan_params* prm, const double* Y, const double* X, double* phi_out,
-              uint8_t* converged_out, eqtl_gene_result* genes, std::vector<eqtl_pair>& pairs,
-              std::vector<eqtl_pair>& cands) {
+              uint8_t* converged_out, eqtl_gene_result* genes, PairList& pairs, PairList& cands) {
   Geno& g = ctx->geno;
   Workspace& ws = ctx->ws;
   const int n = prm->n, G = prm->n_genes, p = prm->p;
@@ -3651,13 +3613,11 @@ void scan_glm(eqtl_ctx* ctx, const eqtl_scan_params* prm, const double* Y, const
     }
   }
   scan_timer.reset();
-  std::vector<int2> todo, deferred;
-  so.collect(genes, todo, deferred);
+  so.collect();
   // ---- FP64 refinement of the candidates, deferred and tiny-|z| pairs
   StageScope refine_timer(ctx, EQTL_STAGE_REFINE);
-  const std::vector<eqtl_pair> refined = glm_refine_pairs(ctx, p, todo);
-  add_deferred_acat(genes, refined, deferred);
-  finish_scan(prm, genes, refined, pairs, cands);
+  glm_refine_pairs(ctx, p, so.n_todo);
+  so.finish(prm, genes, pairs, cands);
 }
 
 }  // namespace eqtl

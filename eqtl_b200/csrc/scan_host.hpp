@@ -21,12 +21,6 @@ std::vector<double> xtx_inverse(const double* X, int n, int p);  // (X'X)^-1, ro
 void residualize_genes(eqtl_ctx* ctx, const double* dX, const double* dXtXinv, int n, int p, int G, double* dY,
                        double* dXtY);
 
-// Splits refined pairs into the pair list (p <= pthr, sorted by snp then
-// gene) and stage-2 candidates (p < perm_thr, sorted by gene, p, snp), and
-// sets each gene's best from the refined pairs (smallest p, lowest snp).
-void finish_scan(const eqtl_scan_params* prm, eqtl_gene_result* genes, const std::vector<eqtl_pair>& refined,
-                 std::vector<eqtl_pair>& pairs, std::vector<eqtl_pair>& cands);
-
 // Uploads the scan windows into the context workspace; returns the device
 // view (mode none when the caller gave no windows).
 dev::Windows upload_windows(eqtl_ctx* ctx, const eqtl_scan_params* prm, int64_t m, int mode);
@@ -54,6 +48,7 @@ const PhenoDev& resolve_pheno(eqtl_ctx* ctx, const eqtl_scan_params* prm, const 
 struct ScanOutputs {
   eqtl_ctx* ctx;
   int G;
+  int64_t m;
   DevBuf<double>& acat;
   DevBuf<int>& used;
   DevBuf<int>& tested;
@@ -66,21 +61,23 @@ struct ScanOutputs {
   void reset();
   // runs `launch` until every candidate fitted in the buffer
   void run(const std::function<void(dev::GeneOut)>& launch);
-  // downloads per-gene sums into genes[] and returns the (gene, snp) pairs to
-  // refine: all candidates plus each gene's best SNP
-  // refine: all candidates plus each gene's best SNP; with `tiny`, the pairs
-  // deferred only for 0 < |t| < tiny_t go there instead of todo / deferred
-  void collect(eqtl_gene_result* genes, std::vector<int2>& todo, std::vector<int2>& deferred,
-               std::vector<int2>* tiny = nullptr);
+  // The pairs to refine, from the candidate buffer and each gene's best SNP:
+  // n_todo distinct ones in (gene, snp) order in ws.ref_pairs, the places of the
+  // n_deferred among them whose ACAT term is missing in ws.res_deferred; with
+  // split_tiny, the n_tiny pairs deferred only for 0 < |t| < tiny_t go to
+  // ws.tiny_pairs instead.
+  void collect(bool split_tiny = false);
+  // From ws.refined (the statistics of ws.ref_pairs): genes[] with each gene's
+  // best (smallest p, lowest snp) and the deferred ACAT terms added, the pairs
+  // with p <= pthr sorted by snp then gene, and the stage-2 candidates (p <
+  // perm_thr) sorted by gene, p, snp.
+  void finish(const eqtl_scan_params* prm, eqtl_gene_result* genes, PairList& pairs, PairList& cands);
+  int n_todo = 0, n_deferred = 0, n_tiny = 0;
 };
 
-// Adds, for every deferred (gene, snp) pair, the reference's long-double ACAT
-// term tan((0.5L - p) pi_L) computed from the refined FP64 p
-// (src/stats_extra.cpp:16-22; p <= 0 -> 1e-300).
-// `refined` is sorted by (gene, snp), as ScanOutputs::collect orders the
-// pairs it hands to the refinement.
-void add_deferred_acat(eqtl_gene_result* genes, const std::vector<eqtl_pair>& refined,
-                       const std::vector<int2>& deferred);
+// The distinct SNPs of ws.ref_pairs[0 .. n_pairs) (n_pairs > 0, SNPs below m) in
+// order, also on the device in ws.ref_snps; ws.ref_col: each pair's place among them.
+std::vector<int> distinct_snps(eqtl_ctx* ctx, int n_pairs, int64_t m);
 
 // Adds the reference's long-double ACAT term and `used` count of each pair
 // whose FP64 p (p_pairs[i]) enters ACAT (src/stats_extra.cpp:16-22).

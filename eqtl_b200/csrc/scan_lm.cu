@@ -368,30 +368,23 @@ static void snp_gtg(eqtl_ctx* ctx, const PhenoDev& ph, int p) {
   else snp_gtg_launch<kMaxP>(ctx, ph, p);
 }
 
-// FP64 statistics of (gene, kept SNP) pairs against the current LM prep
-// (ws.Ys, ws.yty, ws.gtg): gty from the exact decoded dosage, one warp per pair.
-static std::vector<eqtl_pair> lm_refine_pairs(eqtl_ctx* ctx, double df, const std::vector<int2>& todo) {
+// FP64 statistics of the first n_pairs of ws.ref_pairs into ws.refined, against
+// the current LM prep (ws.Ys, ws.yty, ws.gtg): gty from the exact decoded dosage,
+// one warp per pair.
+static void lm_refine_pairs(eqtl_ctx* ctx, double df, int n_pairs) {
   Geno& g = ctx->geno;
   Workspace& ws = ctx->ws;
-  cudaStream_t st = ctx->stream;
-  const int n = g.n;
-  std::vector<eqtl_pair> refined(todo.size());
-  if (!todo.empty()) {
-    ws.ref_pairs.upload(todo.data(), todo.size(), st);
-    ws.refined.alloc(todo.size());
-    ++ctx->launches;
-    lm_refine_kernel<<<static_cast<unsigned>((todo.size() + 7) / 8), 256, 0, st>>>(
-        g.rows(), g.col.p, n, g.kept.p, g.mu.p, ws.Ys.p, ws.gtg.p, ws.yty.p, df, ws.ref_pairs.p,
-        static_cast<int>(todo.size()), ws.refined.p);
-    EQTL_CUDA(cudaGetLastError());
-    ws.refined.download(refined.data(), todo.size(), st);
-    EQTL_CUDA(cudaStreamSynchronize(st));
-  }
-  return refined;
+  if (n_pairs == 0) return;
+  ws.refined.alloc(static_cast<size_t>(n_pairs));
+  ++ctx->launches;
+  lm_refine_kernel<<<static_cast<unsigned>((n_pairs + 7) / 8), 256, 0, ctx->stream>>>(
+      g.rows(), g.col.p, g.n, g.kept.p, g.mu.p, ws.Ys.p, ws.gtg.p, ws.yty.p, df, ws.ref_pairs.p, n_pairs,
+      ws.refined.p);
+  EQTL_CUDA(cudaGetLastError());
 }
 
 void scan_trans_lm(eqtl_ctx* ctx, const eqtl_scan_params* prm, const double* Y, const double* X,
-                   eqtl_gene_result* genes, std::vector<eqtl_pair>& pairs, std::vector<eqtl_pair>& cands) {
+                   eqtl_gene_result* genes, PairList& pairs, PairList& cands) {
   Geno& g = ctx->geno;
   Workspace& ws = ctx->ws;
   EQTL_CHECK(g.m_all > 0, EQTL_E_STATE, "scan_trans_lm: no genotypes loaded");
@@ -506,18 +499,13 @@ void scan_trans_lm(eqtl_ctx* ctx, const eqtl_scan_params* prm, const double* Y, 
   // ---- refine candidates + per-gene best in FP64
   StageScope refine_timer(ctx, EQTL_STAGE_REFINE);
   HostTrace tr("scan_trans_lm");
-  std::vector<int2> todo, deferred;
-  so.collect(genes, todo, deferred);
+  so.collect();
   tr.mark("collect");
-  std::vector<eqtl_pair> refined = lm_refine_pairs(ctx, df, todo);
-  tr.mark("refine pairs (device + download)");
-  add_deferred_acat(genes, refined, deferred);
-  tr.mark("deferred ACAT terms");
-  finish_scan(prm, genes, refined, pairs, cands);
-  tr.mark("finish");
+  lm_refine_pairs(ctx, df, so.n_todo);
+  so.finish(prm, genes, pairs, cands);
+  tr.mark("refine and finish");
   if (tr.on)
-    std::fprintf(stderr, "[eqtl trace] scan_trans_lm counts: refined %zu deferred %zu\n", todo.size(),
-                 deferred.size());
+    std::fprintf(stderr, "[eqtl trace] scan_trans_lm counts: refined %d deferred %d\n", so.n_todo, so.n_deferred);
 }
 
 // FP64 tests of explicit (column of Y, kept SNP) pairs with the scan's prep:
@@ -561,11 +549,12 @@ void test_pairs_lm(eqtl_ctx* ctx, const eqtl_scan_params* prm, const double* Y, 
   if (m > 0) snp_gtg(ctx, ph, p);
   std::vector<uint8_t> ok(static_cast<size_t>(m));
   ws.ok.download(ok.data(), static_cast<size_t>(m), st);
-  const std::vector<eqtl_pair> refined = lm_refine_pairs(ctx, df, todo);
-  for (size_t i = 0; i < todo.size(); ++i) {
-    out[i] = refined[i];
+  ws.ref_pairs.upload(todo.data(), todo.size(), st);
+  lm_refine_pairs(ctx, df, static_cast<int>(todo.size()));
+  ws.refined.download(out, todo.size(), st);
+  EQTL_CUDA(cudaStreamSynchronize(st));
+  for (size_t i = 0; i < todo.size(); ++i)
     if (!ok[todo[i].y]) out[i].p = std::numeric_limits<double>::quiet_NaN();
-  }
 }
 
 }  // namespace eqtl
