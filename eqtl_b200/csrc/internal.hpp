@@ -222,6 +222,7 @@ struct Workspace {
   DevBuf<eqtl_pair> res_pairs;
   PeerWork peer;
   DevBuf<double> Ytil, Xtil, Ys, XtY, XtXinv, delta, chi0, ainv, a00L, rss, gtg, inv_gtg, af_sub, inv_yty, yty;
+  DevBuf<double> reml_w, reml_tot;  // weights and totals of the REML grid
   DevBuf<__half> ops_hi[34], ops_lo[34];  // gene-side operands, one per accumulator (dev::kMaxAcc)
   DevBuf<__half> opsb_hi[34], opsb_lo[34];  // the same re-split into BF16 hi + lo (split-BF16 LMM scans)
   DevBuf<__half*> ops_ptr;

@@ -146,56 +146,6 @@ __device__ bool chol_solve(const double* A, const double* b, double* x, double* 
   return true;
 }
 
-// optimize_delta (src/model_lmm.cpp:39-86): grid 1e-5..1e5 x2 (and 1.0), 40
-// golden-section steps on [best/4, best*4] clipped to [1e-8, 1e6], then up to
-// 8 Newton steps on central differences. f(d) returns -loglik and is called
-// by every thread of the unit (warp or block) that evaluates it.
-template <class F>
-__device__ double optimize_delta_dev(F&& f, int df) {
-  double d = 1.0;
-  if (df <= 0) return d;
-  double best_d = 1.0;
-  double best_ll = f(1.0);
-  for (double dd = 1e-5; dd <= 1e5; dd *= 2.0) {
-    const double v = f(dd);
-    if (v < best_ll) {
-      best_ll = v;
-      best_d = dd;
-    }
-  }
-  double lo = best_d / 4.0, hi = best_d * 4.0;
-  if (lo < 1e-8) lo = 1e-8;
-  if (hi > 1e6) hi = 1e6;
-  const double phi = (1.0 + sqrt(5.0)) / 2.0;
-  for (int it = 0; it < 40; ++it) {
-    const double m1 = hi - (hi - lo) / phi;
-    const double m2 = lo + (hi - lo) / phi;
-    const double f1 = f(m1);
-    const double f2 = f(m2);
-    if (f1 < f2) hi = m2;
-    else lo = m1;
-  }
-  d = 0.5 * (lo + hi);
-  double cur = f(d);
-  for (int it = 0; it < 8; ++it) {
-    const double h = fmax(d * 1e-4, 1e-9);
-    const double fm = f(d - h);
-    const double fp = f(d + h);
-    const double g1 = (fp - fm) / (2.0 * h);
-    const double g2 = (fp - 2.0 * cur + fm) / (h * h);
-    if (!(g2 > 1e-12)) break;
-    const double step = g1 / g2;
-    const double dn = d - step;
-    if (!(dn > 1e-8 && dn < 1e6)) break;
-    const double vn = f(dn);
-    if (!(vn < cur)) break;
-    d = dn;
-    cur = vn;
-    if (fabs(step) < d * 1e-8) break;
-  }
-  return d;
-}
-
 // prep_lmm caches (src/model_lmm.cpp:124-153) from A = X~'DX~ (p x p,
 // row-major), b = X~'Dy~ and y~'Dy~ at the chosen delta; one thread. Besides
 // chi0, A^-1 and rss, the lower Cholesky factor of A (row-major, zeros when A
@@ -226,31 +176,31 @@ __device__ void reml_caches(double* A, const double* b, double y_dy, int p, int 
   for (int k = 0; k < p; ++k) chi0_out[static_cast<int64_t>(g) * p + k] = chi0[k];
 }
 
-// REML -loglik (src/model_lmm.cpp:10-37) for P <= 3 covariate columns,
-// evaluated by one warp:
-// each lane sums log v, w y^2, w x_a x_b and w y x_a over its samples in
-// registers, and xor-shuffle reductions give every lane the same totals
-// (IEEE addition is commutative), so there is no shared memory and no block
-// barrier. tot = [sum log v, y'Dy, X'DX packed (a <= b), X'Dy].
+// Grid of the search: f(1.0), then 1e-5 * 2^k for k = 0..33 (the loop dd <= 1e5,
+// dd *= 2); 1e-5 doubled k times is exact, so this is the reference's dd sequence.
+constexpr int kRbGridN = 35;
+__device__ __forceinline__ double rb_grid_delta(int j) { return j == 0 ? 1.0 : ldexp(1e-5, j - 1); }
+
+// ---- REML -loglik (src/model_lmm.cpp:10-37) for P <= 3 covariate columns,
+// evaluated by one warp: each lane sums log v, w y^2, w x_a x_b and w y x_a over
+// its samples in registers, and xor-shuffle reductions give every lane the same
+// totals (IEEE addition is commutative), so there is no shared memory and no
+// block barrier. tot = [sum log v, y'Dy, X'DX packed (a <= b), X'Dy].
 template <int P>
-__device__ __forceinline__ double reml_eval_warp(double delta, const double* __restrict__ yt,
-                                                 const double* __restrict__ Xt, const double* __restrict__ lam,
-                                                 int n, double* tot) {
-  constexpr int NQ = P * (P + 1) / 2;
-  constexpr int V = 2 + NQ + P;
-  const int lane = threadIdx.x & 31;
-  double acc[V];
-#pragma unroll
-  for (int q = 0; q < V; ++q) acc[q] = 0.0;
-  double prod = 1.0;
+struct RemlSums {
+  static constexpr int NQ = P * (P + 1) / 2, V = 2 + NQ + P;
+  double acc[V], prod = 1.0;
   int nprod = 0;
-  for (int i = lane; i < n; i += 32) {
-    double v = delta * lam[i] + 1.0;
+  __device__ __forceinline__ RemlSums() {
+#pragma unroll
+    for (int q = 0; q < V; ++q) acc[q] = 0.0;
+  }
+  // weight of a sample, and its log v: the sum of logs as the log of products of
+  // up to eight factors; every factor lies in [1e-12, 1e36] (larger ones take
+  // their own log), so a product stays within [1e-96, 1e288]
+  __device__ __forceinline__ double weight(double delta, double lam) {
+    double v = delta * lam + 1.0;
     if (v < 1e-12) v = 1e-12;
-    const double w = 1.0 / v;
-    // sum of log v as the log of products of up to eight factors: every factor
-    // lies in [1e-12, 1e36] (larger ones take their own log), so a product
-    // stays within [1e-96, 1e288]
     if (v <= 1e36) {
       prod *= v;
       if (++nprod == 8) {
@@ -261,27 +211,33 @@ __device__ __forceinline__ double reml_eval_warp(double delta, const double* __r
     } else {
       acc[0] += log(v);
     }
-    const double y = yt[i];
-    acc[1] += w * y * y;
-    double x[P];
+    return 1.0 / v;
+  }
+  __device__ __forceinline__ void add_x(double w, const double (&x)[P]) {
 #pragma unroll
-    for (int a = 0; a < P; ++a) x[a] = Xt[static_cast<int64_t>(a) * n + i];
-#pragma unroll
-    for (int a = 0; a < P; ++a) {
+    for (int a = 0; a < P; ++a)
 #pragma unroll
       for (int b = a; b < P; ++b) acc[2 + a * P - a * (a - 1) / 2 + (b - a)] += w * x[a] * x[b];
-      acc[2 + NQ + a] += w * y * x[a];
-    }
   }
-  acc[0] += log(prod);
+  __device__ __forceinline__ void add_y(double w, double y, const double (&x)[P]) {
+    acc[1] += w * y * y;
 #pragma unroll
-  for (int q = 0; q < V; ++q) {
-    double s = acc[q];
-#pragma unroll
-    for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    tot[q] = s;
+    for (int a = 0; a < P; ++a) acc[2 + NQ + a] += w * y * x[a];
   }
-  // Cholesky of X'DX; q = y'Dy - b'(X'DX)^-1 b as y'Dy - |z|^2 with L z = b
+  __device__ __forceinline__ void end() {
+    acc[0] += log(prod);
+#pragma unroll
+    for (int q = 0; q < V; ++q)
+#pragma unroll
+      for (int o = 16; o; o >>= 1) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], o);
+  }
+};
+
+// -loglik from the totals: Cholesky of X'DX; q = y'Dy - b'(X'DX)^-1 b as
+// y'Dy - |z|^2 with L z = b. No shuffles: lanes may hold different totals.
+template <int P>
+__device__ __forceinline__ double reml_ll(const double (&tot)[RemlSums<P>::V], int n) {
+  constexpr int NQ = RemlSums<P>::NQ;
   double L[P][P];
   double logdet_x = 0.0;
 #pragma unroll
@@ -315,29 +271,207 @@ __device__ __forceinline__ double reml_eval_warp(double delta, const double* __r
   return 0.5 * (df * log(q / df) + tot[0] + logdet_x);
 }
 
-// One warp per gene for P <= 3 (intercept and a few covariates):
-// optimize_delta (src/model_lmm.cpp:39-86) and the prep_lmm caches (:124-153).
-constexpr int kRemlWarpP = 3;
+// The grid's deltas are the same for every gene: one warp per grid point keeps
+// the weights w_k,i in Wg[i + n k] and the totals that y has no part in, sum log v
+// and X'DX, in Gt[k][1 + NQ].
 template <int P>
-__global__ void __launch_bounds__(256) reml_warp_kernel(const double* __restrict__ Ytil,
-                                                        const double* __restrict__ Xtil,
-                                                        const double* __restrict__ lam, int n, int G,
-                                                        double* delta_out, double* chi0_out, double* ainv_out,
-                                                        double* rss_out, double* a00L_out) {
-  constexpr int NQ = P * (P + 1) / 2;
-  const int g = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+__global__ void reml_grid_kernel(const double* __restrict__ Xtil, const double* __restrict__ lam, int n,
+                                 double* __restrict__ Wg, double* __restrict__ Gt) {
+  const int k = blockIdx.x, lane = threadIdx.x;
+  const double delta = rb_grid_delta(k);
+  RemlSums<P> s;
+  for (int i = lane; i < n; i += 32) {
+    const double w = s.weight(delta, lam[i]);
+    double x[P];
+#pragma unroll
+    for (int a = 0; a < P; ++a) x[a] = Xtil[static_cast<int64_t>(a) * n + i];
+    s.add_x(w, x);
+    Wg[static_cast<int64_t>(k) * n + i] = w;
+  }
+  s.end();
+  if (lane == 0) {
+    constexpr int NG = 1 + RemlSums<P>::NQ;
+    Gt[k * NG] = s.acc[0];
+#pragma unroll
+    for (int q = 1; q < NG; ++q) Gt[k * NG + q] = s.acc[1 + q];
+  }
+}
+
+// One warp per gene for P <= 3 (intercept and a few covariates): optimize_delta
+// (src/model_lmm.cpp:39-86: grid 1e-5..1e5 x2 and 1.0, 40 golden-section steps on
+// [best/4, best*4] clipped to [1e-8, 1e6], then up to 8 Newton steps on central
+// differences) and the prep_lmm caches (:124-153).
+//
+// Bound by FP64 issue: ~24 operations a sample and delta, of which the weight's
+// division and log are 15. The grid's weights come from reml_grid_kernel (four
+// operations a sample remain), five grid points share the loads of y and x, as do
+// the two deltas of a golden-section or Newton step; the -logliks of 32 grid
+// points, or of the step's two deltas, are then computed in different lanes of
+// one pass. Every sum keeps its order. n = 1000, 20,000 genes, P = 1: 6.7 ->
+// 4.2 ms; n = 1201, 2,000 genes, P = 2: 1.93 -> 0.93 ms.
+constexpr int kRemlWarpP = 3;
+constexpr int kRemlThreads = 64;  // two genes a block: an even last wave for a few thousand genes
+constexpr int kRemlGridStep = 5;  // grid points per pass over the samples
+template <int P>
+__global__ void __launch_bounds__(kRemlThreads) reml_warp_kernel(
+    const double* __restrict__ Ytil, const double* __restrict__ Xtil, const double* __restrict__ lam, int n, int G,
+    const double* __restrict__ Wg, const double* __restrict__ Gt, double* delta_out, double* chi0_out,
+    double* ainv_out, double* rss_out, double* a00L_out) {
+  constexpr int NQ = RemlSums<P>::NQ, V = RemlSums<P>::V, NG = 1 + NQ;
+  static_assert(kRbGridN % kRemlGridStep == 0 && kRbGridN <= 64, "grid passes");
+  const int g = blockIdx.x * (kRemlThreads >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (g >= G) return;  // whole warps only: no block barrier follows
   const double* yt = Ytil + static_cast<int64_t>(g) * n;
-  double tot[2 + NQ + P];
-  auto f = [&](double d) { return reml_eval_warp<P>(d, yt, Xtil, lam, n, tot); };
-  const double d = optimize_delta_dev(f, n - P);
-  f(d);
-  if ((threadIdx.x & 31) == 0) {
+  auto load_x = [&](int i, double (&x)[P]) {
+#pragma unroll
+    for (int a = 0; a < P; ++a) x[a] = Xtil[static_cast<int64_t>(a) * n + i];
+  };
+  auto f = [&](double d, RemlSums<P>& s) {
+    for (int i = lane; i < n; i += 32) {
+      const double w = s.weight(d, lam[i]), y = yt[i];
+      double x[P];
+      load_x(i, x);
+      s.add_x(w, x);
+      s.add_y(w, y, x);
+    }
+    s.end();
+    return reml_ll<P>(s.acc, n);
+  };
+  auto f1 = [&](double d) {
+    RemlSums<P> s;
+    return f(d, s);
+  };
+  auto f2 = [&](double d0, double d1, double& r0, double& r1) {
+    RemlSums<P> s0, s1;
+    for (int i = lane; i < n; i += 32) {
+      const double l = lam[i], y = yt[i];
+      double x[P];
+      load_x(i, x);
+      const double w0 = s0.weight(d0, l), w1 = s1.weight(d1, l);
+      s0.add_x(w0, x);
+      s0.add_y(w0, y, x);
+      s1.add_x(w1, x);
+      s1.add_y(w1, y, x);
+    }
+    s0.end();
+    s1.end();
+#pragma unroll
+    for (int q = 0; q < V; ++q) s0.acc[q] = lane < 16 ? s0.acc[q] : s1.acc[q];
+    const double r = reml_ll<P>(s0.acc, n);
+    r0 = __shfl_sync(0xffffffffu, r, 0);
+    r1 = __shfl_sync(0xffffffffu, r, 16);
+  };
+
+  double d = 1.0;
+  if (n - P > 0) {
+    // grid: lane l takes the totals of points l and 32 + l
+    double ty[2][1 + P];
+#pragma unroll 1
+    for (int k0 = 0; k0 < kRbGridN; k0 += kRemlGridStep) {
+      double acc[kRemlGridStep][1 + P];
+#pragma unroll
+      for (int j = 0; j < kRemlGridStep; ++j)
+#pragma unroll
+        for (int q = 0; q <= P; ++q) acc[j][q] = 0.0;
+      const double* wk = Wg + static_cast<int64_t>(k0) * n;
+      for (int i = lane; i < n; i += 32) {
+        const double y = yt[i];
+        double x[P];
+        load_x(i, x);
+#pragma unroll
+        for (int j = 0; j < kRemlGridStep; ++j) {
+          const double w = wk[static_cast<int64_t>(j) * n + i];
+          acc[j][0] += w * y * y;
+#pragma unroll
+          for (int a = 0; a < P; ++a) acc[j][1 + a] += w * y * x[a];
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < kRemlGridStep; ++j) {
+#pragma unroll
+        for (int q = 0; q <= P; ++q) {
+#pragma unroll
+          for (int o = 16; o; o >>= 1) acc[j][q] += __shfl_xor_sync(0xffffffffu, acc[j][q], o);
+          if (lane == ((k0 + j) & 31)) {
+            if (k0 + j < 32) ty[0][q] = acc[j][q];
+            else ty[1][q] = acc[j][q];
+          }
+        }
+      }
+    }
+    double ll[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int k = h * 32 + lane;
+      ll[h] = CUDART_NAN;  // no point: never the smallest
+      if (k < kRbGridN) {
+        double tot[V];
+        tot[0] = Gt[k * NG];
+        tot[1] = ty[h][0];
+#pragma unroll
+        for (int q = 1; q < NG; ++q) tot[1 + q] = Gt[k * NG + q];
+#pragma unroll
+        for (int a = 0; a < P; ++a) tot[2 + NQ + a] = ty[h][1 + a];
+        ll[h] = reml_ll<P>(tot, n);
+      }
+    }
+    // the first of the smallest values; where f(1.0) is NaN nothing is below it
+    int best = lane;
+    double bl = ll[0];
+    if (ll[1] < bl || (isnan(bl) && !isnan(ll[1]))) {
+      bl = ll[1];
+      best = 32 + lane;
+    }
+    const double ll0 = __shfl_sync(0xffffffffu, ll[0], 0);
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+      const double v = __shfl_xor_sync(0xffffffffu, bl, o);
+      const int k = __shfl_xor_sync(0xffffffffu, best, o);
+      if (v < bl || (v == bl && k < best) || (isnan(bl) && !isnan(v))) {
+        bl = v;
+        best = k;
+      }
+    }
+    const double best_d = rb_grid_delta(isnan(ll0) ? 0 : best);
+    double lo = best_d / 4.0, hi = best_d * 4.0;
+    if (lo < 1e-8) lo = 1e-8;
+    if (hi > 1e6) hi = 1e6;
+    const double phi = (1.0 + sqrt(5.0)) / 2.0;
+    for (int it = 0; it < 40; ++it) {
+      const double m1 = hi - (hi - lo) / phi;
+      const double m2 = lo + (hi - lo) / phi;
+      double v1, v2;
+      f2(m1, m2, v1, v2);
+      if (v1 < v2) hi = m2;
+      else lo = m1;
+    }
+    d = 0.5 * (lo + hi);
+    double cur = f1(d);
+    for (int it = 0; it < 8; ++it) {
+      const double h = fmax(d * 1e-4, 1e-9);
+      double fm, fp;
+      f2(d - h, d + h, fm, fp);
+      const double g1 = (fp - fm) / (2.0 * h);
+      const double g2 = (fp - 2.0 * cur + fm) / (h * h);
+      if (!(g2 > 1e-12)) break;
+      const double step = g1 / g2;
+      const double dn = d - step;
+      if (!(dn > 1e-8 && dn < 1e6)) break;
+      const double vn = f1(dn);
+      if (!(vn < cur)) break;
+      d = dn;
+      cur = vn;
+      if (fabs(step) < d * 1e-8) break;
+    }
+  }
+  RemlSums<P> s;
+  f(d, s);
+  if (lane == 0) {
     double A[P * P], L[P * P], e[P], x[P];
     for (int a = 0; a < P; ++a)
-      for (int b = a; b < P; ++b) A[a * P + b] = A[b * P + a] = tot[2 + a * P - a * (a - 1) / 2 + (b - a)];
+      for (int b = a; b < P; ++b) A[a * P + b] = A[b * P + a] = s.acc[2 + a * P - a * (a - 1) / 2 + (b - a)];
     delta_out[g] = d;
-    reml_caches(A, tot + 2 + NQ, tot[1], P, g, L, e, x, chi0_out, ainv_out, rss_out, a00L_out);
+    reml_caches(A, s.acc + 2 + NQ, s.acc[1], P, g, L, e, x, chi0_out, ainv_out, rss_out, a00L_out);
   }
 }
 
@@ -351,16 +485,12 @@ __global__ void __launch_bounds__(256) reml_warp_kernel(const double* __restrict
 // column advances its search (golden section, Newton) between rounds; the
 // grid phase, whose deltas every column shares, runs once before them.
 enum : int { kRbGolden = 1, kRbCentre, kRbNewtonPair, kRbNewtonStep, kRbFinal };
-constexpr int kRbGridN = 35;  // f(1.0), then 1e-5 * 2^k for k = 0..33 (the loop dd <= 1e5, dd *= 2)
 constexpr int kRbMaxRounds = 40 + 1 + 2 * 8 + 1;  // golden, centre, Newton, final
 
 struct RemlBatchState {
   int phase, k;
   double best_d, best_ll, lo, hi, d, cur, h, step, dn;
 };
-
-// 1e-5 doubled k times is exact, so this is the reference's dd sequence
-__device__ __forceinline__ double rb_grid_delta(int j) { return j == 0 ? 1.0 : ldexp(1e-5, j - 1); }
 
 __device__ void rb_propose(const RemlBatchState& s, double& d0, double& d1) {
   d0 = d1 = CUDART_NAN;
@@ -594,7 +724,7 @@ __global__ void rb_grid_advance_kernel(int C, int df, const double* __restrict__
 }
 
 // One warp per slot: W, W o y, sum log v (log of eight-factor products, as in
-// reml_eval_warp) and y'Dy. Slots with no delta (NaN) are skipped. Bound by the
+// RemlSums) and y'Dy. Slots with no delta (NaN) are skipped. Bound by the
 // latency of the FP64 reciprocals and loads when the columns are few, so a
 // lane takes eight of its samples per step, whose reciprocals overlap; the
 // sums keep each lane's sample order.
@@ -708,7 +838,7 @@ __device__ __forceinline__ void rb_back_solve(const double (&row)[GW], double y,
 constexpr int kRbThreads = 128;
 
 // Two groups of GW lanes per column, one per slot, evaluate the round's
-// -logliks; one lane then advances the search exactly as optimize_delta_dev
+// -logliks; one lane then advances the search exactly as reml_warp_kernel
 // does and proposes the next round's deltas. A column whose search has ended
 // keeps proposing its delta (kRbFinal) until every column's has: the caches are
 // formed for all of them at once (rb_final_kernel). *active counts the
@@ -2339,19 +2469,25 @@ void lmm_prep(eqtl_ctx* ctx, const PhenoDev& ph, bool y_rotated) {
   ws.ainv.alloc(static_cast<size_t>(G) * p * p);
   ws.a00L.alloc(static_cast<size_t>(G) * p * p);
   ws.rss.alloc(G);
-  ++ctx->launches;
   if (p <= kRemlWarpP) {
-    const unsigned blocks = static_cast<unsigned>((G + 7) / 8);
-    auto args = [&](auto kern) {
-      kern<<<blocks, 256, 0, st>>>(ws.Ytil.p, ws.Xtil.p, ctx->basis.lambda.p, n, G, ws.delta.p, ws.chi0.p,
-                                   ws.ainv.p, ws.rss.p, ws.a00L.p);
+    ws.reml_w.alloc(static_cast<size_t>(kRbGridN) * n);
+    ws.reml_tot.alloc(static_cast<size_t>(kRbGridN) * (1 + p * (p + 1) / 2));
+    ctx->launches += 2;
+    auto run = [&](auto pc) {
+      constexpr int P = decltype(pc)::value;
+      reml_grid_kernel<P><<<kRbGridN, 32, 0, st>>>(ws.Xtil.p, ctx->basis.lambda.p, n, ws.reml_w.p, ws.reml_tot.p);
+      constexpr int per = kRemlThreads / 32;
+      reml_warp_kernel<P><<<static_cast<unsigned>((G + per - 1) / per), kRemlThreads, 0, st>>>(
+          ws.Ytil.p, ws.Xtil.p, ctx->basis.lambda.p, n, G, ws.reml_w.p, ws.reml_tot.p, ws.delta.p, ws.chi0.p,
+          ws.ainv.p, ws.rss.p, ws.a00L.p);
     };
-    if (p == 1) args(reml_warp_kernel<1>);
-    else if (p == 2) args(reml_warp_kernel<2>);
-    else args(reml_warp_kernel<3>);
+    if (p == 1) run(std::integral_constant<int, 1>{});
+    else if (p == 2) run(std::integral_constant<int, 2>{});
+    else run(std::integral_constant<int, 3>{});
     EQTL_CUDA(cudaGetLastError());
     return;
   }
+  ++ctx->launches;
   // lanes per factorisation: the smallest group that holds p rows
   if (p <= 8) reml_batched<8>(ctx, n, p, G);
   else if (p <= 16) reml_batched<16>(ctx, n, p, G);
