@@ -246,12 +246,14 @@ __device__ __forceinline__ float max3_nan(float a, float b, float c) {
 constexpr float kFloorMagic = 8388608.0f;
 
 // The ACAT term of one u in [u_tiny, u_defer), as the lt_u branch of
-// acat_screen_u forms it (the same bits; outside that range a meaningless
-// value, without reading past the tables). tab: screen_tables.
+// acat_screen_u forms it (the same bits, its clamp of the last central interval
+// included; the tail's clamp cannot bind below u_defer; outside that range a
+// meaningless value, without reading past the tables). tab: screen_tables.
 __device__ __forceinline__ float cubic_term(float u, const TTable& T, uint32_t tab) {
   const float up = fminf(fabsf(u), T.u_defer);  // NaN: u_defer
-  const bool central = up < T.uq0;
-  const float x = central ? up * T.dqc_inv : (up - T.uq0) * T.dq_inv;
+  const bool central = up <= T.uq0;
+  const float x =
+      central ? fminf(up * T.dqc_inv, static_cast<float>(kTTableNa) - 1e-3f) : (up - T.uq0) * T.dq_inv;
   const float magic = central ? kFloorMagic : kFloorMagic + static_cast<float>(kTTableNa + 1);
   const float y = __fadd_rd(x, magic);
   const float f = x - (y - magic);
