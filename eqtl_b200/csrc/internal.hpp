@@ -217,7 +217,9 @@ struct Workspace {
   DevBuf<unsigned> res_hist, res_count;
   DevBuf<int> res_deferred, res_cand, res_dg, ref_mark;
   DevBuf<double> res_dp;
-  DevBuf<int2> tiny_pairs;
+  DevBuf<int2> tiny_pairs, pairs_again;
+  DevBuf<int> ref_again;
+  DevBuf<unsigned> ref_n_again;
   DevBuf<eqtl_gene_result> res_genes;
   DevBuf<eqtl_pair> res_pairs;
   PeerWork peer;

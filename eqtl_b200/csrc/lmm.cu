@@ -1814,6 +1814,11 @@ __global__ void snp_gate_kernel(const int64_t* __restrict__ kept, int64_t m, int
 }
 
 // raw dosages of listed kept SNPs, column-major [n, u]
+__global__ void listed_pairs_kernel(const int2* __restrict__ pairs, const int* __restrict__ list, int n,
+                                    int2* __restrict__ out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) out[i] = pairs[list[i]];
+}
 __global__ void raw_dosage_kernel(GenoRows src, const int32_t* __restrict__ col, int n,
                                   const int64_t* __restrict__ kept, const double* __restrict__ mu,
                                   const int* __restrict__ snps, int u, double* out) {
@@ -1839,7 +1844,7 @@ __global__ void raw_dosage_kernel(GenoRows src, const int32_t* __restrict__ col,
 // sum as a DGEMM's, whose products and partial sums round. Missing calls are 0
 // in g; a second pass contracts the 0 / 1 mask of missing calls and adds mu
 // times its sums. The DGEMM this replaces was half of the refinement: n = 2000,
-// 52,000 SNPs QG_FIGS.
+// 52,000 SNPs 11.4 -> 4 ms.
 // Digit rows: eigenvector j has rows 16 (j / 3) + 5 (j % 3) + k, so 16 rows hold
 // three whole eigenvectors (and one zero row).
 constexpr int kQgDigits = 5;
@@ -1848,6 +1853,7 @@ constexpr int kQgMaxN = 4095;
 // and their status checks cost what they save (n = 1,201, 2,400 SNPs: refinement
 // 0.74 ms with the DGEMM, 0.76 without).
 constexpr int64_t kQgMinWork = int64_t(10) << 30;
+constexpr int kQgDgemmCols = 2048;
 __host__ __device__ constexpr int64_t qg_rows(int n) { return static_cast<int64_t>((n + 2) / 3) * 16; }
 
 __global__ void __launch_bounds__(256)
@@ -1969,12 +1975,16 @@ struct QgEpi {
 // One warp per (gene, snp) pair from the FP64 rotated raw dosage Gt = Q'g:
 // gg = Gt'W Gt, yg = Gt'W y~, a = X~'W Gt with W = diag(1 / (delta lambda + 1)),
 // then the pair's printed statistics (test_lmm_gtil, src/scan_trans_lmm.cpp:11-40).
+// where (optional): the place of pair w in out. again (optional): collects the
+// pairs whose S has lost more than kQgCancel of gg.
+constexpr double kQgCancel = 1.0 / 1024;
 __global__ void lmm_refine_kernel(const double* __restrict__ Gt, int n, const int* __restrict__ pair_col,
                                   const int2* __restrict__ pairs, int n_pairs, const double* __restrict__ Ytil,
                                   const double* __restrict__ Xtil, int p, const double* __restrict__ lam,
                                   const double* __restrict__ delta, const double* __restrict__ chi0,
                                   const double* __restrict__ a00L, const double* __restrict__ rss, double df,
-                                  eqtl_pair* out) {
+                                  const int* __restrict__ where, int* __restrict__ again,
+                                  unsigned* __restrict__ n_again, eqtl_pair* out) {
   const int lane = threadIdx.x & 31;
   const int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (w >= n_pairs) return;
@@ -2002,9 +2012,11 @@ __global__ void lmm_refine_kernel(const double* __restrict__ Gt, int n, const in
     q.snp = pairs[w].y;
     q.gene = g;
     q.reserved = 0;
+    double S;
     lmm_stats_fp64(gg, yg, a, chi0 + static_cast<int64_t>(g) * p, a00L + static_cast<int64_t>(g) * p * p, rss[g],
-                   p, df, q);
-    out[w] = q;
+                   p, df, q, &S);
+    out[where ? where[w] : w] = q;
+    if (again && S < kQgCancel * gg) again[atomicAdd(n_again, 1u)] = w;
   }
 }
 
@@ -2662,40 +2674,77 @@ static void exact_qg(eqtl_ctx* ctx, const std::vector<int>& snps, double* out) {
   }
 }
 
+// Gt = Q'g of the u listed SNPs (ws.ref_snps) into ws.gt by DGEMM, with `pad`
+// zero columns after them.
+static void dgemm_qg(eqtl_ctx* ctx, int u, int pad) {
+  Geno& g = ctx->geno;
+  Workspace& ws = ctx->ws;
+  const int n = g.n, cols = u + pad;
+  ws.gt.alloc(static_cast<size_t>(n) * cols);
+  ws.graw.alloc(static_cast<size_t>(n) * cols);
+  ++ctx->launches;
+  raw_dosage_kernel<<<1184, 256, 0, ctx->stream>>>(g.rows(), g.col.p, n, g.kept.p, g.mu.p, ws.ref_snps.p, u, ws.graw.p);
+  EQTL_CUDA(cudaGetLastError());
+  if (pad)
+    EQTL_CUDA(cudaMemsetAsync(ws.graw.p + static_cast<size_t>(n) * u, 0, sizeof(double) * n * pad, ctx->stream));
+  const double one = 1.0, zero = 0.0;
+  EQTL_CHECK(cublasDgemm(blas_of(ctx), CUBLAS_OP_T, CUBLAS_OP_N, n, cols, n, &one, ctx->basis.Q.p, n, ws.graw.p, n,
+                         &zero, ws.gt.p, n) == CUBLAS_STATUS_SUCCESS,
+             EQTL_E_CUDA, "Q'g failed");
+}
+
 // FP64 statistics of the first n_pairs of ws.ref_pairs into ws.refined, against the
 // current LMM prep (ws.Ytil, Xtil, delta, chi0, ainv, rss): Gt = Q'g of the SNPs
 // involved (exactly on the tensor cores for many 2-bit rows, else by DGEMM: FP32
 // dosages, more than kQgMaxN samples, little work), then one warp per pair
 // (lmm_refine_kernel).
+//
+// A gene whose delta is at the top of its search leaves S = gg - a'A00^-1 a with a
+// millionth of gg: its last digits are Q'g's rounding, and p moves by 1e-8 with the
+// way Q'g was summed. Pairs that lose more than kQgCancel so are done again by
+// DGEMM, whose bits do not depend on how many SNPs are listed as long as it has a
+// grid of whole-K tiles (kQgDgemmCols columns), so that such a pair has the same p
+// in a scan of any size.
 static void lmm_refine_pairs(eqtl_ctx* ctx, int p, double df, int n_pairs) {
   Geno& g = ctx->geno;
   Workspace& ws = ctx->ws;
   cudaStream_t st = ctx->stream;
   const int n = g.n;
   if (n_pairs == 0) return;
-  const std::vector<int> snps = distinct_snps(ctx, n_pairs, g.m);
+  const std::vector<int> snps = distinct_snps(ctx, ws.ref_pairs.p, n_pairs, g.m);
   const int u = static_cast<int>(snps.size());
-  DevBuf<double>& gt = ws.gt;
-  gt.alloc(static_cast<size_t>(n) * u);
-  if (!g.dense && n <= kQgMaxN && static_cast<int64_t>(n) * n * u >= kQgMinWork) {
-    exact_qg(ctx, snps, gt.p);
-  } else {
-    DevBuf<double>& graw = ws.graw;
-    graw.alloc(static_cast<size_t>(n) * u);
-    ++ctx->launches;
-    raw_dosage_kernel<<<1184, 256, 0, st>>>(g.rows(), g.col.p, n, g.kept.p, g.mu.p, ws.ref_snps.p, u, graw.p);
-    EQTL_CUDA(cudaGetLastError());
-    const double one = 1.0, zero = 0.0;
-    EQTL_CHECK(cublasDgemm(blas_of(ctx), CUBLAS_OP_T, CUBLAS_OP_N, n, u, n, &one, ctx->basis.Q.p, n, graw.p, n,
-                           &zero, gt.p, n) == CUBLAS_STATUS_SUCCESS,
-               EQTL_E_CUDA, "Q'g failed");
-  }
-  ++ctx->launches;
+  const bool exact = !g.dense && n <= kQgMaxN && static_cast<int64_t>(n) * n * u >= kQgMinWork;
   ws.refined.alloc(static_cast<size_t>(n_pairs));
-  lmm_refine_kernel<<<static_cast<unsigned>((n_pairs + 7) / 8), 256, 0, st>>>(
-      gt.p, n, ws.ref_col.p, ws.ref_pairs.p, n_pairs, ws.Ytil.p, ws.Xtil.p, p, ctx->basis.lambda.p, ws.delta.p,
-      ws.chi0.p, ws.a00L.p, ws.rss.p, df, ws.refined.p);
+  auto refine = [&](const int2* pairs, int count, const int* where, int* again, unsigned* n_again) {
+    ++ctx->launches;
+    lmm_refine_kernel<<<static_cast<unsigned>((count + 7) / 8), 256, 0, st>>>(
+        ws.gt.p, n, ws.ref_col.p, pairs, count, ws.Ytil.p, ws.Xtil.p, p, ctx->basis.lambda.p, ws.delta.p, ws.chi0.p,
+        ws.a00L.p, ws.rss.p, df, where, again, n_again, ws.refined.p);
+    EQTL_CUDA(cudaGetLastError());
+  };
+  if (!exact) {
+    dgemm_qg(ctx, u, 0);
+    refine(ws.ref_pairs.p, n_pairs, nullptr, nullptr, nullptr);
+    return;
+  }
+  ws.gt.alloc(static_cast<size_t>(n) * u);
+  exact_qg(ctx, snps, ws.gt.p);
+  ws.ref_again.alloc(static_cast<size_t>(n_pairs));
+  ws.ref_n_again.alloc(1);
+  ws.ref_n_again.zero(st);
+  refine(ws.ref_pairs.p, n_pairs, nullptr, ws.ref_again.p, ws.ref_n_again.p);
+  unsigned n_again = 0;
+  ws.ref_n_again.download(&n_again, 1, st);
+  EQTL_CUDA(cudaStreamSynchronize(st));
+  if (n_again == 0) return;
+  ws.pairs_again.alloc(n_again);
+  ++ctx->launches;
+  listed_pairs_kernel<<<(n_again + 255) / 256, 256, 0, st>>>(ws.ref_pairs.p, ws.ref_again.p,
+                                                             static_cast<int>(n_again), ws.pairs_again.p);
   EQTL_CUDA(cudaGetLastError());
+  const int v = static_cast<int>(distinct_snps(ctx, ws.pairs_again.p, static_cast<int>(n_again), g.m).size());
+  dgemm_qg(ctx, v, std::max(0, kQgDgemmCols - v));
+  refine(ws.pairs_again.p, static_cast<int>(n_again), ws.ref_again.p, nullptr, nullptr);
 }
 
 // FP64 p of the n_tiny pairs of ws.tiny_pairs against the current LMM prep (see

@@ -599,7 +599,7 @@ void add_acat_terms(eqtl_gene_result* genes, const std::vector<int2>& pairs, con
   add_terms(genes, p_pairs, [&](size_t i) { return pairs[i].x; });
 }
 
-std::vector<int> distinct_snps(eqtl_ctx* ctx, int n_pairs, int64_t m) {
+std::vector<int> distinct_snps(eqtl_ctx* ctx, const int2* pairs, int n_pairs, int64_t m) {
   Workspace& ws = ctx->ws;
   cudaStream_t st = ctx->stream;
   ws.ref_mark.alloc(static_cast<size_t>(m));
@@ -608,9 +608,9 @@ std::vector<int> distinct_snps(eqtl_ctx* ctx, int n_pairs, int64_t m) {
   ws.ref_col.alloc(static_cast<size_t>(n_pairs));
   ws.res_count.alloc(4);
   ctx->launches += 2;
-  mark_snps_kernel<<<blocks(n_pairs, 256), 256, 0, st>>>(ws.ref_pairs.p, n_pairs, ws.ref_mark.p);
+  mark_snps_kernel<<<blocks(n_pairs, 256), 256, 0, st>>>(pairs, n_pairs, ws.ref_mark.p);
   compact(ctx, MarkedSnps{m, ws.ref_mark.p, ws.ref_snps.p}, m, total_of(ws));
-  snp_place_kernel<<<blocks(n_pairs, 256), 256, 0, st>>>(ws.ref_pairs.p, n_pairs, ws.ref_mark.p, ws.ref_col.p);
+  snp_place_kernel<<<blocks(n_pairs, 256), 256, 0, st>>>(pairs, n_pairs, ws.ref_mark.p, ws.ref_col.p);
   EQTL_CUDA(cudaGetLastError());
   uint64_t u = 0;
   EQTL_CUDA(cudaMemcpyAsync(&u, total_of(ws), sizeof(u), cudaMemcpyDeviceToHost, st));

@@ -75,9 +75,9 @@ struct ScanOutputs {
   int n_todo = 0, n_deferred = 0, n_tiny = 0;
 };
 
-// The distinct SNPs of ws.ref_pairs[0 .. n_pairs) (n_pairs > 0, SNPs below m) in
-// order, also on the device in ws.ref_snps; ws.ref_col: each pair's place among them.
-std::vector<int> distinct_snps(eqtl_ctx* ctx, int n_pairs, int64_t m);
+// The distinct SNPs of n_pairs > 0 pairs (device; SNPs below m) in order, also on
+// the device in ws.ref_snps; ws.ref_col: each pair's place among them.
+std::vector<int> distinct_snps(eqtl_ctx* ctx, const int2* pairs, int n_pairs, int64_t m);
 
 // Adds the reference's long-double ACAT term and `used` count of each pair
 // whose FP64 p (p_pairs[i]) enters ACAT (src/stats_extra.cpp:16-22).

@@ -174,9 +174,10 @@ EQTL_HD void lmm_stats_num_s(double num, double S, double rss_null, double df, e
 // and S = gg - a'A00^-1 a can cancel by orders of magnitude.
 constexpr int kStatsMaxP = 32;
 EQTL_HD void lmm_stats_fp64(double gg, double yg, const double* a, const double* chi0, const double* L,
-                            double rss_null, int p, double df, eqtl_pair& q) {
+                            double rss_null, int p, double df, eqtl_pair& q, double* S_out = nullptr) {
   q.beta = q.se = q.t = q.r2 = 0.0;
   q.p = 1.0;
+  if (S_out) *S_out = gg;
   if (gg < 1e-12) return;
   double aTu = 0, aTchi = 0;
   if (p > 0 && L[0] > 0) {
@@ -190,6 +191,7 @@ EQTL_HD void lmm_stats_fp64(double gg, double yg, const double* a, const double*
   }
   for (int x = 0; x < p; ++x) aTchi += a[x] * chi0[x];
   const double S = gg - aTu;
+  if (S_out) *S_out = S;
   if (S <= 1e-15) return;
   const double bg = (yg - aTchi) / S;
   double qq = rss_null - S * bg * bg;
