@@ -150,154 +150,6 @@ void residualize_genes(eqtl_ctx* ctx, const double* dX, const double* dXtXinv, i
 
 
 
-dev::Windows upload_windows(eqtl_ctx* ctx, const eqtl_scan_params* prm, int64_t m, int mode) {
-  dev::Windows w{};
-  w.mode = dev::kWinNone;
-  if (mode == dev::kWinNone || !prm->gene_chrom || !prm->gene_lo || !prm->gene_hi || !prm->snp_chrom ||
-      !prm->snp_pos)
-    return w;
-  Workspace& ws = ctx->ws;
-  ws.win_gc.upload(prm->gene_chrom, prm->n_genes, ctx->stream);
-  ws.win_glo.upload(prm->gene_lo, prm->n_genes, ctx->stream);
-  ws.win_ghi.upload(prm->gene_hi, prm->n_genes, ctx->stream);
-  // 16-SNP blocks, up to one 256-SNP tile past the last padded tile; the
-  // padding's values are not used (its SNPs are not tested)
-  const int64_t nb = ((m + 255) / 256 + 1) * 16;
-  ws.win_sc.alloc(static_cast<size_t>(nb * 16));
-  ws.win_sp.alloc(static_cast<size_t>(nb * 16));
-  ws.win_sc.upload(prm->snp_chrom, m, ctx->stream);
-  ws.win_sp.upload(prm->snp_pos, m, ctx->stream);
-  w.mode = mode;
-  w.gene_chrom = ws.win_gc.p;
-  w.gene_lo = ws.win_glo.p;
-  w.gene_hi = ws.win_ghi.p;
-  w.snp_chrom = ws.win_sc.p;
-  w.snp_pos = ws.win_sp.p;
-  std::vector<int32_t> bc(static_cast<size_t>(nb), -1);
-  std::vector<int64_t> blo(static_cast<size_t>(nb), 0), bhi(static_cast<size_t>(nb), -1);
-  for (int64_t b = 0; b * 16 < m; ++b) {
-    const int64_t s1 = std::min<int64_t>(m, b * 16 + 16);
-    int32_t c = prm->snp_chrom[b * 16];
-    int64_t lo = prm->snp_pos[b * 16], hi = lo;
-    for (int64_t s = b * 16 + 1; s < s1; ++s) {
-      if (prm->snp_chrom[s] != c) c = -1;
-      lo = std::min<int64_t>(lo, prm->snp_pos[s]);
-      hi = std::max<int64_t>(hi, prm->snp_pos[s]);
-    }
-    bc[static_cast<size_t>(b)] = c;
-    blo[static_cast<size_t>(b)] = lo;
-    bhi[static_cast<size_t>(b)] = hi;
-  }
-  ws.win_bc.upload(bc.data(), bc.size(), ctx->stream);
-  ws.win_blo.upload(blo.data(), blo.size(), ctx->stream);
-  ws.win_bhi.upload(bhi.data(), bhi.size(), ctx->stream);
-  w.blk_chrom = ws.win_bc.p;
-  w.blk_lo = ws.win_blo.p;
-  w.blk_hi = ws.win_bhi.p;
-  return w;
-}
-
-// Scans with windows (trans, cis) lay their genes out by window position, so
-// that the 32 genes of a warp and the 128 of a tile have windows close together:
-// a warp's 16-SNP blocks are then mostly in or out for all of its genes
-// (chunk_scope), and a cis tile's band covers few SNP tiles. In the caller's
-// order the windows of 32 genes scattered over the genome make over a quarter of
-// the blocks mixed, and the bands of 128 cover nearly every SNP. Consecutive
-// genes with the same window (permuted columns) stay together. Scans of genes in
-// random order, before and after: cis LMM (p = 16, 500 genes, 45,000 SNPs) 2.07 ->
-// 0.74 ms, cis LM (1,000 genes, 20,000 SNPs) 0.156 -> 0.093 ms, trans LM on dosages
-// (1.8e8 tests) 1.13 -> 0.79 ms. The order changes no pair's arithmetic.
-GeneOrder gene_order(eqtl_ctx* ctx, const eqtl_scan_params* prm) {
-  GeneOrder go;
-  const int G = prm->n_genes;
-  if (prm->exclude_cis == 0 || !prm->gene_chrom || !prm->gene_lo || !prm->gene_hi || !prm->snp_chrom ||
-      !prm->snp_pos)
-    return go;
-  struct Run {
-    uint32_t chrom;  // genes without a location (-1) last
-    int64_t lo;
-    int first, count;
-  };
-  std::vector<Run> runs;
-  for (int g = 0; g < G; ++g) {
-    const uint32_t c = static_cast<uint32_t>(prm->gene_chrom[g]);
-    if (g > 0 && prm->gene_chrom[g] == prm->gene_chrom[g - 1] && prm->gene_lo[g] == prm->gene_lo[g - 1] &&
-        prm->gene_hi[g] == prm->gene_hi[g - 1])
-      ++runs.back().count;
-    else
-      runs.push_back({c, prm->gene_lo[g], g, 1});
-  }
-  auto before = [](const Run& a, const Run& b) {
-    if (a.chrom != b.chrom) return a.chrom < b.chrom;
-    if (a.lo != b.lo) return a.lo < b.lo;
-    return a.first < b.first;
-  };
-  if (std::is_sorted(runs.begin(), runs.end(), before)) return go;
-  std::sort(runs.begin(), runs.end(), before);
-  Workspace& ws = ctx->ws;
-  std::vector<int> gene(static_cast<size_t>(G));
-  ws.gene_row_h.resize(static_cast<size_t>(G));
-  int r = 0;
-  for (const Run& run : runs)
-    for (int k = 0; k < run.count; ++k, ++r) {
-      gene[static_cast<size_t>(r)] = run.first + k;
-      ws.gene_row_h[static_cast<size_t>(run.first + k)] = r;
-    }
-  ws.row_gene.upload(gene.data(), gene.size(), ctx->stream);
-  ws.gene_row.upload(ws.gene_row_h.data(), ws.gene_row_h.size(), ctx->stream);
-  go.row = ws.gene_row.p;
-  go.gene = ws.row_gene.p;
-  return go;
-}
-
-// Banded tile list of a cis scan (scope 2): for every tile of 128 operand rows, the
-// SNP tiles of NT kept SNPs that hold some gene's window. Needs the kept
-// SNPs grouped by chromosome in position order (as in a sorted .bim); returns
-// false otherwise, and the caller runs the full grid masked to the windows.
-bool cis_tile_list(eqtl_ctx* ctx, const eqtl_scan_params* prm, const GeneOrder& go, int64_t m, int NT,
-                   const int2*& list, int& n_list) {
-  list = nullptr;
-  n_list = 0;
-  if (prm->exclude_cis != 2 || !prm->gene_chrom || !prm->snp_chrom || !prm->snp_pos || m == 0) return false;
-  // chromosome blocks [first, last) of the kept SNPs, positions non-decreasing
-  std::map<int32_t, std::pair<int64_t, int64_t>> block;
-  for (int64_t k = 0; k < m; ++k) {
-    const int32_t c = prm->snp_chrom[k];
-    auto it = block.find(c);
-    if (it == block.end()) {
-      block.emplace(c, std::make_pair(k, k + 1));
-      continue;
-    }
-    if (it->second.second != k || prm->snp_pos[k] < prm->snp_pos[k - 1]) return false;
-    it->second.second = k + 1;
-  }
-  const int G = prm->n_genes;
-  const int tiles_a = (G + dev::kTileM - 1) / dev::kTileM;
-  const int64_t tiles_b = (m + NT - 1) / NT;
-  std::vector<uint8_t> mark(static_cast<size_t>(tiles_a) * tiles_b, 0);
-  for (int g = 0; g < G; ++g) {
-    auto it = block.find(prm->gene_chrom[g]);
-    if (prm->gene_chrom[g] < 0 || it == block.end()) continue;
-    const int64_t* p0 = prm->snp_pos + it->second.first;
-    const int64_t* p1 = prm->snp_pos + it->second.second;
-    const int64_t k_lo = std::lower_bound(p0, p1, prm->gene_lo[g]) - prm->snp_pos;
-    const int64_t k_hi = std::upper_bound(p0, p1, prm->gene_hi[g]) - prm->snp_pos;  // exclusive
-    if (k_hi <= k_lo) continue;
-    const int r = go.row ? ctx->ws.gene_row_h[static_cast<size_t>(g)] : g;
-    uint8_t* row = &mark[static_cast<size_t>(r / dev::kTileM) * tiles_b];
-    for (int64_t tb = k_lo / NT; tb <= (k_hi - 1) / NT; ++tb) row[tb] = 1;
-  }
-  std::vector<int2> tl;
-  for (int ta = 0; ta < tiles_a; ++ta)
-    for (int64_t tb = 0; tb < tiles_b; ++tb)
-      if (mark[static_cast<size_t>(ta) * tiles_b + tb]) tl.push_back(make_int2(ta, static_cast<int>(tb)));
-  n_list = static_cast<int>(tl.size());
-  if (n_list == 0) tl.push_back(make_int2(0, 0));  // keeps a valid (unused) device pointer
-  ctx->ws.tile_list.upload(tl.data(), tl.size(), ctx->stream);
-  list = ctx->ws.tile_list.p;
-  return true;
-}
-
 dev::TTable device_ttable(eqtl_ctx* ctx, double df, bool normal) {
   EQTL_CHECK(normal || df > 0, EQTL_E_ARG, "residual degrees of freedom must be positive");
   if (normal) df = kZTableD;

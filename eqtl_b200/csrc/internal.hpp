@@ -240,8 +240,10 @@ struct Workspace {
   DevBuf<eqtl_pair> refined;
   DevBuf<double> tiny_p;
   DevBuf<int2> tile_list;
+  DevBuf<uint64_t> win_count;  // chromosome runs, listed tiles, unsorted
+  DevBuf<int> win_runs;
+  DevBuf<uint8_t> win_mark;
   DevBuf<int> gene_row, row_gene;      // GeneOrder of the current scan
-  std::vector<int> gene_row_h;
   DevBuf<__half> q_hi, q_lo;  // rotation: split eigenvector operand
   DevBuf<int> ref_snps, ref_col;
   DevBuf<__half> qg_dose, qg_mask;  // exact_qg: dosages of the listed SNPs, mask of their missing calls

@@ -3180,7 +3180,7 @@ static void scan_trans_lmm_impl(eqtl_ctx* ctx, const eqtl_scan_params* prm, cons
   ScanOutputs so(ctx, G, m, expected_candidates(prm, m));
   const int2* tiles = nullptr;  // cis: banded tile list (NT of the kernel that runs)
   int n_tiles = 0;
-  if (!simt) cis_tile_list(ctx, prm, go, m, grouped ? LmmGroupEpi::kTileN : 128, tiles, n_tiles);
+  if (!simt) cis_tile_list(ctx, win, G, go, m, grouped ? LmmGroupEpi::kTileN : 128, tiles, n_tiles);
   std::unique_ptr<StageScope> scan_timer(new StageScope(ctx, EQTL_STAGE_SCAN));
   if (m > 0 && grouped) {
     Rotated& Rt = ctx->rot;
@@ -3791,7 +3791,7 @@ void scan_glm(eqtl_ctx* ctx, const eqtl_scan_params* prm, const double* Y, const
   ScanOutputs so(ctx, G, m, expected_candidates(prm, m));
   const int2* tiles = nullptr;
   int n_tiles = 0;
-  cis_tile_list(ctx, prm, go, m, grouped ? GlmGroupEpi::kTileN : 128, tiles, n_tiles);
+  cis_tile_list(ctx, win, G, go, m, grouped ? GlmGroupEpi::kTileN : 128, tiles, n_tiles);
   std::unique_ptr<StageScope> scan_timer(new StageScope(ctx, EQTL_STAGE_SCAN));
   if (m > 0 && grouped) {
     GlmGroupEpiParams ep{};

@@ -10,6 +10,7 @@
 // refined pair and their page faults; now 10, of which the host's long-double terms
 // are 5.
 #include "block_sort.cuh"
+#include "compact.cuh"
 #include "host_par.hpp"
 #include "scan_host.hpp"
 
@@ -33,60 +34,6 @@ __global__ void __launch_bounds__(256) radix_count_kernel(const uint64_t* __rest
   }
   __syncthreads();
   hist[static_cast<int64_t>(threadIdx.x) * gridDim.x + blockIdx.x] = h[threadIdx.x];
-}
-
-// Sum of v over the lower threads of a block (blockDim.x a multiple of 32, at
-// most 1024); total = over all. sm: 33 values.
-template <class T>
-__device__ __forceinline__ T block_prefix(T v, T* sm, T& total) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  T s = v;
-#pragma unroll
-  for (int o = 1; o < 32; o *= 2) {
-    const T x = __shfl_up_sync(0xffffffffu, s, o);
-    if (lane >= o) s += x;
-  }
-  __syncthreads();  // sm of an earlier call has been read
-  if (lane == 31) sm[w] = s;
-  __syncthreads();
-  if (w == 0) {
-    const T x = lane < nw ? sm[lane] : T(0);
-    T y = x;
-#pragma unroll
-    for (int o = 1; o < 32; o *= 2) {
-      const T z = __shfl_up_sync(0xffffffffu, y, o);
-      if (lane >= o) y += z;
-    }
-    sm[lane] = y - x;
-    if (lane == 31) sm[32] = y;
-  }
-  __syncthreads();
-  total = sm[32];
-  return sm[w] + s - v;
-}
-
-// Exclusive prefix sums of v in place, by one block of 1024; total (optional).
-template <class T>
-__global__ void __launch_bounds__(1024) prefix_kernel(T* __restrict__ v, int64_t n, T* total) {
-  __shared__ T sm[33];
-  T carry = 0;
-  for (int64_t base = 0; base < n; base += 4096) {
-    const int64_t i = base + 4 * threadIdx.x;
-    T x[4], s = 0;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      x[j] = i + j < n ? v[i + j] : T(0);
-      s += x[j];
-    }
-    T all, at = carry + block_prefix(s, sm, all);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      if (i + j < n) v[i + j] = at;
-      at += x[j];
-    }
-    carry += all;
-  }
-  if (total && threadIdx.x == 0) *total = carry;
 }
 
 // Stable scatter by the digit at `shift`; hist: prefix sums of radix_count_kernel's.
@@ -130,39 +77,6 @@ __global__ void __launch_bounds__(256) radix_scatter_kernel(const uint64_t* __re
 #pragma unroll
   for (int r = 0; r < R; ++r)
     if (base + r * 32 + lane < n) out[at[w][(k[r] >> shift) & 255] + rank[r]] = k[r];
-}
-
-// Stable compaction into two lists: f.test(i) is 1 in the low half for an entry
-// of the first list, 1 in the high half for one of the second; f.emit(i, t, at)
-// gets the places in both. Blocks of 1024 items.
-constexpr int kCompactTile = 1024;
-template <class F>
-__global__ void __launch_bounds__(256) compact_count_kernel(F f, uint64_t* __restrict__ blk) {
-  __shared__ uint64_t sm[33];
-  const int64_t i = static_cast<int64_t>(blockIdx.x) * kCompactTile + 4 * threadIdx.x, n = f.size();
-  uint64_t s = 0, all;
-#pragma unroll
-  for (int j = 0; j < 4; ++j)
-    if (i + j < n) s += f.test(i + j);
-  block_prefix(s, sm, all);
-  if (threadIdx.x == 0) blk[blockIdx.x] = all;
-}
-template <class F>
-__global__ void __launch_bounds__(256) compact_emit_kernel(F f, const uint64_t* __restrict__ blk) {
-  __shared__ uint64_t sm[33];
-  const int64_t i = static_cast<int64_t>(blockIdx.x) * kCompactTile + 4 * threadIdx.x, n = f.size();
-  uint64_t t[4], s = 0, all;
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    t[j] = i + j < n ? f.test(i + j) : 0;
-    s += t[j];
-  }
-  uint64_t at = blk[blockIdx.x] + block_prefix(s, sm, all);
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    if (t[j]) f.emit(i + j, t[j], at);
-    at += t[j];
-  }
 }
 
 // ------------------------------------------------ the pairs to refine
@@ -428,8 +342,6 @@ int bits_of(int64_t values) {  // bits that hold 0 .. values - 1
   return b;
 }
 
-unsigned blocks(int64_t n, int64_t per) { return static_cast<unsigned>(std::max<int64_t>((n + per - 1) / per, 1)); }
-
 // Sorts *n_dev <= n_max keys by bits [lo, hi); a, b: buffers that hold n_max.
 // Returns the one with the result.
 uint64_t* radix_sort(eqtl_ctx* ctx, uint64_t* a, uint64_t* b, const unsigned* n_dev, int64_t n_max, int lo, int hi) {
@@ -445,18 +357,6 @@ uint64_t* radix_sort(eqtl_ctx* ctx, uint64_t* a, uint64_t* b, const unsigned* n_
     std::swap(a, b);
   }
   return a;
-}
-
-template <class F>
-void compact(eqtl_ctx* ctx, const F& f, int64_t n_max, uint64_t* total) {
-  const unsigned nb = blocks(n_max, kCompactTile);
-  DevBuf<uint64_t>& blk = ctx->ws.res_blk;
-  blk.alloc(nb);
-  ctx->launches += 3;
-  compact_count_kernel<F><<<nb, 256, 0, ctx->stream>>>(f, blk.p);
-  prefix_kernel<uint64_t><<<1, 1024, 0, ctx->stream>>>(blk.p, nb, total);
-  compact_emit_kernel<F><<<nb, 256, 0, ctx->stream>>>(f, blk.p);
-  EQTL_CUDA(cudaGetLastError());
 }
 
 // res_count: [0] keys, [1] tiny pairs, [2, 3] totals of a compaction

@@ -37,7 +37,7 @@ struct GeneOrder {
 };
 GeneOrder gene_order(eqtl_ctx* ctx, const eqtl_scan_params* prm);
 
-bool cis_tile_list(eqtl_ctx* ctx, const eqtl_scan_params* prm, const GeneOrder& go, int64_t m, int NT,
+bool cis_tile_list(eqtl_ctx* ctx, const dev::Windows& w, int G, const GeneOrder& go, int64_t m, int NT,
                    const int2*& list, int& n_list);
 
 // Resolves the phenotypes of a scan call: uploads (Y, X) when given,

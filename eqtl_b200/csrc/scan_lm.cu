@@ -467,7 +467,7 @@ void scan_trans_lm(eqtl_ctx* ctx, const eqtl_scan_params* prm, const double* Y, 
   ScanOutputs so(ctx, G, m, expected_candidates(prm, m));
   const int2* tiles = nullptr;  // cis: banded tile list
   int n_tiles = 0;
-  cis_tile_list(ctx, prm, go, m, 256, tiles, n_tiles);
+  cis_tile_list(ctx, ep.win, G, go, m, 256, tiles, n_tiles);
   std::unique_ptr<StageScope> scan_timer(new StageScope(ctx, EQTL_STAGE_SCAN));
   if (m > 0) {
     so.run([&](GeneOut out) {
