@@ -216,7 +216,7 @@ struct Workspace {
   DevBuf<uint64_t> res_key[2], res_blk;
   DevBuf<unsigned> res_hist, res_count;
   DevBuf<int> res_deferred, res_cand, res_dg, ref_mark;
-  DevBuf<double> res_dp;
+  DevBuf<double> res_dp, ref_sums;
   DevBuf<int2> tiny_pairs, pairs_again;
   DevBuf<int> ref_again;
   DevBuf<unsigned> ref_n_again;

@@ -2020,16 +2020,14 @@ struct QgEpi {
 // One warp per (gene, snp) pair from the FP64 rotated raw dosage Gt = Q'g:
 // gg = Gt'W Gt, yg = Gt'W y~, a = X~'W Gt with W = diag(1 / (delta lambda + 1)),
 // then the pair's printed statistics (test_lmm_gtil, src/scan_trans_lmm.cpp:11-40).
-// where (optional): the place of pair w in out. again (optional): collects the
-// pairs whose S has lost more than kQgCancel of gg.
-constexpr double kQgCancel = 1.0 / 1024;
-__global__ void lmm_refine_kernel(const double* __restrict__ Gt, int n, const int* __restrict__ pair_col,
-                                  const int2* __restrict__ pairs, int n_pairs, const double* __restrict__ Ytil,
-                                  const double* __restrict__ Xtil, int p, const double* __restrict__ lam,
-                                  const double* __restrict__ delta, const double* __restrict__ chi0,
-                                  const double* __restrict__ a00L, const double* __restrict__ rss, double df,
-                                  const int* __restrict__ where, int* __restrict__ again,
-                                  unsigned* __restrict__ n_again, eqtl_pair* out) {
+// FP64 sums [gg, yg, a_0 .. a_{p-1}] of listed (gene, snp) pairs, one warp per pair
+// (p <= PM, the a_k in registers: an array indexed by a runtime p lives in local
+// memory and chains every sample's update through it).
+template <int PM>
+__global__ void lmm_pair_sums_kernel(const double* __restrict__ Gt, int n, const int* __restrict__ pair_col,
+                                     const int2* __restrict__ pairs, int n_pairs, const double* __restrict__ Ytil,
+                                     const double* __restrict__ Xtil, int p, const double* __restrict__ lam,
+                                     const double* __restrict__ delta, double* __restrict__ sums) {
   const int lane = threadIdx.x & 31;
   const int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (w >= n_pairs) return;
@@ -2037,32 +2035,60 @@ __global__ void lmm_refine_kernel(const double* __restrict__ Gt, int n, const in
   const double* gt = Gt + static_cast<int64_t>(pair_col[w]) * n;
   const double* yt = Ytil + static_cast<int64_t>(g) * n;
   const double d = delta[g];
-  double gg = 0, yg = 0, a[kMaxPLmm];
-  for (int k = 0; k < p; ++k) a[k] = 0;
+  double gg = 0, yg = 0, a[PM];
+#pragma unroll
+  for (int k = 0; k < PM; ++k) a[k] = 0;
+#pragma unroll(PM <= 4 ? 8 : 2)
   for (int i = lane; i < n; i += 32) {
     double v = d * lam[i] + 1.0;
     if (v < 1e-12) v = 1e-12;
     const double dg = gt[i] / v;
     gg += dg * gt[i];
     yg += dg * yt[i];
-    for (int k = 0; k < p; ++k) a[k] += Xtil[static_cast<int64_t>(k) * n + i] * dg;
+#pragma unroll
+    for (int k = 0; k < PM; ++k)
+      if (k < p) a[k] += Xtil[static_cast<int64_t>(k) * n + i] * dg;
   }
   for (int o = 16; o; o >>= 1) {
     gg += __shfl_xor_sync(0xffffffffu, gg, o);
     yg += __shfl_xor_sync(0xffffffffu, yg, o);
-    for (int k = 0; k < p; ++k) a[k] += __shfl_xor_sync(0xffffffffu, a[k], o);
+#pragma unroll
+    for (int k = 0; k < PM; ++k)
+      if (k < p) a[k] += __shfl_xor_sync(0xffffffffu, a[k], o);
   }
-  if (lane == 0) {
-    eqtl_pair q;
-    q.snp = pairs[w].y;
-    q.gene = g;
-    q.reserved = 0;
-    double S;
-    lmm_stats_fp64(gg, yg, a, chi0 + static_cast<int64_t>(g) * p, a00L + static_cast<int64_t>(g) * p * p, rss[g],
-                   p, df, q, &S);
-    out[where ? where[w] : w] = q;
-    if (again && S < kQgCancel * gg) again[atomicAdd(n_again, 1u)] = w;
-  }
+  if (lane != 0) return;
+  double* out = sums + static_cast<int64_t>(w) * (p + 2);
+  out[0] = gg;
+  out[1] = yg;
+#pragma unroll
+  for (int k = 0; k < PM; ++k)
+    if (k < p) out[2 + k] = a[k];
+}
+
+// The pairs' statistics from their sums, one thread per pair (the p-value's
+// continued fraction is most of the work and does not fill a warp per pair). where
+// (optional): the place of pair w in out. again (optional): collects the pairs whose
+// S has lost more than kQgCancel of gg. Both kernels, n = 1000, p = 1, 54,600
+// pairs: 0.94 -> 0.45 ms.
+constexpr double kQgCancel = 1.0 / 1024;
+__global__ void lmm_pair_stats_kernel(const double* __restrict__ sums, const int2* __restrict__ pairs, int n_pairs,
+                                      int p, const double* __restrict__ chi0, const double* __restrict__ a00L,
+                                      const double* __restrict__ rss, double df, const int* __restrict__ where,
+                                      int* __restrict__ again, unsigned* __restrict__ n_again,
+                                      eqtl_pair* __restrict__ out) {
+  const int w = blockIdx.x * blockDim.x + threadIdx.x;
+  if (w >= n_pairs) return;
+  const int g = pairs[w].x;
+  const double* s = sums + static_cast<int64_t>(w) * (p + 2);
+  eqtl_pair q;
+  q.snp = pairs[w].y;
+  q.gene = g;
+  q.reserved = 0;
+  double S;
+  lmm_stats_fp64(s[0], s[1], s + 2, chi0 + static_cast<int64_t>(g) * p, a00L + static_cast<int64_t>(g) * p * p, rss[g],
+                 p, df, q, &S);
+  out[where ? where[w] : w] = q;
+  if (again && S < kQgCancel * s[0]) again[atomicAdd(n_again, 1u)] = w;
 }
 
 // ------------------------------------------------- tiny-|t| pairs in FP64
@@ -2090,12 +2116,15 @@ __global__ void lmm_wr_kernel(const double* __restrict__ Ytil, const double* __r
   }
 }
 
-__global__ void lmm_tiny_kernel(GenoRows src, const int32_t* __restrict__ col, int n, int k_pad, const int64_t* __restrict__ kept, const double* __restrict__ mu,
-                                const double* __restrict__ U, int64_t u_stride, const __half* __restrict__ gt_hi,
-                                const __half* __restrict__ gt_lo, double inv_s1, const double* __restrict__ Xtil,
-                                int p, const double* __restrict__ lam, const double* __restrict__ delta,
-                                const double* __restrict__ ainv, const double* __restrict__ rss, double df,
-                                const int2* __restrict__ pairs, int n_pairs, double* p_out) {
+// Sums [num, gg, a_0 .. a_{p-1}] by a warp per pair, then p by a thread per pair, as
+// for the refined pairs. n = 1000, p = 1, 62,000 pairs: 1.00 -> 0.65 ms.
+template <int PM>
+__global__ void lmm_tiny_sums_kernel(GenoRows src, const int32_t* __restrict__ col, int n, int k_pad,
+                                     const int64_t* __restrict__ kept, const double* __restrict__ mu,
+                                     const double* __restrict__ U, int64_t u_stride, const __half* __restrict__ gt_hi,
+                                     const __half* __restrict__ gt_lo, double inv_s1, const double* __restrict__ Xtil,
+                                     int p, const double* __restrict__ lam, const double* __restrict__ delta,
+                                     const int2* __restrict__ pairs, int n_pairs, double* __restrict__ sums) {
   const int lane = threadIdx.x & 31;
   const int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (w >= n_pairs) return;
@@ -2107,8 +2136,10 @@ __global__ void lmm_tiny_kernel(GenoRows src, const int32_t* __restrict__ col, i
   const __half* gh = gt_hi + r * k_pad;
   const __half* gl = gt_lo + r * k_pad;
   const double d = delta[g];
-  double num = 0, gg = 0, a[kMaxPLmm];
-  for (int k = 0; k < p; ++k) a[k] = 0;
+  double num = 0, gg = 0, a[PM];
+#pragma unroll
+  for (int k = 0; k < PM; ++k) a[k] = 0;
+#pragma unroll(PM <= 4 ? 8 : 2)
   for (int i = lane; i < n; i += 32) {
     const double dose = src.dosage(s, col[i]);
     num += (isnan(dose) ? mus : dose) * u[i];
@@ -2117,29 +2148,47 @@ __global__ void lmm_tiny_kernel(GenoRows src, const int32_t* __restrict__ col, i
     const double gt = (static_cast<double>(__half2float(gh[i])) + static_cast<double>(__half2float(gl[i]))) * inv_s1;
     const double dg = gt / v;
     gg += dg * gt;
-    for (int k = 0; k < p; ++k) a[k] += Xtil[static_cast<int64_t>(k) * n + i] * dg;
+#pragma unroll
+    for (int k = 0; k < PM; ++k)
+      if (k < p) a[k] += Xtil[static_cast<int64_t>(k) * n + i] * dg;
   }
   for (int o = 16; o; o >>= 1) {
     num += __shfl_xor_sync(0xffffffffu, num, o);
     gg += __shfl_xor_sync(0xffffffffu, gg, o);
-    for (int k = 0; k < p; ++k) a[k] += __shfl_xor_sync(0xffffffffu, a[k], o);
+#pragma unroll
+    for (int k = 0; k < PM; ++k)
+      if (k < p) a[k] += __shfl_xor_sync(0xffffffffu, a[k], o);
   }
-  if (lane == 0) {
-    eqtl_pair q;
-    double S = -1.0;
-    if (!(gg < 1e-12)) {
-      const double* A = ainv + static_cast<int64_t>(g) * p * p;
-      double aTu = 0;
-      for (int x = 0; x < p; ++x) {
-        double ux = 0;
-        for (int y = 0; y < p; ++y) ux += A[x * p + y] * a[y];
-        aTu += a[x] * ux;
-      }
-      S = gg - aTu;
+  if (lane != 0) return;
+  double* out = sums + static_cast<int64_t>(w) * (p + 2);
+  out[0] = num;
+  out[1] = gg;
+#pragma unroll
+  for (int k = 0; k < PM; ++k)
+    if (k < p) out[2 + k] = a[k];
+}
+__global__ void lmm_tiny_p_kernel(const double* __restrict__ sums, const int2* __restrict__ pairs, int n_pairs, int p,
+                                  const double* __restrict__ ainv, const double* __restrict__ rss, double df,
+                                  double* __restrict__ p_out) {
+  const int w = blockIdx.x * blockDim.x + threadIdx.x;
+  if (w >= n_pairs) return;
+  const int g = pairs[w].x;
+  const double* s = sums + static_cast<int64_t>(w) * (p + 2);
+  const double gg = s[1], *a = s + 2;
+  eqtl_pair q;
+  double S = -1.0;
+  if (!(gg < 1e-12)) {
+    const double* A = ainv + static_cast<int64_t>(g) * p * p;
+    double aTu = 0;
+    for (int x = 0; x < p; ++x) {
+      double ux = 0;
+      for (int y = 0; y < p; ++y) ux += A[x * p + y] * a[y];
+      aTu += a[x] * ux;
     }
-    lmm_stats_num_s(num, S, rss[g], df, q);
-    p_out[w] = q.p;
+    S = gg - aTu;
   }
+  lmm_stats_num_s(s[0], S, rss[g], df, q);
+  p_out[w] = q.p;
 }
 
 }  // namespace dev
@@ -2717,6 +2766,16 @@ static void exact_qg(eqtl_ctx* ctx, const std::vector<int>& snps, double* out) {
   }
 }
 
+// f(std::integral_constant<int, PM>) with the least PM >= p of the per-pair kernels.
+template <class F>
+static void with_p(int p, F&& f) {
+  if (p <= 2) f(std::integral_constant<int, 2>{});
+  else if (p <= 4) f(std::integral_constant<int, 4>{});
+  else if (p <= 8) f(std::integral_constant<int, 8>{});
+  else if (p <= 16) f(std::integral_constant<int, 16>{});
+  else f(std::integral_constant<int, kMaxPLmm>{});
+}
+
 // Gt = Q'g of the u listed SNPs (ws.ref_snps) into ws.gt by DGEMM, with `pad`
 // zero columns after them.
 static void dgemm_qg(eqtl_ctx* ctx, int u, int pad) {
@@ -2739,8 +2798,8 @@ static void dgemm_qg(eqtl_ctx* ctx, int u, int pad) {
 // FP64 statistics of the first n_pairs of ws.ref_pairs into ws.refined, against the
 // current LMM prep (ws.Ytil, Xtil, delta, chi0, ainv, rss): Gt = Q'g of the SNPs
 // involved (exactly on the tensor cores for many 2-bit rows, else by DGEMM: FP32
-// dosages, more than kQgMaxN samples, little work), then one warp per pair
-// (lmm_refine_kernel).
+// dosages, more than kQgMaxN samples, little work), then the pairs' sums and
+// statistics.
 //
 // A gene whose delta is at the top of its search leaves S = gg - a'A00^-1 a with a
 // millionth of gg: its last digits are Q'g's rounding, and p moves by 1e-8 with the
@@ -2759,10 +2818,15 @@ static void lmm_refine_pairs(eqtl_ctx* ctx, int p, double df, int n_pairs) {
   const bool exact = !g.dense && n <= kQgMaxN && static_cast<int64_t>(n) * n * u >= kQgMinWork;
   ws.refined.alloc(static_cast<size_t>(n_pairs));
   auto refine = [&](const int2* pairs, int count, const int* where, int* again, unsigned* n_again) {
-    ++ctx->launches;
-    lmm_refine_kernel<<<static_cast<unsigned>((count + 7) / 8), 256, 0, st>>>(
-        ws.gt.p, n, ws.ref_col.p, pairs, count, ws.Ytil.p, ws.Xtil.p, p, ctx->basis.lambda.p, ws.delta.p, ws.chi0.p,
-        ws.a00L.p, ws.rss.p, df, where, again, n_again, ws.refined.p);
+    ctx->launches += 2;
+    ws.ref_sums.alloc(static_cast<size_t>(count) * (p + 2));
+    with_p(p, [&](auto pm) {
+      lmm_pair_sums_kernel<decltype(pm)::value><<<static_cast<unsigned>((count + 7) / 8), 256, 0, st>>>(
+          ws.gt.p, n, ws.ref_col.p, pairs, count, ws.Ytil.p, ws.Xtil.p, p, ctx->basis.lambda.p, ws.delta.p,
+          ws.ref_sums.p);
+    });
+    lmm_pair_stats_kernel<<<static_cast<unsigned>((count + 63) / 64), 64, 0, st>>>(
+        ws.ref_sums.p, pairs, count, p, ws.chi0.p, ws.a00L.p, ws.rss.p, df, where, again, n_again, ws.refined.p);
     EQTL_CUDA(cudaGetLastError());
   };
   if (!exact) {
@@ -2791,7 +2855,7 @@ static void lmm_refine_pairs(eqtl_ctx* ctx, int p, double df, int n_pairs) {
 }
 
 // FP64 p of the n_tiny pairs of ws.tiny_pairs against the current LMM prep (see
-// lmm_tiny_kernel).
+// lmm_tiny_sums_kernel).
 // U_pre (optional): u = Q (w o r~) of gene g at U_pre + g * u_stride, as the
 // exact-operand scan has it already; otherwise it is computed here.
 static std::vector<double> lmm_tiny_p(eqtl_ctx* ctx, int p, double df, int n_tiny,
@@ -2819,14 +2883,18 @@ static std::vector<double> lmm_tiny_p(eqtl_ctx* ctx, int p, double df, int n_tin
     U = ws.gt.p;
     u_stride = n;
   }
-  ctx->launches += 1;
+  ctx->launches += 2;
   float s1, s2;
   output_scales(n, s1, s2);
   ws.tiny_p.alloc(static_cast<size_t>(n_tiny));
-  lmm_tiny_kernel<<<static_cast<unsigned>((n_tiny + 7) / 8), 256, 0, st>>>(
-      g.rows(), g.col.p, n, R.k_pad, g.kept.p, g.mu.p, U, u_stride, R.gt_hi.p, R.gt_lo.p, 1.0 / s1,
-      ws.Xtil.p, p, ctx->basis.lambda.p, ws.delta.p, ws.ainv.p, ws.rss.p, df, ws.tiny_pairs.p, n_tiny,
-      ws.tiny_p.p);
+  ws.ref_sums.alloc(static_cast<size_t>(n_tiny) * (p + 2));
+  with_p(p, [&](auto pm) {
+    lmm_tiny_sums_kernel<decltype(pm)::value><<<static_cast<unsigned>((n_tiny + 7) / 8), 256, 0, st>>>(
+        g.rows(), g.col.p, n, R.k_pad, g.kept.p, g.mu.p, U, u_stride, R.gt_hi.p, R.gt_lo.p, 1.0 / s1, ws.Xtil.p, p,
+        ctx->basis.lambda.p, ws.delta.p, ws.tiny_pairs.p, n_tiny, ws.ref_sums.p);
+  });
+  lmm_tiny_p_kernel<<<static_cast<unsigned>((n_tiny + 63) / 64), 64, 0, st>>>(
+      ws.ref_sums.p, ws.tiny_pairs.p, n_tiny, p, ws.ainv.p, ws.rss.p, df, ws.tiny_p.p);
   EQTL_CUDA(cudaGetLastError());
   ws.tiny_p.download(out.data(), out.size(), st);
   EQTL_CUDA(cudaStreamSynchronize(st));
@@ -3325,7 +3393,7 @@ void test_pairs_lmm(eqtl_ctx* ctx, const eqtl_scan_params* prm, const double* Y,
 // gene-side operands w, w o x_k (or w o (X U)_k, U U' = (X'WX)^-1, for
 // p > 2) and r against the unrotated centred dosages gc and gc^2, the
 // score-test epilogues (LmmEpi<P, true>, GlmGroupEpi), and the FP64
-// refinement of every candidate from the exact dosages (glm_refine_kernel).
+// refinement of every candidate from the exact dosages (glm_pair_sums_kernel).
 namespace dev {
 
 constexpr int kGlmThreads = 256;
@@ -3621,24 +3689,26 @@ __global__ void glm_means_kernel(const int64_t* __restrict__ kept, int64_t m, co
 // One warp per (gene, kept SNP) pair: the score test in FP64 from the exact
 // mean-imputed dosages g, as test_glm_nb computes it: U = g'r, g'Wg,
 // X'Wg, and the dosage variance (mean of squares - squared mean).
-__global__ void glm_refine_kernel(GenoRows src, const int32_t* __restrict__ col, int n,
-                                  const int64_t* __restrict__ kept, const double* __restrict__ mu_imp,
-                                  const double* __restrict__ W, const double* __restrict__ Rr,
-                                  const double* __restrict__ X, int p, const double* __restrict__ ainv,
-                                  const uint8_t* __restrict__ gene_ok, const int2* __restrict__ pairs, int n_pairs,
-                                  eqtl_pair* out) {
+// Sums [U, g'Wg, sum g, sum g^2, (X'Wg)_k] by a warp per pair, then the statistics by a
+// thread per pair, as for the LMM. n = 1000, p = 3, 2e8 tests: 0.35 -> 0.07 ms.
+template <int PM>
+__global__ void glm_pair_sums_kernel(GenoRows src, const int32_t* __restrict__ col, int n,
+                                     const int64_t* __restrict__ kept, const double* __restrict__ mu_imp,
+                                     const double* __restrict__ W, const double* __restrict__ Rr,
+                                     const double* __restrict__ X, int p, const int2* __restrict__ pairs, int n_pairs,
+                                     double* __restrict__ sums) {
   const int lane = threadIdx.x & 31;
   const int wid = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (wid >= n_pairs) return;
   const int g = pairs[wid].x;
-  const int64_t r = pairs[wid].y;
-  const int64_t s = kept[r];
+  const int64_t s = kept[pairs[wid].y];
   const double mus = mu_imp[s];
   const double* wg = W + static_cast<int64_t>(g) * n;
   const double* rg = Rr + static_cast<int64_t>(g) * n;
-  double U = 0, gwg = 0, sd = 0, sd2 = 0, xw[kMaxPLmm];
+  double U = 0, gwg = 0, sd = 0, sd2 = 0, xw[PM];
 #pragma unroll
-  for (int k = 0; k < kMaxPLmm; ++k) xw[k] = 0;
+  for (int k = 0; k < PM; ++k) xw[k] = 0;
+#pragma unroll(PM <= 4 ? 8 : 2)
   for (int i = lane; i < n; i += 32) {
     double d = src.dosage(s, col[i]);
     if (isnan(d)) d = mus;
@@ -3648,7 +3718,7 @@ __global__ void glm_refine_kernel(GenoRows src, const int32_t* __restrict__ col,
     sd += d;
     sd2 += d * d;
 #pragma unroll
-    for (int k = 0; k < kMaxPLmm; ++k)
+    for (int k = 0; k < PM; ++k)
       if (k < p) xw[k] += X[static_cast<int64_t>(k) * n + i] * wd;
   }
   for (int o = 16; o; o >>= 1) {
@@ -3657,10 +3727,27 @@ __global__ void glm_refine_kernel(GenoRows src, const int32_t* __restrict__ col,
     sd += __shfl_xor_sync(0xffffffffu, sd, o);
     sd2 += __shfl_xor_sync(0xffffffffu, sd2, o);
 #pragma unroll
-    for (int k = 0; k < kMaxPLmm; ++k)
+    for (int k = 0; k < PM; ++k)
       if (k < p) xw[k] += __shfl_xor_sync(0xffffffffu, xw[k], o);
   }
-  if (lane) return;
+  if (lane != 0) return;
+  double* out = sums + static_cast<int64_t>(wid) * (p + 4);
+  out[0] = U;
+  out[1] = gwg;
+  out[2] = sd;
+  out[3] = sd2;
+#pragma unroll
+  for (int k = 0; k < PM; ++k)
+    if (k < p) out[4 + k] = xw[k];
+}
+__global__ void glm_pair_stats_kernel(const double* __restrict__ sums, int n, int p, const double* __restrict__ ainv,
+                                      const uint8_t* __restrict__ gene_ok, const int2* __restrict__ pairs, int n_pairs,
+                                      eqtl_pair* __restrict__ out) {
+  const int wid = blockIdx.x * blockDim.x + threadIdx.x;
+  if (wid >= n_pairs) return;
+  const int g = pairs[wid].x;
+  const double* s = sums + static_cast<int64_t>(wid) * (p + 4);
+  const double* xw = s + 4;
   const double* A = ainv + static_cast<int64_t>(g) * p * p;
   double xAx = 0;
   for (int a = 0; a < p; ++a) {
@@ -3668,12 +3755,12 @@ __global__ void glm_refine_kernel(GenoRows src, const int32_t* __restrict__ col,
     for (int b = 0; b < p; ++b) t += A[a * p + b] * xw[b];
     xAx += xw[a] * t;
   }
-  const double mean = sd / n;
+  const double mean = s[2] / n;
   eqtl_pair q;
-  q.snp = r;
+  q.snp = pairs[wid].y;
   q.gene = g;
   q.reserved = 0;
-  glm_stats_fp64(U, gwg, xAx, sd2 / n - mean * mean, q);
+  glm_stats_fp64(s[0], s[1], xAx, s[3] / n - mean * mean, q);
   // a gene whose null fit failed tests nothing (p = NaN, test_glm_nb)
   if (!gene_ok[g]) q.p = CUDART_NAN;
   out[wid] = q;
@@ -3687,10 +3774,15 @@ static void glm_refine_pairs(eqtl_ctx* ctx, int p, int n_pairs) {
   Workspace& ws = ctx->ws;
   if (n_pairs == 0) return;
   ws.refined.alloc(static_cast<size_t>(n_pairs));
-  ++ctx->launches;
-  glm_refine_kernel<<<static_cast<unsigned>((n_pairs + 7) / 8), 256, 0, ctx->stream>>>(
-      g.rows(), g.col.p, g.n, g.kept.p, g.mu.p, ws.glm_w.p, ws.glm_r.p, ctx->pheno.X.p, p, ws.ainv.p, ws.glm_ok.p,
-      ws.ref_pairs.p, n_pairs, ws.refined.p);
+  ws.ref_sums.alloc(static_cast<size_t>(n_pairs) * (p + 4));
+  ctx->launches += 2;
+  with_p(p, [&](auto pm) {
+    glm_pair_sums_kernel<decltype(pm)::value><<<static_cast<unsigned>((n_pairs + 7) / 8), 256, 0, ctx->stream>>>(
+        g.rows(), g.col.p, g.n, g.kept.p, g.mu.p, ws.glm_w.p, ws.glm_r.p, ctx->pheno.X.p, p, ws.ref_pairs.p, n_pairs,
+        ws.ref_sums.p);
+  });
+  glm_pair_stats_kernel<<<static_cast<unsigned>((n_pairs + 63) / 64), 64, 0, ctx->stream>>>(
+      ws.ref_sums.p, g.n, p, ws.ainv.p, ws.glm_ok.p, ws.ref_pairs.p, n_pairs, ws.refined.p);
   EQTL_CUDA(cudaGetLastError());
 }
 

@@ -302,14 +302,15 @@ __global__ void __launch_bounds__(kGtgSnps)
   af_sub[r] = af;
 }
 
-// One warp per pair: FP64 gty = sum_i (g_i - mu) y_s[i] (y_s sums to zero).
-// One warp per (gene, snp) pair: gty from the exact decoded dosage in FP64,
-// then the pair's printed statistics (hit_from_gty, src/scan_trans_lm.cpp:21-36).
-__global__ void lm_refine_kernel(GenoRows src, const int32_t* __restrict__ col, int n,
-                                 const int64_t* __restrict__ kept, const double* __restrict__ mu,
-                                 const double* __restrict__ Ys, const double* __restrict__ gtg,
-                                 const double* __restrict__ yty, double df, const int2* __restrict__ pairs,
-                                 int n_pairs, eqtl_pair* out) {
+// FP64 gty = sum_i (g_i - mu) y_s[i] of listed (gene, snp) pairs from the exact
+// decoded dosages (y_s sums to zero), one warp per pair; then the pairs' printed
+// statistics (hit_from_gty, src/scan_trans_lm.cpp:21-36), one thread per pair: the
+// p-value's continued fraction costs thousands of FP64 operations, which a warp per
+// pair issued for one lane each. n = 1000, 418,000 pairs: 1.74 -> 0.78 ms.
+__global__ void lm_pair_sums_kernel(GenoRows src, const int32_t* __restrict__ col, int n,
+                                    const int64_t* __restrict__ kept, const double* __restrict__ mu,
+                                    const double* __restrict__ Ys, const int2* __restrict__ pairs, int n_pairs,
+                                    double* __restrict__ sums) {
   const int lane = threadIdx.x & 31;
   const int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (w >= n_pairs) return;
@@ -318,20 +319,27 @@ __global__ void lm_refine_kernel(GenoRows src, const int32_t* __restrict__ col, 
   const double mus = mu[s];
   const double* y = Ys + static_cast<int64_t>(pr.x) * n;
   double acc = 0;
+#pragma unroll 4
   for (int i = lane; i < n; i += 32) {
     const double d = src.dosage(s, __ldg(col + i));
     const double gc = isnan(d) ? 0.0 : d - mus;
     acc += gc * y[i];
   }
   for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  if (lane == 0) {
-    eqtl_pair q;
-    q.snp = pr.y;
-    q.gene = pr.x;
-    q.reserved = 0;
-    lm_stats_fp64(gtg[pr.y], acc, yty[pr.x], df, q);
-    out[w] = q;
-  }
+  if (lane == 0) sums[w] = acc;
+}
+__global__ void lm_pair_stats_kernel(const double* __restrict__ sums, const double* __restrict__ gtg,
+                                     const double* __restrict__ yty, double df, const int2* __restrict__ pairs,
+                                     int n_pairs, eqtl_pair* __restrict__ out) {
+  const int w = blockIdx.x * blockDim.x + threadIdx.x;
+  if (w >= n_pairs) return;
+  const int2 pr = pairs[w];
+  eqtl_pair q;
+  q.snp = pr.y;
+  q.gene = pr.x;
+  q.reserved = 0;
+  lm_stats_fp64(gtg[pr.y], sums[w], yty[pr.x], df, q);
+  out[w] = q;
 }
 
 }  // namespace dev
@@ -369,17 +377,18 @@ static void snp_gtg(eqtl_ctx* ctx, const PhenoDev& ph, int p) {
 }
 
 // FP64 statistics of the first n_pairs of ws.ref_pairs into ws.refined, against
-// the current LM prep (ws.Ys, ws.yty, ws.gtg): gty from the exact decoded dosage,
-// one warp per pair.
+// the current LM prep (ws.Ys, ws.yty, ws.gtg).
 static void lm_refine_pairs(eqtl_ctx* ctx, double df, int n_pairs) {
   Geno& g = ctx->geno;
   Workspace& ws = ctx->ws;
   if (n_pairs == 0) return;
   ws.refined.alloc(static_cast<size_t>(n_pairs));
-  ++ctx->launches;
-  lm_refine_kernel<<<static_cast<unsigned>((n_pairs + 7) / 8), 256, 0, ctx->stream>>>(
-      g.rows(), g.col.p, g.n, g.kept.p, g.mu.p, ws.Ys.p, ws.gtg.p, ws.yty.p, df, ws.ref_pairs.p, n_pairs,
-      ws.refined.p);
+  ws.ref_sums.alloc(static_cast<size_t>(n_pairs));
+  ctx->launches += 2;
+  lm_pair_sums_kernel<<<static_cast<unsigned>((n_pairs + 7) / 8), 256, 0, ctx->stream>>>(
+      g.rows(), g.col.p, g.n, g.kept.p, g.mu.p, ws.Ys.p, ws.ref_pairs.p, n_pairs, ws.ref_sums.p);
+  lm_pair_stats_kernel<<<static_cast<unsigned>((n_pairs + 63) / 64), 64, 0, ctx->stream>>>(
+      ws.ref_sums.p, ws.gtg.p, ws.yty.p, df, ws.ref_pairs.p, n_pairs, ws.refined.p);
   EQTL_CUDA(cudaGetLastError());
 }
 
