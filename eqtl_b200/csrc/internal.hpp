@@ -215,7 +215,7 @@ struct Workspace {
   // a scan's results: sort keys and their histograms, compaction counts, lists
   DevBuf<uint64_t> res_key[2], res_blk;
   DevBuf<unsigned> res_hist, res_count;
-  DevBuf<int> res_deferred, res_cand, res_dg, ref_mark;
+  DevBuf<int> res_deferred, res_cand, res_placed, res_dg, ref_mark;
   DevBuf<double> res_dp, ref_sums;
   DevBuf<int2> tiny_pairs, pairs_again;
   DevBuf<int> ref_again;

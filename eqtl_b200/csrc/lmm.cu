@@ -306,8 +306,8 @@ __global__ void reml_grid_kernel(const double* __restrict__ Xtil, const double* 
 // operations a sample remain), five grid points share the loads of y and x, as do
 // the two deltas of a golden-section or Newton step; the -logliks of 32 grid
 // points, or of the step's two deltas, are then computed in different lanes of
-// one pass. Every sum keeps its order. n = 1000, 20,000 genes, P = 1: 6.7 ->
-// 4.2 ms; n = 1201, 2,000 genes, P = 2: 1.93 -> 0.93 ms.
+// one pass. Every sum keeps its order. n = 2000, 10,000 genes, P = 1: 6.7 ->
+// 3.9 ms; n = 1201, 1,503 genes, P = 2: 1.93 -> 0.88 ms.
 constexpr int kRemlWarpP = 3;
 constexpr int kRemlThreads = 64;  // two genes a block: an even last wave for a few thousand genes
 constexpr int kRemlGridStep = 5;  // grid points per pass over the samples
@@ -2068,7 +2068,7 @@ __global__ void lmm_pair_sums_kernel(const double* __restrict__ Gt, int n, const
 // The pairs' statistics from their sums, one thread per pair (the p-value's
 // continued fraction is most of the work and does not fill a warp per pair). where
 // (optional): the place of pair w in out. again (optional): collects the pairs whose
-// S has lost more than kQgCancel of gg. Both kernels, n = 1000, p = 1, 54,600
+// S has lost more than kQgCancel of gg. Both kernels, n = 2000, p = 1, 54,600
 // pairs: 0.94 -> 0.45 ms.
 constexpr double kQgCancel = 1.0 / 1024;
 __global__ void lmm_pair_stats_kernel(const double* __restrict__ sums, const int2* __restrict__ pairs, int n_pairs,
@@ -2117,7 +2117,7 @@ __global__ void lmm_wr_kernel(const double* __restrict__ Ytil, const double* __r
 }
 
 // Sums [num, gg, a_0 .. a_{p-1}] by a warp per pair, then p by a thread per pair, as
-// for the refined pairs. n = 1000, p = 1, 62,000 pairs: 1.00 -> 0.65 ms.
+// for the refined pairs. n = 2000, p = 1, 62,000 pairs: 1.00 -> 0.65 ms.
 template <int PM>
 __global__ void lmm_tiny_sums_kernel(GenoRows src, const int32_t* __restrict__ col, int n, int k_pad,
                                      const int64_t* __restrict__ kept, const double* __restrict__ mu,
@@ -2393,7 +2393,7 @@ void lmm_rotate(eqtl_ctx* ctx) {
   R.gt2_lo.alloc(elems);
   // The epilogue's 128-row tiles reach past k_pad (a multiple of 64), so it writes
   // the zero columns from n on too: clearing the four operands first took 1.25 of
-  // 9.9 ms (n = 1000, 1e6 SNPs).
+  // 9.9 ms (n = 2000, 5e5 SNPs).
   RotEpiParams ep{};
   ep.m = m;
   ep.k_pad = k_pad;

@@ -304,6 +304,40 @@ __global__ void __launch_bounds__(T) select_block_kernel(SelectPairs f, uint64_t
   }
 }
 
+// The candidates, listed by gene and SNP, into the order gene, p, SNP: a candidate's
+// place among its gene's is the number of those before it. Quadratic in the gene's
+// candidates, of which there are a few; a gene with more than kCandRankMax sets
+// *big and the host sorts.
+constexpr int kCandRankMax = 2048;
+__global__ void cand_place_kernel(const eqtl_pair* __restrict__ refined, const int* __restrict__ cand, int n,
+                                  int* __restrict__ placed, unsigned* big) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const int ci = cand[i], g = refined[ci].gene;
+  auto lower = [&](int gene) {
+    int lo = 0, hi = n;
+    while (lo < hi) {
+      const int mid = (lo + hi) >> 1;
+      if (refined[cand[mid]].gene < gene) lo = mid + 1;
+      else hi = mid;
+    }
+    return lo;
+  };
+  const int lo = lower(g), hi = lower(g + 1);
+  if (hi - lo > kCandRankMax) {
+    placed[i] = ci;
+    *big = 1;
+    return;
+  }
+  const double p = refined[ci].p;
+  int rank = 0;
+  for (int j = lo; j < hi; ++j) {
+    const double q = refined[cand[j]].p;
+    rank += q < p || (q == p && j < i) ? 1 : 0;
+  }
+  placed[lo + rank] = ci;
+}
+
 // out: the n_pairs selected pairs in key order, then the n_cand candidates;
 // a thread per 8-byte word
 __global__ void gather_pairs_kernel(const eqtl_pair* __restrict__ refined, const uint64_t* __restrict__ key,
@@ -475,11 +509,20 @@ void ScanOutputs::finish(const eqtl_scan_params* prm, eqtl_gene_result* genes, P
   const int64_t np = static_cast<int64_t>(total & 0xFFFFFFFFull), nc = static_cast<int64_t>(total >> 32);
   pairs.n = np;
   cands.n = nc;
+  unsigned big = 0;  // some gene has too many candidates for cand_place_kernel
   if (np + nc > 0 && np <= pairs.cap && nc <= cands.cap) {
     ws.res_pairs.alloc(static_cast<size_t>(np + nc));
     ++ctx->launches;
+    if (nc > 0) {
+      ws.res_placed.alloc(static_cast<size_t>(nc));
+      EQTL_CUDA(cudaMemsetAsync(ws.res_count.p, 0, sizeof(unsigned), st));
+      ++ctx->launches;
+      cand_place_kernel<<<blocks(nc, 128), 128, 0, st>>>(refined, ws.res_cand.p, static_cast<int>(nc),
+                                                         ws.res_placed.p, ws.res_count.p);
+      ws.res_count.download(&big, 1, st);
+    }
     gather_pairs_kernel<<<static_cast<unsigned>(std::min<int64_t>(blocks((np + nc) * 7, 256), 4096)), 256, 0, st>>>(
-        refined, key, np, ws.res_cand.p, nc, ws.res_pairs.p);
+        refined, key, np, ws.res_placed.p, nc, ws.res_pairs.p);
     EQTL_CUDA(cudaGetLastError());
     ws.res_pairs.download(pairs.p, static_cast<size_t>(np), st);
     if (nc > 0)
@@ -487,7 +530,7 @@ void ScanOutputs::finish(const eqtl_scan_params* prm, eqtl_gene_result* genes, P
   }
   add_terms(genes, dp, [&](size_t i) { return dg[i]; });
   EQTL_CUDA(cudaStreamSynchronize(st));
-  if (nc <= cands.cap && np <= pairs.cap)
+  if (big)
     std::sort(cands.p, cands.p + nc, [](const eqtl_pair& a, const eqtl_pair& b) {
       if (a.gene != b.gene) return a.gene < b.gene;
       if (a.p != b.p) return a.p < b.p;

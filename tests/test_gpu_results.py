@@ -1,5 +1,6 @@
 """GPU: a scan's result lists at the sizes where their making changes: one block's
-sort (up to 4096 keys), the radix sort, several of its blocks. With pthr = 1 every
+sort (up to 4096 keys), the radix sort, several of its blocks, a gene with more
+candidates than are ranked on the device. With pthr = 1 every
 tested pair is a candidate, so the lists have exactly genes x SNPs entries."""
 import numpy as np
 import pytest
@@ -10,7 +11,7 @@ from gpu_util import check_scan
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("G,m", [(1, 3), (8, 511), (8, 512), (17, 241), (40, 700), (300, 301)])
+@pytest.mark.parametrize("G,m", [(1, 3), (8, 511), (8, 512), (17, 241), (40, 700), (300, 301), (2, 9000)])
 def test_result_lists(G, m):
     from eqtl_b200 import capi, synth
     n = 40
