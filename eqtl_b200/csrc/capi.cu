@@ -13,7 +13,6 @@
 #include <map>
 #include <mutex>
 
-#include "host_par.hpp"
 #include "internal.hpp"
 #include "scan_host.hpp"
 #include "tstat.hpp"
