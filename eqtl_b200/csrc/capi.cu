@@ -278,6 +278,9 @@ ScanOutputs::ScanOutputs(eqtl_ctx* c, int genes, int64_t snps, int64_t cap_hint)
   count.alloc(1);
   cap = static_cast<unsigned int>(std::min<int64_t>(std::max<int64_t>(cap_hint, 1 << 16), 1 << 26));
   cand.alloc(cap);
+  // here and not in run(): a scan of no kept SNPs launches nothing and still
+  // collects, and the buffers are the previous scan's
+  reset();
 }
 
 void ScanOutputs::reset() {
@@ -291,7 +294,7 @@ void ScanOutputs::reset() {
 
 void ScanOutputs::run(const std::function<void(dev::GeneOut)>& launch) {
   for (int attempt = 0; attempt < 3; ++attempt) {
-    reset();
+    if (attempt > 0) reset();
     dev::GeneOut o{acat.p, used.p, tested.p, best.p, cand.p, count.p, cap};
     launch(o);
     count.download(&n_cand, 1, ctx->stream);
