@@ -210,10 +210,16 @@ constexpr int kMaxP = 32;
 // SNP's 32 samples together) and those samples' covariates in shared memory,
 // and each thread runs its SNP's p + 1 sums over them, so a covariate value is
 // read once per block (a broadcast, two values a load) instead of once per SNP.
-// What bounds it is then the FP64 adds, n (p + 1) per SNP. The form it replaces,
-// one warp per SNP with p <= 32 guarded sums per lane, reread X from L1 for each
-// SNP and reduced p + 1 sums across the lanes: the prep stage it leads took
-// 23.6 ms at n = 1000, p = 11, 1e6 SNPs, 5.8 ms here. PM: p rounded up (the padding columns are zero).
+// What bounds it is then the FP64 adds, n (p + 1) per SNP. One warp per SNP with
+// p <= 32 guarded sums per lane rereads X from L1 for each SNP and reduces p + 1 sums
+// across the lanes: the prep stage that this kernel leads took 4.7 ms so at n = 1000,
+// p = 11, 2e5 SNPs, 1.5 here.
+// The sums are cut into runs of 16 samples, |g|^2 into runs of 4, and its runs of 16
+// meet in a compensated total: a SNP has three dosages, so one chain over the samples
+// adds the same few values again and again, and its roundings do not cancel (rms
+// error of gtg 1.0e-14 of it at n = 1000, 2.0e-14 at 2000). Here it is 1.4e-16 at both,
+// with a warp's 32 chains and their tree 3.1e-16 and 5.9e-16; the time is one chain's.
+// PM: p rounded up (the padding columns are zero).
 constexpr int kGtgSnps = 128;
 template <int PM>
 constexpr int gtg_smem_bytes() {
@@ -234,7 +240,7 @@ __global__ void __launch_bounds__(kGtgSnps)
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int64_t r0 = static_cast<int64_t>(blockIdx.x) * kGtgSnps;
   for (int e = tid; e < p * p; e += kGtgSnps) inv[e] = XtXinv[e];
-  double gg = 0.0, v[PM];
+  double gg = 0.0, gg_lost = 0.0, v[PM];
 #pragma unroll
   for (int k = 0; k < PM; ++k) v[k] = 0.0;
   for (int i0 = 0; i0 < n; i0 += 32) {
@@ -259,20 +265,37 @@ __global__ void __launch_bounds__(kGtgSnps)
       xs[(e & 31) * PM + k] = k < p && j < n ? X[static_cast<int64_t>(k) * n + j] : 0.0;
     }
     __syncthreads();
-    const int cnt = min(32, n - i0);
-#pragma unroll 4
-    for (int j = 0; j < cnt; ++j) {
-      const double g = gs[tid * 33 + j];
-      gg = fma(g, g, gg);
-      const double2* x2 = reinterpret_cast<const double2*>(xs + j * PM);
+#pragma unroll 1
+    for (int h = 0; h < 32 && i0 + h < n; h += 16) {  // samples past n are zero
+      double s16 = 0.0, sv[PM];
 #pragma unroll
-      for (int k = 0; k < PM / 2; ++k) {
-        const double2 x = x2[k];
-        v[2 * k] = fma(x.x, g, v[2 * k]);
-        v[2 * k + 1] = fma(x.y, g, v[2 * k + 1]);
+      for (int k = 0; k < PM; ++k) sv[k] = 0.0;
+#pragma unroll 1
+      for (int j0 = h; j0 < h + 16; j0 += 4) {
+        double s4 = 0.0;
+#pragma unroll
+        for (int j = j0; j < j0 + 4; ++j) {
+          const double g = gs[tid * 33 + j];
+          s4 = fma(g, g, s4);
+          const double2* x2 = reinterpret_cast<const double2*>(xs + j * PM);
+#pragma unroll
+          for (int k = 0; k < PM / 2; ++k) {
+            const double2 x = x2[k];
+            sv[2 * k] = fma(x.x, g, sv[2 * k]);
+            sv[2 * k + 1] = fma(x.y, g, sv[2 * k + 1]);
+          }
+        }
+        s16 += s4;
       }
+      // gg + s16 and what the addition rounds away
+      const double t = gg + s16, z = t - gg;
+      gg_lost += (gg - (t - z)) + (s16 - z);
+      gg = t;
+#pragma unroll
+      for (int k = 0; k < PM; ++k) v[k] += sv[k];
     }
   }
+  gg += gg_lost;
   __syncthreads();
 #pragma unroll
   for (int k = 0; k < PM; ++k) gs[tid * (PM + 1) + k] = v[k];  // each thread reads its own row back
