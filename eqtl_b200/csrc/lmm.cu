@@ -1242,7 +1242,7 @@ struct LmmEpi {
   __device__ LmmEpi(const Params& p, const TileShape&, uint8_t* smem)
       : Pr(p), tsm(reinterpret_cast<float*>(smem)), u_cand(p.t_cand * p.t_cand) {}
   __device__ void init(int tid, int nthr) {
-    if (tsm && Pr.tt.lt_u) tab = screen_tables(Pr.tt, tsm, tid, nthr);
+    if (tsm) tab = screen_tables(Pr.tt, tsm, tid, nthr);
   }
   __device__ void begin_tile(int row, int64_t s0) {
     snp0 = s0;
@@ -1754,7 +1754,7 @@ struct LmmGroupEpiT {
   __device__ LmmGroupEpiT(const Params& p, const TileShape&, uint8_t* smem)
       : Pr(p), tsm(reinterpret_cast<float*>(smem)), u_cand(p.t_cand * p.t_cand) {}
   __device__ void init(int tid, int nthr) {
-    if (Pr.tt.lt_u) tab = screen_tables(Pr.tt, tsm, tid, nthr);
+    tab = screen_tables(Pr.tt, tsm, tid, nthr);
   }
   __device__ void begin_tile(int row, int64_t s0) {
     snp0 = s0;

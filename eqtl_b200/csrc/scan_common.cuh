@@ -181,24 +181,28 @@ __device__ __noinline__ inline ChunkSums screen16_general(const TTable& tt, uint
                                                           int64_t s0) {
   ChunkSums r{0.0f, -1.0f, __popc(valid), 0, 0};
   const float uc = fminf(u_cand, tt.u_defer);
-  if (tt.lt_u && tab) {
+  if (tab) {
     const float u_tiny = tt.u_tiny, u_defer = tt.u_defer;
     float uv[16];
 #pragma unroll
     for (int j = 0; j < 16; ++j) uv[j] = u[j];
+    auto screen = [&](auto&& term_of) {
 #pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      const float uj = uv[j];
-      const bool v = (valid >> j) & 1u;
-      const float term = cubic_term(uj, tt, tab);
-      const bool lo = uj < u_tiny;
-      const bool use = v && !lo && uj < u_defer;
-      r.sum += use ? term : 0.0f;
-      r.used += use ? 1 : 0;
-      const float key = v ? uj : -1.0f;
-      r.j = key > r.score ? j : r.j;
-      r.score = fmaxf(key, r.score);
-    }
+      for (int j = 0; j < 16; ++j) {
+        const float uj = uv[j];
+        const bool v = (valid >> j) & 1u;
+        const float term = term_of(uj);
+        const bool lo = uj < u_tiny;
+        const bool use = v && !lo && uj < u_defer;
+        r.sum += use ? term : 0.0f;
+        r.used += use ? 1 : 0;
+        const float key = v ? uj : -1.0f;
+        r.j = key > r.score ? j : r.j;
+        r.score = fmaxf(key, r.score);
+      }
+    };
+    if (tt.lt_u) screen([&](float uj) { return cubic_term(uj, tt, tab); });
+    else screen([&](float uj) { return node_term(uj, tt, tab); });
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
       const bool lo = uv[j] < u_tiny;
@@ -224,6 +228,18 @@ __device__ __noinline__ inline ChunkSums screen16_general(const TTable& tt, uint
   return r;
 }
 
+// Sum of the terms of 16 pairs from the node tables (long tails, df below about 29).
+// Out of line for its registers, as screen16_general. Scan of 8e8 tests at n = 24
+// (200,000 SNPs, 4,000 genes): LM 5.3 ms, LMM (p = 1) 6.8, p = 3 10.6; with these
+// chunks left to the general form 6.3, 8.0, 12.8, and with the tables in global
+// memory besides 9.9, 11.8, 16.4.
+__device__ __noinline__ inline float node_sum16(const TTable& tt, uint32_t tab, const float* u) {
+  float sum = 0.0f;
+#pragma unroll
+  for (int j = 0; j < 16; ++j) sum += node_term(u[j], tt, tab);
+  return sum;
+}
+
 // The same screen of 16 pairs that are all tested (no SNP of the block gated,
 // none out of scope), for tables in shared memory: u_of(j) gives u = t^2 of
 // pair j, computed without the guards of the general form. Returns false,
@@ -243,13 +259,25 @@ template <class U>
 __device__ __forceinline__ bool screen16_fast(const TTable& tt, uint32_t tab, float u_cand, U&& u_of,
                                               const GeneOut& out, int gene, int64_t s0, GeneAcc& acc) {
   float sum = 0.0f, umin = INFINITY, umax = 0.0f;
+  if (tt.lt_u) {  // uniform across the launch
 #pragma unroll
-  for (int j = 0; j < 16; j += 2) {
-    const float ua = u_of(j), ub = u_of(j + 1);
-    umin = min3(umin, ua, ub);
-    umax = max3_nan(umax, ua, ub);
-    sum += cubic_term(ua, tt, tab);
-    sum += cubic_term(ub, tt, tab);
+    for (int j = 0; j < 16; j += 2) {
+      const float ua = u_of(j), ub = u_of(j + 1);
+      umin = min3(umin, ua, ub);
+      umax = max3_nan(umax, ua, ub);
+      sum += cubic_term(ua, tt, tab);
+      sum += cubic_term(ub, tt, tab);
+    }
+  } else {
+    float u[16];
+#pragma unroll
+    for (int j = 0; j < 16; j += 2) {
+      u[j] = u_of(j);
+      u[j + 1] = u_of(j + 1);
+      umin = min3(umin, u[j], u[j + 1]);
+      umax = max3_nan(umax, u[j], u[j + 1]);
+    }
+    sum = node_sum16(tt, tab, u);
   }
   if (!(umin >= tt.u_tiny && umax < tt.u_defer)) return false;
   float score = -1.0f;
@@ -289,7 +317,7 @@ __device__ __forceinline__ ChunkScope chunk_scope(const Windows& w, const GeneAc
 }
 
 // One chunk of 16 pairs through the two forms. ok: every SNP of the chunk is
-// tested and the fast form's denominators are sound; tab: cubic_base of the
+// tested and the fast form's denominators are sound; tab: screen_tables of the
 // tables in shared memory (0: none); u_fast(j): u without guards; u_gen(j, valid)
 // sets whether pair j is tested (its scope aside) and gives u with guards, never
 // NaN.
@@ -299,8 +327,7 @@ __device__ __forceinline__ void screen_chunk(const TTable& tt, uint32_t tab, flo
                                              UG&& u_gen, GeneAcc& acc) {
   const ChunkScope sc = chunk_scope(win, acc, s0);
   if (sc == kScopeNone) return;
-  if (ok && sc == kScopeAll && tab && tt.lt_u &&  // (tt.lt_u: uniform across the launch)
-      screen16_fast(tt, tab, u_cand, u_fast, out, gene, s0, acc))
+  if (ok && sc == kScopeAll && tab && screen16_fast(tt, tab, u_cand, u_fast, out, gene, s0, acc))
     return;
   float u[16];
   uint32_t valid = 0;

@@ -64,7 +64,7 @@ struct LmEpi {
   __device__ LmEpi(const Params& p, const TileShape&, uint8_t* smem)
       : P(p), tsm(reinterpret_cast<float*>(smem)), u_cand(p.t_cand * p.t_cand) {}
   __device__ void init(int tid, int nthr) {
-    if (P.tt.lt_u) tab = screen_tables(P.tt, tsm, tid, nthr);
+    tab = screen_tables(P.tt, tsm, tid, nthr);
   }
   __device__ void begin_tile(int row, int64_t s0) {
     snp0 = s0;

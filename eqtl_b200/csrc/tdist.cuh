@@ -59,12 +59,8 @@ struct TTable {
   float u_defer;    // t_defer^2, rounded down
 };
 
-__device__ __forceinline__ float lagrange4(const float* y, float x, int n_int) {
-  // x in node-step units from the region start; clamp into [0, n_int)
-  x = fminf(fmaxf(x, 0.0f), static_cast<float>(n_int) - 1e-3f);
-  const int i = static_cast<int>(x);
-  const float f = x - static_cast<float>(i);
-  const float* q = y + i;  // q[0] = node i-1 (stored with +1 offset); global or shared
+// cubic through the nodes q[0] .. q[3] at -1, 0, 1, 2
+__device__ __forceinline__ float lagrange4_at(const float* q, float f) {
   const float y0 = q[0], y1 = q[1], y2 = q[2], y3 = q[3];
   const float fm1 = f - 1.0f, fm2 = f - 2.0f, fp1 = f + 1.0f;
   const float w0 = -f * fm1 * fm2 * (1.0f / 6.0f);
@@ -72,6 +68,14 @@ __device__ __forceinline__ float lagrange4(const float* y, float x, int n_int) {
   const float w2 = -fp1 * f * fm2 * 0.5f;
   const float w3 = fp1 * f * fm1 * (1.0f / 6.0f);
   return fmaf(w0, y0, fmaf(w1, y1, fmaf(w2, y2, w3 * y3)));
+}
+
+__device__ __forceinline__ float lagrange4(const float* y, float x, int n_int) {
+  // x in node-step units from the region start; clamp into [0, n_int)
+  x = fminf(fmaxf(x, 0.0f), static_cast<float>(n_int) - 1e-3f);
+  const int i = static_cast<int>(x);
+  const float f = x - static_cast<float>(i);
+  return lagrange4_at(y + i, f);  // node i-1 first (stored with +1 offset); global or shared
 }
 
 struct TailOut {
@@ -264,12 +268,30 @@ __device__ __forceinline__ float cubic_term(float u, const TTable& T, uint32_t t
   return central ? v * rsqrt_ftz(up) : v;
 }
 
-// Copies the screen's cubics (T.lt_u) into shared memory as screen_to_smem does
-// and returns the address operand of cubic_term (never 0); the caller
-// synchronises before use.
+// The same from the node tables (long tails, !T.lt_u), with acat_screen_u's bits.
+__device__ __forceinline__ float node_term(float u, const TTable& T, uint32_t tab) {
+  const bool central = u <= T.u0;
+  const float xs = sqrtf(log1pf(u * T.inv_df));
+  const int n_int = central ? T.na + 1 : T.nb + 1;
+  float x = central ? u * T.du_inv : (xs - T.x0) * T.dl_inv;
+  x = fminf(fmaxf(x, 0.0f), static_cast<float>(n_int) - 1e-3f);
+  const int i = static_cast<int>(x);
+  const uint32_t addr = tab + 4 * static_cast<uint32_t>(central ? i : T.na + 4 + i);
+  float q[4];
+  asm("ld.shared.f32 %0, [%4];\n\tld.shared.f32 %1, [%4+4];\n\tld.shared.f32 %2, [%4+8];\n\tld.shared.f32 %3, [%4+12];"
+      : "=f"(q[0]), "=f"(q[1]), "=f"(q[2]), "=f"(q[3])
+      : "r"(addr));
+  const float y = lagrange4_at(q, x - static_cast<float>(i));
+  return central ? y * rsqrtf(u) : __expf(y);
+}
+
+// Copies the screen's tables into shared memory as screen_to_smem does and
+// returns the address operand of cubic_term (T.lt_u) or node_term (never 0); the
+// caller synchronises before use.
 __device__ __forceinline__ uint32_t screen_tables(const TTable& T, float* sm, int tid, int nthr) {
   screen_to_smem(T, sm, tid, nthr);
-  return static_cast<uint32_t>(__cvta_generic_to_shared(sm)) - (0x4B000000u << 4);
+  const uint32_t base = static_cast<uint32_t>(__cvta_generic_to_shared(sm));
+  return T.lt_u ? base - (0x4B000000u << 4) : base;
 }
 
 // Copies the t_tail tables into shared memory (cooperatively, by `nthr`
