@@ -313,24 +313,31 @@ void ScanOutputs::run(const std::function<void(dev::GeneOut)>& launch) {
 // ===================================================================== ABI
 using eqtl::Error;
 
+// What a call does with the buffers of table preparations (TableWork): those calls
+// themselves, queries and the call that allocates nothing keep them.
+enum class Tables { kGiveBack, kKeep };
+
 template <class F>
-static int guarded(eqtl_ctx* ctx, F&& f) {
+static int guarded(eqtl_ctx* ctx, F&& f, Tables tables = Tables::kGiveBack) {
   if (!ctx) return EQTL_E_ARG;
+  int rc = EQTL_E_INTERNAL;
   try {
     EQTL_CUDA(cudaSetDevice(ctx->device));
+    if (tables == Tables::kGiveBack) ctx->tables.reset();
     f();
     ctx->last_error.clear();
-    return EQTL_OK;
+    rc = EQTL_OK;
   } catch (const Error& e) {
     ctx->last_error = e.what();
-    return e.code;
+    rc = e.code;
   } catch (const std::bad_alloc&) {
     ctx->last_error = "host allocation failed";
-    return EQTL_E_NOMEM;
+    rc = EQTL_E_NOMEM;
   } catch (const std::exception& e) {
     ctx->last_error = e.what();
-    return EQTL_E_INTERNAL;
   }
+  if (ctx->tables && (rc != EQTL_OK || ctx->tables->bytes() > eqtl::kTableKeep)) ctx->tables.reset();
+  return rc;
 }
 
 extern "C" {
@@ -402,14 +409,14 @@ int eqtl_stage_ms(eqtl_ctx* ctx, int stage, double* ms) {
     float f = 0;
     EQTL_CUDA(cudaEventElapsedTime(&f, ctx->timer.start[stage], ctx->timer.stop[stage]));
     *ms = f;
-  });
+  }, Tables::kKeep);
 }
 
 int eqtl_launch_count(eqtl_ctx* ctx, uint64_t* count) {
   return guarded(ctx, [&] {
     EQTL_CHECK(count, EQTL_E_ARG, "null output");
     *count = ctx->launches;
-  });
+  }, Tables::kKeep);
 }
 
 int eqtl_lmm_form(eqtl_ctx* ctx, int32_t* nodes, int32_t* node_cols) {
@@ -417,14 +424,14 @@ int eqtl_lmm_form(eqtl_ctx* ctx, int32_t* nodes, int32_t* node_cols) {
     EQTL_CHECK(nodes && node_cols, EQTL_E_ARG, "null output");
     *nodes = ctx->ws.lr_nodes;
     *node_cols = ctx->ws.lr_nodes > 0 ? ctx->ws.lr_kn : 0;
-  });
+  }, Tables::kKeep);
 }
 
 int eqtl_stream(eqtl_ctx* ctx, void** stream) {
   return guarded(ctx, [&] {
     EQTL_CHECK(stream, EQTL_E_ARG, "null output");
     *stream = static_cast<void*>(ctx->stream);
-  });
+  }, Tables::kKeep);
 }
 
 int eqtl_lmm_rotate(eqtl_ctx* ctx) {
@@ -571,14 +578,14 @@ int eqtl_peer(eqtl_ctx* ctx, const double* Y, int32_t n, int32_t n_genes, int32_
     EQTL_CHECK(Y && X0 && W0 && X_out, EQTL_E_ARG, "null input");
     const int it = eqtl::peer_factors(ctx, Y, n, n_genes, K, max_iter, tol, X0, W0, X_out);
     if (iters_out) *iters_out = it;
-  });
+  }, Tables::kKeep);
 }
 
 int eqtl_pheno_int(eqtl_ctx* ctx, double* Y, int32_t n, int32_t n_cols) {
   return guarded(ctx, [&] {
     EQTL_CHECK(Y, EQTL_E_ARG, "null input");
     eqtl::pheno_int(ctx, Y, n, n_cols);
-  });
+  }, Tables::kKeep);
 }
 
 int eqtl_grm(eqtl_ctx* ctx, double* K_out, int32_t* N_packed_out, int64_t* m_used_out) {
@@ -601,7 +608,7 @@ int eqtl_grm_noalloc(eqtl_ctx* ctx, const uint8_t* bed_dev, int64_t m, int64_t b
     const int64_t mu = eqtl::grm_noalloc(ctx, bed_dev, m, bytes_per_snp, sample_col_dev, n, miss_hand, max_miss,
                                          maf_min, K_dev, N_packed_dev);
     if (m_used_out) *m_used_out = mu;
-  });
+  }, Tables::kKeep);
 }
 
 int eqtl_lmm_basis(eqtl_ctx* ctx, const double* K, int32_t n, double* lambda_out, double* Q_out) {

@@ -10,6 +10,7 @@
 #include <chrono>
 #include <cstdio>
 #include <cstdlib>
+#include <memory>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -209,9 +210,18 @@ struct PeerWork {
   DevBuf<int> fail;
 };
 
+// What preparing phenotype tables takes (--pheno-norm int, PEER). Programs prepare
+// several tables in a row and scan later, so the buffers stay between such calls, up
+// to kTableKeep; every other call of the context gives them back first.
+struct TableWork {
+  DevBuf<double> int_y;  // --pheno-norm int: the table
+  PeerWork peer;
+  size_t bytes() const;
+};
+constexpr size_t kTableKeep = size_t(1) << 30;
+
 // Per-call workspaces reused across calls (capacity grows, never shrinks).
 struct Workspace {
-  DevBuf<double> int_y;  // --pheno-norm int: the table
   // a scan's results: sort keys and their histograms, compaction counts, lists
   DevBuf<uint64_t> res_key[2], res_blk;
   DevBuf<unsigned> res_hist, res_count;
@@ -222,7 +232,6 @@ struct Workspace {
   DevBuf<unsigned> ref_n_again;
   DevBuf<eqtl_gene_result> res_genes;
   DevBuf<eqtl_pair> res_pairs;
-  PeerWork peer;
   DevBuf<double> Ytil, Xtil, Ys, XtY, XtXinv, delta, chi0, ainv, a00L, rss, gtg, inv_gtg, af_sub, inv_yty, yty;
   DevBuf<double> reml_w, reml_tot;  // weights and totals of the REML grid
   DevBuf<__half> ops_hi[34], ops_lo[34];  // gene-side operands, one per accumulator (dev::kMaxAcc)
@@ -338,6 +347,7 @@ struct eqtl_ctx {
   eqtl::LmmBasisDev basis;
   eqtl::PhenoDev pheno;
   eqtl::Workspace ws;
+  std::unique_ptr<eqtl::TableWork> tables;  // null: given back
   bool have_basis = false;
   int precision = EQTL_PREC_SPLIT_F16;
 };
@@ -413,6 +423,9 @@ void scan_glm(eqtl_ctx* ctx, const eqtl_scan_params* prm, const double* Y, const
               uint8_t* converged_out, eqtl_gene_result* genes, PairList& pairs, PairList& cands);
 void test_pairs_lmm(eqtl_ctx* ctx, const eqtl_scan_params* prm, const double* Y, const double* X,
                     const std::vector<int2>& todo, eqtl_pair* out, double* delta_out);
+
+// The context's table buffers, made where it has none (peer.cu).
+TableWork& table_work(eqtl_ctx* ctx);
 
 // -- stage timing (capi.cu)
 void stage_begin(eqtl_ctx* ctx, int stage);

@@ -241,6 +241,20 @@ cublasHandle_t peer_blas(eqtl_ctx* ctx) {
 
 }  // namespace
 
+size_t TableWork::bytes() const {
+  const PeerWork& w = peer;
+  size_t doubles = int_y.cap;
+  for (const DevBuf<double>* b : {&w.Yraw, &w.Y, &w.XtY, &w.E2, &w.W, &w.epsW, &w.X, &w.T1, &w.XE2S, &w.W_E2S,
+                                  &w.W_Xprec, &w.Xcov, &w.Alpha, &w.Eps, &w.b1, &w.b2, &w.part})
+    doubles += b->cap;
+  return doubles * sizeof(double);
+}
+
+TableWork& table_work(eqtl_ctx* ctx) {
+  if (!ctx->tables) ctx->tables.reset(new TableWork);
+  return *ctx->tables;
+}
+
 int peer_factors(eqtl_ctx* ctx, const double* Y_host, int n, int G, int K, int max_iter, double tol,
                  const double* X0, const double* W0, double* X_out) {
   EQTL_CHECK(n > 0 && G > 0 && K >= 1, EQTL_E_ARG, "peer: bad sizes");
@@ -251,7 +265,7 @@ int peer_factors(eqtl_ctx* ctx, const double* Y_host, int n, int G, int K, int m
   cublasHandle_t h = peer_blas(ctx);
   const int KK = K * K;
   const int64_t nG = static_cast<int64_t>(n) * G;
-  PeerWork& w = ctx->ws.peer;
+  PeerWork& w = table_work(ctx).peer;
   auto &Yraw = w.Yraw, &Y = w.Y, &XtY = w.XtY, &E2 = w.E2, &W = w.W, &epsW = w.epsW, &X = w.X, &T1 = w.T1,
        &XE2S = w.XE2S, &W_E2S = w.W_E2S, &W_Xprec = w.W_Xprec, &Xcov = w.Xcov, &Alpha = w.Alpha, &Eps = w.Eps,
        &b1 = w.b1, &b2 = w.b2, &part = w.part;

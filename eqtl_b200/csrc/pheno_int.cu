@@ -125,7 +125,7 @@ void pheno_int(eqtl_ctx* ctx, double* Y_host, int n, int G) {
              "pheno_int: more than 2^31 values in one call");
   cudaStream_t st = ctx->stream;
   const int64_t total = static_cast<int64_t>(n) * G;
-  DevBuf<double>& y = ctx->ws.int_y;
+  DevBuf<double>& y = table_work(ctx).int_y;
   y.upload(Y_host, static_cast<size_t>(total), st);
   if (n <= dev::kBlockSortMax) {
     ++ctx->launches;
