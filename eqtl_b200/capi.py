@@ -268,9 +268,25 @@ class Context:
         self.pheno_shape = (n, G * n_perm, X.shape[1])
         return Y
 
-    def _result_cap(self, G, thr):
+    def _cis_pairs(self, windows):
+        """(gene, SNP) pairs inside the windows."""
+        gchrom, glo, ghi, schrom, spos = (np.asarray(a) for a in windows[:5])
+        order = np.lexsort((spos, schrom))
+        c, s = schrom[order], spos[order]
+        total = 0
+        for ch in np.unique(gchrom[gchrom >= 0]):
+            pos = s[np.searchsorted(c, ch, "left"):np.searchsorted(c, ch, "right")]
+            g = gchrom == ch
+            count = np.searchsorted(pos, ghi[g], "right") - np.searchsorted(pos, glo[g], "left")
+            total += int(np.maximum(count, 0).sum())
+        return total
+
+    def _result_cap(self, G, thr, windows):
         """Entries to hold for the pairs of a scan below the threshold thr."""
-        expected = 3.0 * self.n_kept * G * min(max(thr, 0.0), 1.0)
+        share = 3.0 * min(max(thr, 0.0), 1.0)
+        expected = share * self.n_kept * G
+        if expected > 1 << 16 and windows is not None and int(windows[5]) == 2:
+            expected = share * self._cis_pairs(windows)  # a cis scan tests a small part of all pairs
         return (1 << 16) + int(min(expected, 1 << 24))
 
     def _scan(self, fn, Y, X, pthr, perm_thr, windows, extra=(), rotated=False):
@@ -286,11 +302,19 @@ class Context:
         # A result that does not fit costs a second scan (the full LM scan, 2e10
         # tests, 216,000 pairs: 222 ms against 117), so each list has room for
         # three times the pairs expected under the null; zeroed pages that
-        # nothing touches are never mapped.
-        cap_p, cap_c = self._result_cap(G, pthr), self._result_cap(G, perm_thr)
+        # nothing touches are never mapped, and the lists are cut to their
+        # entries in place.
+        cap_p, cap_c = self._result_cap(G, pthr, windows), self._result_cap(G, perm_thr, windows)
+        first = True
         while True:
-            pairs = np.zeros(cap_p, PAIR_DTYPE)
-            cands = np.zeros(cap_c, PAIR_DTYPE)
+            try:
+                pairs, cands = np.zeros(cap_p, PAIR_DTYPE), np.zeros(cap_c, PAIR_DTYPE)
+            except MemoryError:  # address space is limited: ask for what is found
+                if not first:
+                    raise
+                first, cap_p, cap_c = False, 1 << 16, 1 << 16
+                continue
+            first = False
             npair, ncand = C.c_int64(), C.c_int64()
             rc = fn(self.h, C.byref(prm), _ptr(Y), _ptr(X), *extra, _ptr(genes), _ptr(pairs), cap_p,
                     C.byref(npair), _ptr(cands), cap_c, C.byref(ncand))
@@ -298,7 +322,9 @@ class Context:
                 cap_p, cap_c = max(cap_p, npair.value), max(cap_c, ncand.value)
                 continue
             self._check(rc)
-            return genes, pairs[: npair.value], cands[: ncand.value]
+            pairs.resize(npair.value, refcheck=False)
+            cands.resize(ncand.value, refcheck=False)
+            return genes, pairs, cands
 
     def scan_trans_lm(self, Y, X, pthr, perm_thr=0.0, windows=None):
         """eqtl_scan_trans_lm: Y [n, G] (gene columns), X [n, p] with intercept."""
