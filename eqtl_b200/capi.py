@@ -283,7 +283,7 @@ class Context:
 
     def _result_cap(self, G, thr, windows):
         """Entries to hold for the pairs of a scan below the threshold thr."""
-        share = 3.0 * min(max(thr, 0.0), 1.0)
+        share = 3.0 * min(max(thr, 0.0), 1.0) if thr == thr else 0.0  # nothing is below NaN
         expected = share * self.n_kept * G
         if expected > 1 << 16 and windows is not None and int(windows[5]) == 2:
             expected = share * self._cis_pairs(windows)  # a cis scan tests a small part of all pairs

@@ -72,3 +72,10 @@ def test_limited_address_space(monkeypatch):
     scan.found = 1 << 23
     with pytest.raises(MemoryError):
         _run(scan, 0.05)
+
+
+def test_nan_threshold():
+    """Nothing is below it; it is the library's to accept."""
+    scan = Scan(0)
+    genes, pairs, cands = _run(scan, float("nan"), perm_thr=float("nan"))
+    assert len(genes) == G and len(pairs) == 0 and scan.offered == [(1 << 16, 1 << 16)]
