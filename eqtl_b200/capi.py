@@ -268,26 +268,10 @@ class Context:
         self.pheno_shape = (n, G * n_perm, X.shape[1])
         return Y
 
-    def _cis_pairs(self, windows):
-        """(gene, SNP) pairs inside the windows."""
-        gchrom, glo, ghi, schrom, spos = (np.asarray(a) for a in windows[:5])
-        order = np.lexsort((spos, schrom))
-        c, s = schrom[order], spos[order]
-        total = 0
-        for ch in np.unique(gchrom[gchrom >= 0]):
-            pos = s[np.searchsorted(c, ch, "left"):np.searchsorted(c, ch, "right")]
-            g = gchrom == ch
-            count = np.searchsorted(pos, ghi[g], "right") - np.searchsorted(pos, glo[g], "left")
-            total += int(np.maximum(count, 0).sum())
-        return total
-
-    def _result_cap(self, G, thr, windows):
+    def _result_cap(self, G, thr):
         """Entries to hold for the pairs of a scan below the threshold thr."""
         share = 3.0 * min(max(thr, 0.0), 1.0) if thr == thr else 0.0  # nothing is below NaN
-        expected = share * self.n_kept * G
-        if expected > 1 << 16 and windows is not None and int(windows[5]) == 2:
-            expected = share * self._cis_pairs(windows)  # a cis scan tests a small part of all pairs
-        return (1 << 16) + int(min(expected, 1 << 24))
+        return (1 << 16) + int(min(share * self.n_kept * G, 1 << 24))
 
     def _scan(self, fn, Y, X, pthr, perm_thr, windows, extra=(), rotated=False):
         if Y is None:
@@ -303,8 +287,9 @@ class Context:
         # tests, 216,000 pairs: 222 ms against 117), so each list has room for
         # three times the pairs expected under the null; zeroed pages that
         # nothing touches are never mapped, and the lists are cut to their
-        # entries in place.
-        cap_p, cap_c = self._result_cap(G, pthr, windows), self._result_cap(G, perm_thr, windows)
+        # entries in place. (A cis scan tests a small part of its pairs; counting
+        # them would cost more than the address space.)
+        cap_p, cap_c = self._result_cap(G, pthr), self._result_cap(G, perm_thr)
         first = True
         while True:
             try:

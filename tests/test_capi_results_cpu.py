@@ -43,18 +43,12 @@ def test_results_hold_their_entries(found):
     assert _held(pairs) == pairs.nbytes and _held(cands) == 0
 
 
-def test_room_of_a_cis_scan():
-    rng = np.random.default_rng(1)
-    chrom = np.sort(rng.integers(0, 20, M)).astype(np.int32)
-    pos = rng.integers(1, 1_000_000, M)
-    gchrom, lo = rng.integers(-1, 21, G).astype(np.int32), rng.integers(1, 1_000_000, G)
-    hi = lo + rng.integers(-10, 2_000, G)
+def test_room_offered():
     scan = Scan(0)
-    _run(scan, 0.05, (gchrom, lo, hi, chrom, pos, 2), perm_thr=1.0)
-    inside = sum(int(((chrom == gchrom[g]) & (pos >= lo[g]) & (pos <= hi[g])).sum()) for g in range(G) if gchrom[g] >= 0)
-    assert scan.offered == [((1 << 16) + int(0.15 * inside), (1 << 16) + 3 * inside)]
-    _run(scan, 0.05, (gchrom, lo, hi, chrom, pos, 1))
-    assert scan.offered[1][0] == (1 << 16) + (1 << 24)
+    for thr in (0.0, 1e-6, 0.05, 2.0):
+        _run(scan, thr, perm_thr=thr / 2)
+    room = [(1 << 16) + min(int(3 * M * G * t), 1 << 24) for t in (0.0, 5e-7, 1e-6, 0.025, 0.05, 1.0)]
+    assert scan.offered == [(room[0], room[0]), (room[2], room[1]), (room[4], room[3]), (room[5], room[5])]
 
 
 def test_limited_address_space(monkeypatch):
