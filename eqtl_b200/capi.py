@@ -285,7 +285,7 @@ class Context:
         genes = np.zeros(G, GENE_DTYPE)
         # A result that does not fit costs a second scan (the full LM scan, 2e10
         # tests, 216,000 pairs: 222 ms against 117), so each list has room for
-        # three times the pairs expected under the null; zeroed pages that
+        # three times the pairs expected under the null; pages that
         # nothing touches are never mapped, and the lists are cut to their
         # entries in place. (A cis scan tests a small part of its pairs; counting
         # them would cost more than the address space.)
@@ -293,7 +293,7 @@ class Context:
         first = True
         while True:
             try:
-                pairs, cands = np.zeros(cap_p, PAIR_DTYPE), np.zeros(cap_c, PAIR_DTYPE)
+                pairs, cands = np.empty(cap_p, PAIR_DTYPE), np.empty(cap_c, PAIR_DTYPE)
             except MemoryError:  # address space is limited: ask for what is found
                 if not first:
                     raise

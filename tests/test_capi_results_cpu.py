@@ -52,15 +52,15 @@ def test_room_offered():
 
 
 def test_limited_address_space(monkeypatch):
-    zeros = np.zeros
+    empty = np.empty
 
     def limited(shape, *a, **k):
         if np.prod(shape) > 1 << 22:
             raise MemoryError
-        return zeros(shape, *a, **k)
+        return empty(shape, *a, **k)
 
     scan = Scan(100_000)
-    monkeypatch.setattr(capi.np, "zeros", limited)
+    monkeypatch.setattr(capi.np, "empty", limited)
     _, pairs, _ = _run(scan, 0.05)
     assert len(pairs) == 100_000 and scan.offered == [(1 << 16, 1 << 16), (100_000, 1 << 16)]
     scan.found = 1 << 23
