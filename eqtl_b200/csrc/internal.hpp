@@ -251,6 +251,7 @@ struct Workspace {
   DevBuf<int2> tile_list;
   DevBuf<uint64_t> win_count;  // chromosome runs, listed tiles, unsorted
   DevBuf<int> win_runs;
+  DevBuf<unsigned long long> win_table;  // runs by chromosome
   DevBuf<uint8_t> win_mark;
   DevBuf<int> gene_row, row_gene;      // GeneOrder of the current scan
   DevBuf<__half> q_hi, q_lo;  // rotation: split eigenvector operand

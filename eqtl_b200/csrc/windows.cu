@@ -53,42 +53,73 @@ __global__ void win_sorted_kernel(const int32_t* __restrict__ chrom, const int64
   if (k > 0 && k < m && chrom[k] == chrom[k - 1] && pos[k] < pos[k - 1]) *unsorted = 1;
 }
 
-// Chromosome runs that a tile list is made from: more are taken for SNPs in no
-// order (a genome has tens, a draft assembly thousands of sequences).
-constexpr int64_t kWinMaxRuns = 1 << 14;
+// The runs by chromosome: a table of chromosome << 32 | run with open addressing, at
+// most half full. A genome has tens of runs, a draft assembly tens of thousands, SNPs
+// in no order as many as SNPs.
+constexpr unsigned long long kNoRun = ~0ull;
+__host__ __device__ __forceinline__ uint32_t run_slots(uint32_t n_runs) {  // power of two in [2 n, 4 n]
+  uint32_t s = 2;
+  while (s < 2 * n_runs) s *= 2;
+  return s;
+}
+__device__ __forceinline__ uint32_t run_slot(int32_t chrom, uint32_t slots) {
+  const uint32_t h = static_cast<uint32_t>(chrom) * 0x9E3779B1u;
+  return (h ^ (h >> 16)) & (slots - 1);
+}
 
-// A chromosome with two runs: the SNPs are not grouped.
-__global__ void win_runs_kernel(const int32_t* __restrict__ chrom, const int* __restrict__ start,
-                                const uint64_t* __restrict__ n_runs, unsigned* unsorted) {
-  const int64_t n = static_cast<int64_t>(*n_runs);
-  if (n > kWinMaxRuns) {
-    if (threadIdx.x == 0) *unsorted = 1;
-    return;
-  }
-  for (int64_t i = threadIdx.x; i < n; i += blockDim.x) {
+// Fills the table; a chromosome with two runs: the SNPs are not grouped. One block.
+// Cis LM call of 20,000 genes over 200,000 SNPs: 3.1 ms on 16,000 chromosomes as on
+// 100,000, against 14.1 with all runs compared with one another and searched in a row,
+// and 23.5 on the whole masked grid.
+__global__ void __launch_bounds__(1024)
+    win_runs_kernel(const int32_t* __restrict__ chrom, const int* __restrict__ start,
+                    const uint64_t* __restrict__ n_runs, unsigned long long* table, unsigned* unsorted) {
+  __shared__ unsigned stop;
+  const uint32_t n = static_cast<uint32_t>(*n_runs), slots = run_slots(n);
+  if (threadIdx.x == 0) stop = *unsorted;
+  __syncthreads();
+  if (stop) return;
+  for (uint32_t i = threadIdx.x; i < slots; i += blockDim.x) table[i] = kNoRun;
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < n && !*static_cast<volatile unsigned*>(&stop); i += blockDim.x) {
     const int32_t c = chrom[start[i]];
-    for (int64_t j = 0; j < i; ++j)
-      if (chrom[start[j]] == c) *unsorted = 1;
+    const unsigned long long entry = static_cast<unsigned long long>(static_cast<uint32_t>(c)) << 32 | i;
+    for (uint32_t h = run_slot(c, slots), k = 0; k < slots; h = (h + 1) & (slots - 1), ++k) {
+      const unsigned long long old = atomicCAS(table + h, kNoRun, entry);
+      if (old == kNoRun) break;
+      if (static_cast<int32_t>(old >> 32) == c) {
+        stop = 1;
+        *unsorted = 1;
+        break;
+      }
+    }
   }
+}
+// The run of a chromosome, or -1.
+__device__ __forceinline__ int64_t find_run(const unsigned long long* __restrict__ table, uint32_t slots,
+                                            int32_t chrom) {
+  for (uint32_t h = run_slot(chrom, slots), k = 0; k < slots; h = (h + 1) & (slots - 1), ++k) {
+    const unsigned long long e = table[h];
+    if (e == kNoRun) return -1;
+    if (static_cast<int32_t>(e >> 32) == chrom) return static_cast<int64_t>(e & 0xFFFFFFFFu);
+  }
+  return -1;
 }
 
 // Marks the tiles (128 operand rows, NT SNPs) that hold some gene's window.
 __global__ void win_mark_kernel(Windows w, int G, int64_t m, const int* __restrict__ gene_row,
                                 const int* __restrict__ start, const uint64_t* __restrict__ n_runs,
-                                const unsigned* __restrict__ unsorted, int NT, int64_t tiles_b,
+                                const unsigned long long* __restrict__ table, const unsigned* __restrict__ unsorted,
+                                int NT, int64_t tiles_b,
                                 uint8_t* __restrict__ mark) {
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= G || *unsorted) return;
   const int32_t c = w.gene_chrom[g];
   if (c < 0) return;
   const int64_t n = static_cast<int64_t>(*n_runs);
-  int64_t beg = -1, end = 0;
-  for (int64_t i = 0; i < n; ++i)
-    if (w.snp_chrom[start[i]] == c) {
-      beg = start[i];
-      end = i + 1 < n ? start[i + 1] : m;
-    }
-  if (beg < 0) return;
+  const int64_t run = find_run(table, run_slots(static_cast<uint32_t>(n)), c);
+  if (run < 0) return;
+  const int64_t beg = start[run], end = run + 1 < n ? start[run + 1] : m;
   auto first = [&](int64_t bound) {  // first SNP of the run at `bound` or after it
     int64_t lo = beg, hi = end;
     while (lo < hi) {
@@ -233,9 +264,10 @@ bool cis_tile_list(eqtl_ctx* ctx, const dev::Windows& w, int G, const GeneOrder&
   ctx->launches += 3;
   win_sorted_kernel<<<blocks(m, 256), 256, 0, st>>>(w.snp_chrom, w.snp_pos, m, unsorted);
   compact(ctx, ChromRuns{w.snp_chrom, m, ws.win_runs.p}, m, count);
-  win_runs_kernel<<<1, 1024, 0, st>>>(w.snp_chrom, ws.win_runs.p, count, unsorted);
-  win_mark_kernel<<<blocks(G, 128), 128, 0, st>>>(w, G, m, go.row, ws.win_runs.p, count, unsorted, NT, tiles_b,
-                                                  ws.win_mark.p);
+  ws.win_table.alloc(run_slots(static_cast<uint32_t>(m)));
+  win_runs_kernel<<<1, 1024, 0, st>>>(w.snp_chrom, ws.win_runs.p, count, ws.win_table.p, unsorted);
+  win_mark_kernel<<<blocks(G, 128), 128, 0, st>>>(w, G, m, go.row, ws.win_runs.p, count, ws.win_table.p, unsorted, NT,
+                                                  tiles_b, ws.win_mark.p);
   EQTL_CUDA(cudaGetLastError());
   compact(ctx, MarkedTiles{ws.win_mark.p, n_tiles, tiles_b, ws.tile_list.p}, n_tiles, count + 1);
   uint64_t c[3];
