@@ -2017,6 +2017,11 @@ struct QgEpi {
   __device__ void finish() {}
 };
 
+// The pairs [first, end) of a list, whose sums stand at the front of a buffer.
+struct PairRange {
+  int first, end;
+};
+
 // One warp per (gene, snp) pair from the FP64 rotated raw dosage Gt = Q'g:
 // gg = Gt'W Gt, yg = Gt'W y~, a = X~'W Gt with W = diag(1 / (delta lambda + 1)),
 // then the pair's printed statistics (test_lmm_gtil, src/scan_trans_lmm.cpp:11-40).
@@ -2025,12 +2030,12 @@ struct QgEpi {
 // memory and chains every sample's update through it).
 template <int PM>
 __global__ void lmm_pair_sums_kernel(const double* __restrict__ Gt, int n, const int* __restrict__ pair_col,
-                                     const int2* __restrict__ pairs, int n_pairs, const double* __restrict__ Ytil,
+                                     const int2* __restrict__ pairs, PairRange pr, const double* __restrict__ Ytil,
                                      const double* __restrict__ Xtil, int p, const double* __restrict__ lam,
                                      const double* __restrict__ delta, double* __restrict__ sums) {
   const int lane = threadIdx.x & 31;
-  const int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (w >= n_pairs) return;
+  const int w = pr.first + blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (w >= pr.end) return;
   const int g = pairs[w].x;
   const double* gt = Gt + static_cast<int64_t>(pair_col[w]) * n;
   const double* yt = Ytil + static_cast<int64_t>(g) * n;
@@ -2057,7 +2062,7 @@ __global__ void lmm_pair_sums_kernel(const double* __restrict__ Gt, int n, const
       if (k < p) a[k] += __shfl_xor_sync(0xffffffffu, a[k], o);
   }
   if (lane != 0) return;
-  double* out = sums + static_cast<int64_t>(w) * (p + 2);
+  double* out = sums + static_cast<int64_t>(w - pr.first) * (p + 2);
   out[0] = gg;
   out[1] = yg;
 #pragma unroll
@@ -2071,15 +2076,15 @@ __global__ void lmm_pair_sums_kernel(const double* __restrict__ Gt, int n, const
 // S has lost more than kQgCancel of gg. Both kernels, n = 2000, p = 1, 54,600
 // pairs: 0.94 -> 0.45 ms.
 constexpr double kQgCancel = 1.0 / 1024;
-__global__ void lmm_pair_stats_kernel(const double* __restrict__ sums, const int2* __restrict__ pairs, int n_pairs,
+__global__ void lmm_pair_stats_kernel(const double* __restrict__ sums, const int2* __restrict__ pairs, PairRange pr,
                                       int p, const double* __restrict__ chi0, const double* __restrict__ a00L,
                                       const double* __restrict__ rss, double df, const int* __restrict__ where,
                                       int* __restrict__ again, unsigned* __restrict__ n_again,
                                       eqtl_pair* __restrict__ out) {
-  const int w = blockIdx.x * blockDim.x + threadIdx.x;
-  if (w >= n_pairs) return;
+  const int w = pr.first + blockIdx.x * blockDim.x + threadIdx.x;
+  if (w >= pr.end) return;
   const int g = pairs[w].x;
-  const double* s = sums + static_cast<int64_t>(w) * (p + 2);
+  const double* s = sums + static_cast<int64_t>(w - pr.first) * (p + 2);
   eqtl_pair q;
   q.snp = pairs[w].y;
   q.gene = g;
@@ -2124,10 +2129,10 @@ __global__ void lmm_tiny_sums_kernel(GenoRows src, const int32_t* __restrict__ c
                                      const double* __restrict__ U, int64_t u_stride, const __half* __restrict__ gt_hi,
                                      const __half* __restrict__ gt_lo, double inv_s1, const double* __restrict__ Xtil,
                                      int p, const double* __restrict__ lam, const double* __restrict__ delta,
-                                     const int2* __restrict__ pairs, int n_pairs, double* __restrict__ sums) {
+                                     const int2* __restrict__ pairs, PairRange pr, double* __restrict__ sums) {
   const int lane = threadIdx.x & 31;
-  const int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (w >= n_pairs) return;
+  const int w = pr.first + blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (w >= pr.end) return;
   const int g = pairs[w].x;
   const int64_t r = pairs[w].y;
   const int64_t s = kept[r];
@@ -2160,20 +2165,20 @@ __global__ void lmm_tiny_sums_kernel(GenoRows src, const int32_t* __restrict__ c
       if (k < p) a[k] += __shfl_xor_sync(0xffffffffu, a[k], o);
   }
   if (lane != 0) return;
-  double* out = sums + static_cast<int64_t>(w) * (p + 2);
+  double* out = sums + static_cast<int64_t>(w - pr.first) * (p + 2);
   out[0] = num;
   out[1] = gg;
 #pragma unroll
   for (int k = 0; k < PM; ++k)
     if (k < p) out[2 + k] = a[k];
 }
-__global__ void lmm_tiny_p_kernel(const double* __restrict__ sums, const int2* __restrict__ pairs, int n_pairs, int p,
+__global__ void lmm_tiny_p_kernel(const double* __restrict__ sums, const int2* __restrict__ pairs, PairRange pr, int p,
                                   const double* __restrict__ ainv, const double* __restrict__ rss, double df,
                                   double* __restrict__ p_out) {
-  const int w = blockIdx.x * blockDim.x + threadIdx.x;
-  if (w >= n_pairs) return;
+  const int w = pr.first + blockIdx.x * blockDim.x + threadIdx.x;
+  if (w >= pr.end) return;
   const int g = pairs[w].x;
-  const double* s = sums + static_cast<int64_t>(w) * (p + 2);
+  const double* s = sums + static_cast<int64_t>(w - pr.first) * (p + 2);
   const double gg = s[1], *a = s + 2;
   eqtl_pair q;
   double S = -1.0;
@@ -2776,6 +2781,16 @@ static void with_p(int p, F&& f) {
   else f(std::integral_constant<int, kMaxPLmm>{});
 }
 
+// f(PairRange) over n_pairs pairs in pieces whose sums, `width` doubles a pair, take at
+// most 32 MB of ws.ref_sums (a threshold near 1 refines every pair: 10^8 of them with
+// ten covariates would take 10 GB).
+template <class F>
+static void by_sums(Workspace& ws, int n_pairs, int width, F&& f) {
+  const int piece = std::min(n_pairs, (1 << 22) / width);
+  ws.ref_sums.alloc(static_cast<size_t>(piece) * width);
+  for (int first = 0; first < n_pairs; first += piece) f(PairRange{first, first + std::min(piece, n_pairs - first)});
+}
+
 // Gt = Q'g of the u listed SNPs (ws.ref_snps) into ws.gt by DGEMM, with `pad`
 // zero columns after them.
 static void dgemm_qg(eqtl_ctx* ctx, int u, int pad) {
@@ -2818,16 +2833,18 @@ static void lmm_refine_pairs(eqtl_ctx* ctx, int p, double df, int n_pairs) {
   const bool exact = !g.dense && n <= kQgMaxN && static_cast<int64_t>(n) * n * u >= kQgMinWork;
   ws.refined.alloc(static_cast<size_t>(n_pairs));
   auto refine = [&](const int2* pairs, int count, const int* where, int* again, unsigned* n_again) {
-    ctx->launches += 2;
-    ws.ref_sums.alloc(static_cast<size_t>(count) * (p + 2));
-    with_p(p, [&](auto pm) {
-      lmm_pair_sums_kernel<decltype(pm)::value><<<static_cast<unsigned>((count + 7) / 8), 256, 0, st>>>(
-          ws.gt.p, n, ws.ref_col.p, pairs, count, ws.Ytil.p, ws.Xtil.p, p, ctx->basis.lambda.p, ws.delta.p,
-          ws.ref_sums.p);
+    by_sums(ws, count, p + 2, [&](PairRange pr) {
+      const int k = pr.end - pr.first;
+      ctx->launches += 2;
+      with_p(p, [&](auto pm) {
+        lmm_pair_sums_kernel<decltype(pm)::value><<<static_cast<unsigned>((k + 7) / 8), 256, 0, st>>>(
+            ws.gt.p, n, ws.ref_col.p, pairs, pr, ws.Ytil.p, ws.Xtil.p, p, ctx->basis.lambda.p, ws.delta.p,
+            ws.ref_sums.p);
+      });
+      lmm_pair_stats_kernel<<<static_cast<unsigned>((k + 63) / 64), 64, 0, st>>>(
+          ws.ref_sums.p, pairs, pr, p, ws.chi0.p, ws.a00L.p, ws.rss.p, df, where, again, n_again, ws.refined.p);
+      EQTL_CUDA(cudaGetLastError());
     });
-    lmm_pair_stats_kernel<<<static_cast<unsigned>((count + 63) / 64), 64, 0, st>>>(
-        ws.ref_sums.p, pairs, count, p, ws.chi0.p, ws.a00L.p, ws.rss.p, df, where, again, n_again, ws.refined.p);
-    EQTL_CUDA(cudaGetLastError());
   };
   if (!exact) {
     dgemm_qg(ctx, u, 0);
@@ -2883,19 +2900,21 @@ static std::vector<double> lmm_tiny_p(eqtl_ctx* ctx, int p, double df, int n_tin
     U = ws.gt.p;
     u_stride = n;
   }
-  ctx->launches += 2;
   float s1, s2;
   output_scales(n, s1, s2);
   ws.tiny_p.alloc(static_cast<size_t>(n_tiny));
-  ws.ref_sums.alloc(static_cast<size_t>(n_tiny) * (p + 2));
-  with_p(p, [&](auto pm) {
-    lmm_tiny_sums_kernel<decltype(pm)::value><<<static_cast<unsigned>((n_tiny + 7) / 8), 256, 0, st>>>(
-        g.rows(), g.col.p, n, R.k_pad, g.kept.p, g.mu.p, U, u_stride, R.gt_hi.p, R.gt_lo.p, 1.0 / s1, ws.Xtil.p, p,
-        ctx->basis.lambda.p, ws.delta.p, ws.tiny_pairs.p, n_tiny, ws.ref_sums.p);
+  by_sums(ws, n_tiny, p + 2, [&](PairRange pr) {
+    const int k = pr.end - pr.first;
+    ctx->launches += 2;
+    with_p(p, [&](auto pm) {
+      lmm_tiny_sums_kernel<decltype(pm)::value><<<static_cast<unsigned>((k + 7) / 8), 256, 0, st>>>(
+          g.rows(), g.col.p, n, R.k_pad, g.kept.p, g.mu.p, U, u_stride, R.gt_hi.p, R.gt_lo.p, 1.0 / s1, ws.Xtil.p, p,
+          ctx->basis.lambda.p, ws.delta.p, ws.tiny_pairs.p, pr, ws.ref_sums.p);
+    });
+    lmm_tiny_p_kernel<<<static_cast<unsigned>((k + 63) / 64), 64, 0, st>>>(
+        ws.ref_sums.p, ws.tiny_pairs.p, pr, p, ws.ainv.p, ws.rss.p, df, ws.tiny_p.p);
+    EQTL_CUDA(cudaGetLastError());
   });
-  lmm_tiny_p_kernel<<<static_cast<unsigned>((n_tiny + 63) / 64), 64, 0, st>>>(
-      ws.ref_sums.p, ws.tiny_pairs.p, n_tiny, p, ws.ainv.p, ws.rss.p, df, ws.tiny_p.p);
-  EQTL_CUDA(cudaGetLastError());
   ws.tiny_p.download(out.data(), out.size(), st);
   EQTL_CUDA(cudaStreamSynchronize(st));
   return out;
@@ -3695,11 +3714,11 @@ template <int PM>
 __global__ void glm_pair_sums_kernel(GenoRows src, const int32_t* __restrict__ col, int n,
                                      const int64_t* __restrict__ kept, const double* __restrict__ mu_imp,
                                      const double* __restrict__ W, const double* __restrict__ Rr,
-                                     const double* __restrict__ X, int p, const int2* __restrict__ pairs, int n_pairs,
+                                     const double* __restrict__ X, int p, const int2* __restrict__ pairs, PairRange pr,
                                      double* __restrict__ sums) {
   const int lane = threadIdx.x & 31;
-  const int wid = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (wid >= n_pairs) return;
+  const int wid = pr.first + blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (wid >= pr.end) return;
   const int g = pairs[wid].x;
   const int64_t s = kept[pairs[wid].y];
   const double mus = mu_imp[s];
@@ -3731,7 +3750,7 @@ __global__ void glm_pair_sums_kernel(GenoRows src, const int32_t* __restrict__ c
       if (k < p) xw[k] += __shfl_xor_sync(0xffffffffu, xw[k], o);
   }
   if (lane != 0) return;
-  double* out = sums + static_cast<int64_t>(wid) * (p + 4);
+  double* out = sums + static_cast<int64_t>(wid - pr.first) * (p + 4);
   out[0] = U;
   out[1] = gwg;
   out[2] = sd;
@@ -3741,12 +3760,12 @@ __global__ void glm_pair_sums_kernel(GenoRows src, const int32_t* __restrict__ c
     if (k < p) out[4 + k] = xw[k];
 }
 __global__ void glm_pair_stats_kernel(const double* __restrict__ sums, int n, int p, const double* __restrict__ ainv,
-                                      const uint8_t* __restrict__ gene_ok, const int2* __restrict__ pairs, int n_pairs,
+                                      const uint8_t* __restrict__ gene_ok, const int2* __restrict__ pairs, PairRange pr,
                                       eqtl_pair* __restrict__ out) {
-  const int wid = blockIdx.x * blockDim.x + threadIdx.x;
-  if (wid >= n_pairs) return;
+  const int wid = pr.first + blockIdx.x * blockDim.x + threadIdx.x;
+  if (wid >= pr.end) return;
   const int g = pairs[wid].x;
-  const double* s = sums + static_cast<int64_t>(wid) * (p + 4);
+  const double* s = sums + static_cast<int64_t>(wid - pr.first) * (p + 4);
   const double* xw = s + 4;
   const double* A = ainv + static_cast<int64_t>(g) * p * p;
   double xAx = 0;
@@ -3774,16 +3793,18 @@ static void glm_refine_pairs(eqtl_ctx* ctx, int p, int n_pairs) {
   Workspace& ws = ctx->ws;
   if (n_pairs == 0) return;
   ws.refined.alloc(static_cast<size_t>(n_pairs));
-  ws.ref_sums.alloc(static_cast<size_t>(n_pairs) * (p + 4));
-  ctx->launches += 2;
-  with_p(p, [&](auto pm) {
-    glm_pair_sums_kernel<decltype(pm)::value><<<static_cast<unsigned>((n_pairs + 7) / 8), 256, 0, ctx->stream>>>(
-        g.rows(), g.col.p, g.n, g.kept.p, g.mu.p, ws.glm_w.p, ws.glm_r.p, ctx->pheno.X.p, p, ws.ref_pairs.p, n_pairs,
-        ws.ref_sums.p);
+  by_sums(ws, n_pairs, p + 4, [&](PairRange pr) {
+    const int k = pr.end - pr.first;
+    ctx->launches += 2;
+    with_p(p, [&](auto pm) {
+      glm_pair_sums_kernel<decltype(pm)::value><<<static_cast<unsigned>((k + 7) / 8), 256, 0, ctx->stream>>>(
+          g.rows(), g.col.p, g.n, g.kept.p, g.mu.p, ws.glm_w.p, ws.glm_r.p, ctx->pheno.X.p, p, ws.ref_pairs.p, pr,
+          ws.ref_sums.p);
+    });
+    glm_pair_stats_kernel<<<static_cast<unsigned>((k + 63) / 64), 64, 0, ctx->stream>>>(
+        ws.ref_sums.p, g.n, p, ws.ainv.p, ws.glm_ok.p, ws.ref_pairs.p, pr, ws.refined.p);
+    EQTL_CUDA(cudaGetLastError());
   });
-  glm_pair_stats_kernel<<<static_cast<unsigned>((n_pairs + 63) / 64), 64, 0, ctx->stream>>>(
-      ws.ref_sums.p, g.n, p, ws.ainv.p, ws.glm_ok.p, ws.ref_pairs.p, n_pairs, ws.refined.p);
-  EQTL_CUDA(cudaGetLastError());
 }
 
 void scan_glm(eqtl_ctx* ctx, const eqtl_scan_params* prm, const double* Y, const double* X, double* phi_out,

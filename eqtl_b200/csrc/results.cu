@@ -338,20 +338,20 @@ __global__ void cand_place_kernel(const eqtl_pair* __restrict__ refined, const i
   placed[lo + rank] = ci;
 }
 
-// out: the n_pairs selected pairs in key order, then the n_cand candidates;
-// a thread per 8-byte word
+// out: rows [first, end) of the list of the n_pairs selected pairs in key order, then
+// the candidates; a thread per 8-byte word
 __global__ void gather_pairs_kernel(const eqtl_pair* __restrict__ refined, const uint64_t* __restrict__ key,
-                                    int64_t n_pairs, const int* __restrict__ cand, int64_t n_cand,
+                                    int64_t n_pairs, const int* __restrict__ cand, int64_t first, int64_t end,
                                     eqtl_pair* __restrict__ out) {
   constexpr int W = sizeof(eqtl_pair) / 8;
   static_assert(sizeof(eqtl_pair) % 8 == 0 && alignof(eqtl_pair) == 8, "eqtl_pair words");
   const uint64_t* src = reinterpret_cast<const uint64_t*>(refined);
   uint64_t* dst = reinterpret_cast<uint64_t*>(out);
-  for (int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; t < (n_pairs + n_cand) * W;
+  for (int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; t < (end - first) * W;
        t += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int64_t j = t / W;
+    const int64_t j = first + t / W;
     const int64_t i = j < n_pairs ? static_cast<int64_t>(static_cast<uint32_t>(key[j])) : cand[j - n_pairs];
-    dst[t] = src[i * W + (t - j * W)];
+    dst[t] = src[i * W + t % W];
   }
 }
 
@@ -511,8 +511,6 @@ void ScanOutputs::finish(const eqtl_scan_params* prm, eqtl_gene_result* genes, P
   cands.n = nc;
   unsigned big = 0;  // some gene has too many candidates for cand_place_kernel
   if (np + nc > 0 && np <= pairs.cap && nc <= cands.cap) {
-    ws.res_pairs.alloc(static_cast<size_t>(np + nc));
-    ++ctx->launches;
     if (nc > 0) {
       ws.res_placed.alloc(static_cast<size_t>(nc));
       EQTL_CUDA(cudaMemsetAsync(ws.res_count.p, 0, sizeof(unsigned), st));
@@ -521,12 +519,20 @@ void ScanOutputs::finish(const eqtl_scan_params* prm, eqtl_gene_result* genes, P
                                                          ws.res_placed.p, ws.res_count.p);
       ws.res_count.download(&big, 1, st);
     }
-    gather_pairs_kernel<<<static_cast<unsigned>(std::min<int64_t>(blocks((np + nc) * 7, 256), 4096)), 256, 0, st>>>(
-        refined, key, np, ws.res_placed.p, nc, ws.res_pairs.p);
-    EQTL_CUDA(cudaGetLastError());
-    ws.res_pairs.download(pairs.p, static_cast<size_t>(np), st);
-    if (nc > 0)
-      EQTL_CUDA(cudaMemcpyAsync(cands.p, ws.res_pairs.p + np, sizeof(eqtl_pair) * nc, cudaMemcpyDeviceToHost, st));
+    // in pieces of 56 MB, however long the lists
+    constexpr int64_t kPiece = 1 << 20;
+    ws.res_pairs.alloc(static_cast<size_t>(std::min(kPiece, np + nc)));
+    for (int64_t first = 0; first < np + nc; first += kPiece) {
+      const int64_t end = std::min(np + nc, first + kPiece), split = std::min(std::max(first, np), end);
+      ++ctx->launches;
+      gather_pairs_kernel<<<static_cast<unsigned>(std::min<int64_t>(blocks((end - first) * 7, 256), 4096)), 256, 0, st>>>(
+          refined, key, np, ws.res_placed.p, first, end, ws.res_pairs.p);
+      EQTL_CUDA(cudaGetLastError());
+      if (split > first) ws.res_pairs.download(pairs.p + first, static_cast<size_t>(split - first), st);
+      if (end > split)
+        EQTL_CUDA(cudaMemcpyAsync(cands.p + (split - np), ws.res_pairs.p + (split - first),
+                                  sizeof(eqtl_pair) * (end - split), cudaMemcpyDeviceToHost, st));
+    }
   }
   add_terms(genes, dp, [&](size_t i) { return dg[i]; });
   EQTL_CUDA(cudaStreamSynchronize(st));
