@@ -18,6 +18,8 @@ namespace dev {
 
 // ~2 s at 1.9 GHz: far above any legitimate wait in these kernels.
 constexpr long long kWaitCycles = 4000000000LL;
+// what a CTA of a pair that gave up leaves its copies in flight (about 2 ms)
+constexpr long long kAbortCycles = 4000000LL;
 
 // status codes written by device code into the per-launch status word
 enum DevStatus : uint32_t {

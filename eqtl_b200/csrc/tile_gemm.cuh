@@ -273,6 +273,14 @@ __global__ void __launch_bounds__(kTileThreads, 1)
         if (rank == 0) drained(&full[s], issued_phase[s]);
         if (CG == 2 && ok) drained(&empty[s], issued_phase[s]);
       }
+      // After a wait that expired the second CTA cannot tell when its last loads and
+      // the arrivals on its barriers are through (the loads count on the leader's):
+      // it stays for a thousand times what they take.
+      if (CG == 2 && rank == 1 && !ok) {
+        const long long t0 = clock64();
+        while (clock64() - t0 < kAbortCycles) {
+        }
+      }
     }
   } else if (warp == 1) {
     // ---------------------------------------------------------- MMA issuer
