@@ -480,9 +480,10 @@ __global__ void __launch_bounds__(kRemlThreads) reml_warp_kernel(
 // sums over the n samples run as FP64 GEMMs shared by all columns,
 //   A[q, s] = sum_i P[q, i] W[i, s]     P[q, i] = x~_ai x~_bi (q = tri(a, b))
 //   b[a, s] = sum_i x~_ai (W o Y)[i, s]
-// with W[i, s] = 1 / max(delta_s lambda_i + 1, 1e-12), and one thread per
-// column advances its search (golden section, Newton) between rounds; the
-// grid phase, whose deltas every column shares, runs once before them.
+// with W[i, s] = 1 / max(delta_s lambda_i + 1, 1e-12), and groups of 8, 16 or 32
+// lanes factorise a column's sums and advance its search (golden section, Newton)
+// between rounds; the grid phase, whose deltas every column shares, runs once before
+// them.
 enum : int { kRbGolden = 1, kRbCentre, kRbNewtonPair, kRbNewtonStep, kRbFinal };
 constexpr int kRbMaxRounds = 40 + 1 + 2 * 8 + 1;  // golden, centre, Newton, final
 
@@ -2818,10 +2819,11 @@ static void dgemm_qg(eqtl_ctx* ctx, int u, int pad) {
 //
 // A gene whose delta is at the top of its search leaves S = gg - a'A00^-1 a with a
 // millionth of gg: its last digits are Q'g's rounding, and p moves by 1e-8 with the
-// way Q'g was summed. Pairs that lose more than kQgCancel so are done again by
-// DGEMM, whose bits do not depend on how many SNPs are listed as long as it has a
-// grid of whole-K tiles (kQgDgemmCols columns), so that such a pair has the same p
-// in a scan of any size.
+// way Q'g was summed. Pairs of an exact list that lose more than kQgCancel so are done
+// again by DGEMM over at least kQgDgemmCols columns, where its bits depended on the
+// number of columns at one of ten n tried, so that two long lists agree about such a
+// pair. A list below kQgMinWork takes the DGEMM of its own width, which sums in another
+// order when it has few columns: there the pair keeps only what its S keeps.
 static void lmm_refine_pairs(eqtl_ctx* ctx, int p, double df, int n_pairs) {
   Geno& g = ctx->geno;
   Workspace& ws = ctx->ws;
@@ -3179,7 +3181,7 @@ static void scan_trans_lmm_impl(eqtl_ctx* ctx, const eqtl_scan_params* prm, cons
   EQTL_CHECK(p >= 1 && p <= kMaxPLmm, EQTL_E_UNSUPPORTED,
              "the LMM scan handles 1 to 32 covariate columns (intercept included)");
   EQTL_CHECK(!(simt && p > 2), EQTL_E_UNSUPPORTED, "the FP32 CUDA-core comparator covers 1 or 2 covariate columns");
-  const bool grouped = p > 2;  // accumulators run in groups of four (LmmGroupEpi)
+  const bool grouped = p > 2;  // accumulators run in groups of two (LmmGroupEpi)
   cudaStream_t st = ctx->stream;
   const double df = static_cast<double>(n - p - 1);
   const PhenoDev& ph = resolve_pheno(ctx, prm, Y, X);

@@ -278,7 +278,7 @@ struct SelectPairs {
 
 // the selection and the pairs' sort in one block, for n <= 4 T
 template <int T>
-__global__ void __launch_bounds__(T) select_block_kernel(SelectPairs f, uint64_t* total, unsigned* n_sel) {
+__global__ void __launch_bounds__(T) select_block_kernel(SelectPairs f, uint64_t* total) {
   extern __shared__ uint64_t key[];  // 4 T
   __shared__ uint64_t sm[33];
   uint64_t t[4], k[4], s = 0, all;
@@ -298,10 +298,7 @@ __global__ void __launch_bounds__(T) select_block_kernel(SelectPairs f, uint64_t
   block_sort_u64<T>(k, key);
   const int n = static_cast<int>(static_cast<uint32_t>(all));
   for (int i = threadIdx.x; i < n; i += T) f.key[i] = key[i];
-  if (threadIdx.x == 0) {
-    *total = all;
-    *n_sel = static_cast<unsigned>(n);
-  }
+  if (threadIdx.x == 0) *total = all;
 }
 
 // The candidates, listed by gene and SNP, into the order gene, p, SNP: a candidate's
@@ -490,7 +487,7 @@ void ScanOutputs::finish(const eqtl_scan_params* prm, eqtl_gene_result* genes, P
       with_sort_block(n_todo, [&](auto t) {
         constexpr int T = decltype(t)::value;
         ++ctx->launches;
-        select_block_kernel<T><<<1, T, 4 * T * sizeof(uint64_t), st>>>(f, total_of(ws), ws.res_count.p);
+        select_block_kernel<T><<<1, T, 4 * T * sizeof(uint64_t), st>>>(f, total_of(ws));
       });
       EQTL_CUDA(cudaGetLastError());
     } else {

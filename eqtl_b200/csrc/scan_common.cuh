@@ -124,10 +124,6 @@ struct GeneAcc {
   }
 };
 
-__device__ __forceinline__ void named_barrier_sync(int id, int nthreads) {
-  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
-}
-
 // 16 per-SNP flag bytes starting at a multiple of 16 (arrays padded to 16).
 __device__ __forceinline__ void load_flags16(const uint8_t* p, uint32_t (&w)[4]) {
   const uint4 v = *reinterpret_cast<const uint4*>(p);

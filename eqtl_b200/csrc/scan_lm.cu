@@ -58,7 +58,7 @@ struct LmEpi {
   bool gvalid = false;
   float w = 0;   // gscale^2 / yty
   float u_cand;  // t_cand^2
-  uint32_t tab = 0;  // cubic_base of the tables in shared memory
+  uint32_t tab = 0;  // screen_tables
   GeneAcc acc;
 
   __device__ LmEpi(const Params& p, const TileShape&, uint8_t* smem)
