@@ -1587,8 +1587,8 @@ __global__ void lr_coef_kernel(const double* __restrict__ delta, int G, const do
 // then moves 160 KB through shared memory for 128 x 128 pairs, or 120 KB on SM
 // pairs, where the 64-wide tiles that NUM and S of a thread once limited it to
 // moved 120 KB for half as many; shared memory's 128 bytes a cycle is what bounds
-// the kernel. NB-GLM scan (n = 1000, p = 3, 2e8 tests) 6.3 -> 5.2 ms (1.15 PFLOP/s
-// issued), LMM scan (n = 1000, p = 6, 2e8 tests) 10.0 -> 7.8 ms (1.23 PFLOP/s).
+// the kernel. NB-GLM scan (n = 1000, p = 3, 2e8 tests) 6.3 -> 4.3 ms (1.42 PFLOP/s
+// issued), LMM scan (n = 1000, p = 6, 2e8 tests) 10.0 -> 6.8 ms (1.44 PFLOP/s).
 //
 // Both passes (largest entry of each operand, then its halves) form a sample's
 // values from its weight and covariates in registers: one division and p PM fused
